@@ -86,22 +86,30 @@ int handles(Handles **out)
     return TCG_OK;
 }
 
-// scratch of one call, freed on return
+// scratch of one call: one device allocation, parts handed out in order, freed on return
 struct Scratch {
-    std::vector<void *> p;
+    char *base = nullptr;
+    size_t used = 0, cap = 0;
     ~Scratch()
     {
-        for (void *q : p) cudaFree(q);
+        if (base) cudaFree(base);
     }
-    int get(void **out, size_t bytes)
+    static size_t part(size_t bytes) { return (std::max<size_t>(bytes, 16) + 255) / 256 * 256; }
+    int reserve(size_t bytes)
     {
-        *out = nullptr;
-        if (cudaMalloc(out, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+        if (cudaMalloc((void **)&base, std::max<size_t>(bytes, 256)) != cudaSuccess) {
             cudaGetLastError();
+            base = nullptr;
             return fail(TCG_ERR_NOMEM, "device allocation failed");
         }
-        p.push_back(*out);
+        cap = std::max<size_t>(bytes, 256);
         return TCG_OK;
+    }
+    template <typename X> X *get(size_t n)
+    {
+        X *p = reinterpret_cast<X *>(base + used);
+        used += part(n * sizeof(X));
+        return p;
     }
 };
 
@@ -229,6 +237,194 @@ __global__ void k_scale_inv(int npw, const double2 *c, int conj_c, double2 *v)
     }
 }
 
+// ------------------------------------------- blocked Gram-Schmidt ---------
+// Modified Gram-Schmidt in the reference's order (each vector loses its
+// components along the earlier ones one after the other), arranged so that
+// many vectors advance at once: k_mgs_update takes a range of finished rows
+// out of every remaining vector (one CTA per vector, its elements in
+// registers), k_mgs_panel finishes PANEL vectors in one cluster of PANEL CTAs
+// (a vector each; the cluster barrier orders them).  The sequence of
+// operations of each vector is that of the vector-by-vector loop.
+// What bounds a projection is the read of one row by one SM (16 npw bytes) and
+// one block reduction; with one CTA for all vectors in turn the eight-atom
+// cell's step (48 new vectors on 48, 4600 plane waves) took 3400 of them in a
+// row, here 48 + 6 x 16.
+constexpr int GT = 512;          // threads per vector
+constexpr int PANEL = 8;         // vectors per cluster
+
+// sum of (x, y) over the block, the same value in every thread
+__device__ __forceinline__ double2 block_sum(double2 s)
+{
+    __shared__ double2 part[GT / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    __syncthreads();                          // the previous sum has been read
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    double2 r = part[0];
+#pragma unroll
+    for (int w = 1; w < GT / 32; w++) r = {r.x + part[w].x, r.y + part[w].y};
+    return r;
+}
+
+// A vector of npw elements spread over the block: E elements per thread in
+// registers (npw <= E GT), or, with E = 0, left in global memory.
+template <int E> struct Vec {
+    double2 v[E > 0 ? E : 1];
+    double2 *g;
+    int npw;
+    __device__ __forceinline__ void open(double2 *p, int n)
+    {
+        g = p;
+        npw = n;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int q = threadIdx.x + e * GT;
+            v[e] = q < n ? p[q] : double2{0, 0};
+        }
+    }
+    // v -= <row|v> row
+    __device__ __forceinline__ void project(const double2 *row)
+    {
+        if constexpr (E > 0) {
+            double2 r[E], s = {0, 0};
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const int q = threadIdx.x + e * GT;
+                r[e] = q < npw ? row[q] : double2{0, 0};
+            }
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                s.x += r[e].x * v[e].x + r[e].y * v[e].y;
+                s.y += r[e].x * v[e].y - r[e].y * v[e].x;
+            }
+            const double2 c = block_sum(s);
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                v[e].x -= c.x * r[e].x - c.y * r[e].y;
+                v[e].y -= c.x * r[e].y + c.y * r[e].x;
+            }
+        } else {
+            double2 s = {0, 0};
+            for (int q = threadIdx.x; q < npw; q += GT) {
+                const double2 a = row[q], b = g[q];
+                s.x += a.x * b.x + a.y * b.y;
+                s.y += a.x * b.y - a.y * b.x;
+            }
+            const double2 c = block_sum(s);
+            for (int q = threadIdx.x; q < npw; q += GT) {
+                const double2 a = row[q];
+                g[q].x -= c.x * a.x - c.y * a.y;
+                g[q].y -= c.x * a.y + c.y * a.x;
+            }
+        }
+    }
+    __device__ __forceinline__ double norm() const
+    {
+        double2 s = {0, 0};
+        if constexpr (E > 0) {
+#pragma unroll
+            for (int e = 0; e < E; e++) s.x += v[e].x * v[e].x + v[e].y * v[e].y;
+        } else {
+            for (int q = threadIdx.x; q < npw; q += GT) s.x += g[q].x * g[q].x + g[q].y * g[q].y;
+        }
+        return sqrt(block_sum(s).x);
+    }
+    __device__ __forceinline__ void store(double2 *out, double scale) const
+    {
+        if constexpr (E > 0) {
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const int q = threadIdx.x + e * GT;
+                if (q < npw) out[q] = {v[e].x * scale, v[e].y * scale};
+            }
+        } else if (out != g || scale != 1.0) {
+            for (int q = threadIdx.x; q < npw; q += GT) out[q] = {g[q].x * scale, g[q].y * scale};
+        }
+    }
+};
+
+// rows [lo[0], hi[0]) of V out of vector blockIdx.x of T (lo, hi on the device)
+template <int E>
+__global__ void __launch_bounds__(GT) k_mgs_update(int npw, const double2 *V, const int *lo, const int *hi, double2 *T)
+{
+    Vec<E> x;
+    double2 *t = T + (size_t)blockIdx.x * npw;
+    x.open(t, npw);
+    const int a = *lo, b = *hi;
+    for (int i = a; i < b; i++) x.project(V + (size_t)i * npw);
+    x.store(t, 1.0);
+}
+
+// One cluster: vectors 0 .. nv - 1 (nv <= PANEL) of T orthonormalised in order
+// and appended to V from row *count on; one whose norm is below 1e-8 is left
+// out.  count_out: the new number of rows; kept: its flag per vector.
+template <int E>
+__global__ void __cluster_dims__(PANEL, 1, 1) __launch_bounds__(GT)
+    k_mgs_panel(int npw, int nv, double2 *V, double2 *T, const int *count, int *count_out, int *kept)
+{
+    const int me = blockIdx.x;
+    Vec<E> x;
+    if (me < nv) x.open(T + (size_t)me * npw, npw);
+    int row = *count;
+    for (int j = 0; j < nv; j++) {
+        if (me == j) {
+            const double nrm = x.norm();
+            const bool ok = !(nrm < 1e-8);
+            if (ok) x.store(V + (size_t)row * npw, 1.0 / nrm);
+            if (threadIdx.x == 0) kept[j] = ok ? 1 : 0;
+        }
+        // the row and its flag become visible to the cluster
+        asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
+        const bool on = *(volatile int *)&kept[j] != 0;
+        if (on && me > j && me < nv) x.project(V + (size_t)row * npw);
+        row += on ? 1 : 0;
+    }
+    if (me == 0 && threadIdx.x == 0) *count_out = row;
+}
+
+template <int E>
+int mgs_run(int nv, int npw, double2 *V, double2 *T, int nbasis, int *counts, int *kept, cudaStream_t st)
+{
+    // counts[0] = 0, counts[1] = nbasis, then one entry per panel
+    if (nbasis > 0) k_mgs_update<E><<<nv, GT, 0, st>>>(npw, V, counts, counts + 1, T);
+    int *cnt = counts + 1;
+    for (int j0 = 0; j0 < nv; j0 += PANEL, cnt++) {
+        const int n = std::min(PANEL, nv - j0);
+        k_mgs_panel<E><<<PANEL, GT, 0, st>>>(npw, n, V, T + (size_t)j0 * npw, cnt, cnt + 1, kept + j0);
+        if (j0 + n < nv)
+            k_mgs_update<E><<<nv - j0 - n, GT, 0, st>>>(npw, V, cnt, cnt + 1, T + (size_t)(j0 + n) * npw);
+    }
+    SUB_CUDA(cudaGetLastError());
+    return TCG_OK;
+}
+
+// number of ints mgs needs
+size_t mgs_ints(int nv) { return 2 + (nv + PANEL - 1) / PANEL + (size_t)nv; }
+
+// Orthonormalise the nv vectors T against the nbasis rows of V and one another
+// and append them to V (see k_mgs_panel; V may be T when nbasis = 0 and no vector
+// vanishes).  ints: mgs_ints(nv) device ints; *rows: the new number of rows.
+int mgs(int nv, int npw, double2 *V, double2 *T, int nbasis, int *ints, int *rows, cudaStream_t st)
+{
+    const int np = (nv + PANEL - 1) / PANEL;
+    const int init[2] = {0, nbasis};
+    SUB_CUDA(cudaMemcpyAsync(ints, init, sizeof init, cudaMemcpyHostToDevice, st));
+    int *kept = ints + 2 + np, rc;
+    if (npw <= 2 * GT) rc = mgs_run<2>(nv, npw, V, T, nbasis, ints, kept, st);
+    else if (npw <= 6 * GT) rc = mgs_run<6>(nv, npw, V, T, nbasis, ints, kept, st);
+    else if (npw <= 10 * GT) rc = mgs_run<10>(nv, npw, V, T, nbasis, ints, kept, st);
+    else rc = mgs_run<0>(nv, npw, V, T, nbasis, ints, kept, st);
+    if (rc) return rc;
+    SUB_CUDA(cudaMemcpyAsync(rows, ints + 1 + np, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SUB_CUDA(cudaStreamSynchronize(st));
+    return TCG_OK;
+}
+
 // make_a_new_trial_vector (diagonalization_utils.cpp:165-211) for vector b
 // of a block, one CTA each: with the kinetic expectation
 // t = <phi| |k+G|^2 |phi> / <phi|phi> and x = |k+G|^2 / t, the Payne
@@ -299,39 +495,23 @@ extern "C" int tcg_davidson_expand(int32_t nbasis, int32_t nblock, int32_t npw, 
     if (nblock == 0) return TCG_OK;
     cudaStream_t st = (cudaStream_t)stream;
     Scratch S;
-    double2 *T, *de, *c;
     int rc;
-    if ((rc = S.get((void **)&T, (size_t)nblock * npw * sizeof(double2))) ||
-        (rc = S.get((void **)&de, nblock * sizeof(double2))) || (rc = S.get((void **)&c, sizeof(double2))))
+    const size_t nt = (size_t)nblock * npw;
+    if ((rc = S.reserve(Scratch::part(nt * sizeof(double2)) + Scratch::part(nblock * sizeof(double2)) +
+                        Scratch::part(mgs_ints(nblock) * sizeof(int)))))
         return rc;
+    double2 *T = S.get<double2>(nt), *de = S.get<double2>(nblock);
+    int *ints = S.get<int>(mgs_ints(nblock));
     SUB_CUDA(cudaMemcpyAsync(de, eig_ref, nblock * sizeof(double2), cudaMemcpyHostToDevice, st));
     k_precondition<<<nblock, 256, 0, st>>>(npw, kG2, (const double2 *)phi, (const double2 *)H1phi,
                                            (const double2 *)H2phi, (const double2 *)H3phi, de, T);
     SUB_CUDA(cudaGetLastError());
-    double2 *v = (double2 *)V;
-    int r = nbasis;
-    for (int b = 0; b < nblock; b++) {
-        // Gram_Schmidt against the whole current basis, the new vectors of
-        // this block included; a vector below norm 1e-8 is dropped
-        // (diagonalization_davidson.cpp:297-318)
-        double2 *tr = v + (size_t)r * npw;
-        SUB_CUDA(cudaMemcpyAsync(tr, T + (size_t)b * npw, npw * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-        k_gs_project<<<1, 256, 0, st>>>(npw, r, v, v, tr);
-        k_dotc<<<1, 256, 0, st>>>(npw, tr, tr, c);
-        SUB_CUDA(cudaGetLastError());
-        double2 nrm2;
-        SUB_CUDA(cudaMemcpyAsync(&nrm2, c, sizeof(double2), cudaMemcpyDeviceToHost, st));
-        SUB_CUDA(cudaStreamSynchronize(st));
-        const double nrm = std::sqrt(nrm2.x);
-        if (nrm < 1e-8) continue;
-        const double2 hn = make_double2(nrm, 0.0);
-        SUB_CUDA(cudaMemcpyAsync(c, &hn, sizeof(double2), cudaMemcpyHostToDevice, st));
-        k_scale_inv<<<8, 256, 0, st>>>(npw, c, 0, tr);
-        SUB_CUDA(cudaGetLastError());
-        SUB_CUDA(cudaStreamSynchronize(st));
-        r++;
-    }
-    *nbasis_out = r;
+    // Gram_Schmidt of each new vector against the whole current basis, the new
+    // vectors of this block included; a vector below norm 1e-8 is dropped
+    // (diagonalization_davidson.cpp:297-318)
+    int rows = 0;
+    if ((rc = mgs(nblock, npw, (double2 *)V, T, nbasis, ints, &rows, st))) return rc;
+    *nbasis_out = rows;
     return TCG_OK;
 }
 
@@ -351,15 +531,27 @@ extern "C" int tcg_subspace_ritz(int32_t ndim, int32_t npw, int32_t nout, int32_
     SUB_SOLV(cusolverDnSetStream(hd->solver, st));
     Scratch S;
     const size_t nn = (size_t)ndim * ndim;
-    double2 *Hn[3] = {nullptr, nullptr, nullptr}, *H, *A, *W, *VR, *X, *Xinv, *XL, *E;
     const void *HV[3] = {H1V, H2V, H3V};
-    for (int n = 0; n < 3; n++)
-        if (HV[n] && (rc = S.get((void **)&Hn[n], nn * sizeof(double2)))) return rc;
-    if ((rc = S.get((void **)&H, nn * sizeof(double2))) || (rc = S.get((void **)&A, nn * sizeof(double2))) ||
-        (rc = S.get((void **)&W, ndim * sizeof(double2))) || (rc = S.get((void **)&VR, nn * sizeof(double2))) ||
-        (rc = S.get((void **)&X, nn * sizeof(double2))) || (rc = S.get((void **)&Xinv, nn * sizeof(double2))) ||
-        (rc = S.get((void **)&XL, nn * sizeof(double2))) || (rc = S.get((void **)&E, 3 * (size_t)ndim * sizeof(double2))))
+    // workspace sizes of the eigensolve and the LU (the matrix arguments are not read)
+    size_t dws = 0, hws = 0;
+    int lwork = 0;
+    SUB_SOLV(cusolverDnXgeev_bufferSize(hd->solver, hd->params, CUSOLVER_EIG_MODE_NOVECTOR, CUSOLVER_EIG_MODE_VECTOR,
+                                        ndim, CUDA_C_64F, nullptr, ndim, CUDA_C_64F, nullptr, CUDA_C_64F, nullptr, ndim,
+                                        CUDA_C_64F, nullptr, ndim, CUDA_C_64F, &dws, &hws));
+    SUB_SOLV(cusolverDnZgetrf_bufferSize(hd->solver, ndim, ndim, nullptr, ndim, &lwork));
+    if ((rc = S.reserve(9 * Scratch::part(nn * sizeof(double2)) + Scratch::part(ndim * sizeof(double2)) +
+                        Scratch::part(3 * (size_t)ndim * sizeof(double2)) + Scratch::part(dws) +
+                        Scratch::part((size_t)lwork * sizeof(double2)) + 2 * Scratch::part(ndim * sizeof(int)) +
+                        Scratch::part(64 * sizeof(int)))))
         return rc;
+    double2 *Hn[3] = {nullptr, nullptr, nullptr};
+    for (int n = 0; n < 3; n++)
+        if (HV[n]) Hn[n] = S.get<double2>(nn);
+    double2 *H = S.get<double2>(nn), *A = S.get<double2>(nn), *VR = S.get<double2>(nn), *X = S.get<double2>(nn);
+    double2 *Xinv = S.get<double2>(nn), *XL = S.get<double2>(nn), *W = S.get<double2>(ndim);
+    double2 *E = S.get<double2>(3 * (size_t)ndim);
+    void *dwork = S.get<char>(dws), *lw = S.get<double2>(lwork);
+    int *dinfo = S.get<int>(64), *dperm = S.get<int>(ndim), *ipiv = S.get<int>(ndim);
     // H_n,sub(i, j) = <Vref_i | H_n V_j>   (diagonalization_davidson.cpp:462-475)
     const cuDoubleComplex one = make_cuDoubleComplex(1, 0), zero = make_cuDoubleComplex(0, 0);
     for (int n = 0; n < 3; n++)
@@ -370,13 +562,6 @@ extern "C" int tcg_subspace_ritz(int32_t ndim, int32_t npw, int32_t nout, int32_
     SUB_CUDA(cudaGetLastError());
     SUB_CUDA(cudaMemcpyAsync(A, H, nn * sizeof(double2), cudaMemcpyDeviceToDevice, st));
     // H_sub X = X D (ComplexEigenSolver, :479-486)
-    size_t dws = 0, hws = 0;
-    SUB_SOLV(cusolverDnXgeev_bufferSize(hd->solver, hd->params, CUSOLVER_EIG_MODE_NOVECTOR, CUSOLVER_EIG_MODE_VECTOR,
-                                        ndim, CUDA_C_64F, A, ndim, CUDA_C_64F, W, CUDA_C_64F, nullptr, ndim, CUDA_C_64F,
-                                        VR, ndim, CUDA_C_64F, &dws, &hws));
-    void *dwork;
-    int *dinfo;
-    if ((rc = S.get(&dwork, dws)) || (rc = S.get((void **)&dinfo, 64 * sizeof(int)))) return rc;
     std::vector<unsigned char> hwork(std::max<size_t>(hws, 16));
     SUB_SOLV(cusolverDnXgeev(hd->solver, hd->params, CUSOLVER_EIG_MODE_NOVECTOR, CUSOLVER_EIG_MODE_VECTOR, ndim,
                              CUDA_C_64F, A, ndim, CUDA_C_64F, W, CUDA_C_64F, nullptr, ndim, CUDA_C_64F, VR, ndim,
@@ -395,16 +580,9 @@ extern "C" int tcg_subspace_ritz(int32_t ndim, int32_t npw, int32_t nout, int32_
         eig_out[2 * i] = w[perm[i]].x;
         eig_out[2 * i + 1] = w[perm[i]].y;
     }
-    int *dperm;
-    if ((rc = S.get((void **)&dperm, ndim * sizeof(int)))) return rc;
     SUB_CUDA(cudaMemcpyAsync(dperm, perm.data(), ndim * sizeof(int), cudaMemcpyHostToDevice, st));
     k_permute_cols<<<ndim, 128, 0, st>>>(ndim, dperm, VR, X);
     // X^-1 by LU (eigenvectors.inverse(), :494); left eigenvectors (X^-1)^H
-    int lwork = 0;
-    SUB_SOLV(cusolverDnZgetrf_bufferSize(hd->solver, ndim, ndim, (cuDoubleComplex *)A, ndim, &lwork));
-    void *lw;
-    int *ipiv;
-    if ((rc = S.get(&lw, (size_t)lwork * sizeof(double2))) || (rc = S.get((void **)&ipiv, ndim * sizeof(int)))) return rc;
     SUB_CUDA(cudaMemcpyAsync(A, X, nn * sizeof(double2), cudaMemcpyDeviceToDevice, st));
     SUB_SOLV(cusolverDnZgetrf(hd->solver, ndim, ndim, (cuDoubleComplex *)A, ndim, (cuDoubleComplex *)lw, ipiv, dinfo));
     k_identity<<<ndim, 128, 0, st>>>(ndim, Xinv);
@@ -446,37 +624,43 @@ extern "C" int tcg_gram_schmidt(int32_t nvec, int32_t npw, void *V, void *Vl, vo
 {
     if (nvec < 0 || npw < 1 || !V) return fail(TCG_ERR_ARG, "bad Gram-Schmidt arguments");
     cudaStream_t st = (cudaStream_t)stream;
+    if (nvec == 0) return TCG_OK;
     Scratch S;
-    double2 *c;
     int rc;
-    if ((rc = S.get((void **)&c, nvec * sizeof(double2)))) return rc;
     double2 *v = (double2 *)V, *l = (double2 *)Vl;
+    if (!l) {
+        if ((rc = S.reserve(Scratch::part(mgs_ints(nvec) * sizeof(int))))) return rc;
+        int rows = 0;
+        if ((rc = mgs(nvec, npw, v, v, 0, S.get<int>(mgs_ints(nvec)), &rows, st))) return rc;
+        if (rows < nvec) return fail(TCG_ERR_NUMERIC, "Linear independence breaks in block-Davidson algorithm.");
+        return TCG_OK;
+    }
+    if ((rc = S.reserve(Scratch::part(nvec * sizeof(double2))))) return rc;
+    double2 *c = S.get<double2>(nvec);
     for (int j = 0; j < nvec; j++) {
         double2 *tj = v + (size_t)j * npw;
         // |j> -= <ref_i|j> |i>, i < j  (Gram_Schmidt / Gram_Schmidt_biortho, utils:7-77)
-        k_gs_project<<<1, 256, 0, st>>>(npw, j, l ? l : v, v, tj);
+        k_gs_project<<<1, 256, 0, st>>>(npw, j, l, v, tj);
         k_dotc<<<1, 256, 0, st>>>(npw, tj, tj, c + j);            // |j|^2
         SUB_CUDA(cudaGetLastError());
         double2 nrm2;
         SUB_CUDA(cudaMemcpyAsync(&nrm2, c + j, sizeof(double2), cudaMemcpyDeviceToHost, st));
         SUB_CUDA(cudaStreamSynchronize(st));
         const double nrm = std::sqrt(nrm2.x);
-        if (nrm < (l ? 1e-10 : 1e-8)) return fail(TCG_ERR_NUMERIC, "Linear independence breaks in block-Davidson algorithm.");
+        if (nrm < 1e-10) return fail(TCG_ERR_NUMERIC, "Linear independence breaks in block-Davidson algorithm.");
         double2 hn = make_double2(nrm, 0.0);
         SUB_CUDA(cudaMemcpyAsync(c + j, &hn, sizeof(double2), cudaMemcpyHostToDevice, st));
         k_scale_inv<<<8, 256, 0, st>>>(npw, c + j, 0, tj);
-        if (l) {
-            double2 *lj = l + (size_t)j * npw;
-            // <j| -= <j|i> <i|, then <j|j> = 1 by dividing the left vector by conj(<l_j|v_j>)
-            k_gs_project<<<1, 256, 0, st>>>(npw, j, v, l, lj);
-            k_dotc<<<1, 256, 0, st>>>(npw, lj, tj, c + j);
-            double2 cc;
-            SUB_CUDA(cudaMemcpyAsync(&cc, c + j, sizeof(double2), cudaMemcpyDeviceToHost, st));
-            SUB_CUDA(cudaStreamSynchronize(st));
-            if (std::sqrt(cc.x * cc.x + cc.y * cc.y) < 1e-10)
-                return fail(TCG_ERR_NUMERIC, "Linear independence breaks in block-Davidson algorithm.");
-            k_scale_inv<<<8, 256, 0, st>>>(npw, c + j, 1, lj);
-        }
+        double2 *lj = l + (size_t)j * npw;
+        // <j| -= <j|i> <i|, then <j|j> = 1 by dividing the left vector by conj(<l_j|v_j>)
+        k_gs_project<<<1, 256, 0, st>>>(npw, j, v, l, lj);
+        k_dotc<<<1, 256, 0, st>>>(npw, lj, tj, c + j);
+        double2 cc;
+        SUB_CUDA(cudaMemcpyAsync(&cc, c + j, sizeof(double2), cudaMemcpyDeviceToHost, st));
+        SUB_CUDA(cudaStreamSynchronize(st));
+        if (std::sqrt(cc.x * cc.x + cc.y * cc.y) < 1e-10)
+            return fail(TCG_ERR_NUMERIC, "Linear independence breaks in block-Davidson algorithm.");
+        k_scale_inv<<<8, 256, 0, st>>>(npw, c + j, 1, lj);
         SUB_CUDA(cudaGetLastError());
     }
     SUB_CUDA(cudaStreamSynchronize(st));
