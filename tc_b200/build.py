@@ -2,7 +2,7 @@
 
 api.cu (C-ABI, orchestration, generic kernels), subspace.cu (the dense
 Davidson subspace step on cuBLAS / cuSOLVER) and one instance of fast_inst.cu
-per compiled cubic grid size are compiled in parallel into tc_b200/_build/
+per compiled cubic grid size and precision are compiled in parallel into tc_b200/_build/
 and linked into tc_b200/libtcg_b200.so.
 """
 import concurrent.futures as cf
@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 SO = os.path.join(HERE, "libtcg_b200.so")
 SRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
-FAST_SIZES = (12, 16, 24, 32, 36, 40, 48)
+FAST_SIZES = (12, 15, 16, 18, 20, 24, 25, 27, 30, 32, 36, 40, 45, 48)     # ctx.cuh: TCG_FAST_SIZES
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
 
@@ -34,8 +34,10 @@ def stale():
 def _units():
     units = [(os.path.join(SRC, "api.cu"), os.path.join(OBJ, "api.o"), []),
              (os.path.join(SRC, "subspace.cu"), os.path.join(OBJ, "subspace.o"), [])]
-    for n in FAST_SIZES:
-        units.append((os.path.join(SRC, "fast_inst.cu"), os.path.join(OBJ, f"fast_{n}.o"), [f"-DTCG_FAST_N={n}"]))
+    for t in ("double", "float"):                 # the longest units first
+        for n in reversed(FAST_SIZES):
+            units.append((os.path.join(SRC, "fast_inst.cu"), os.path.join(OBJ, f"fast_{n}_{t}.o"),
+                          [f"-DTCG_FAST_N={n}", f"-DTCG_FAST_T={t}"]))
     return units
 
 

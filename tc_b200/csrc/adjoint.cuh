@@ -230,10 +230,21 @@ static int energy_grad_impl(tcg_ctx *c, uint32_t mask, double *e_out, void *dchi
         double2 *dv2 = c->adjt.as<double2>(), *du = dv2 + (size_t)h.nspin * N;
         TCG_CUDA(cudaMemsetAsync(dv2, 0, (size_t)2 * h.nspin * N * sizeof(double2), c->stream));
         for (int s = 0; s < h.nspin; s++) TRY(grad_tables_tc2x<T>(c, s, dv2 + (size_t)s * N, du + (size_t)s * N));
-        if (dv2_out)
-            TCG_CUDA(cudaMemcpyAsync(dv2_out, dv2, (size_t)h.nspin * N * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
-        if (du_out)
-            TCG_CUDA(cudaMemcpyAsync(du_out, du, (size_t)h.nspin * N * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
+        // the tables vanish beyond the pair densities' sphere, which a smaller work grid holds
+        const size_t uN = h.uN;
+        const double2 *from[2] = {dv2, du};
+        double *to[2] = {dv2_out, du_out};
+        for (int q = 0; q < 2; q++)
+            for (int s = 0; s < h.nspin && to[q]; s++) {
+                const double2 *src = from[q] + (size_t)s * N;
+                if (h.reduced) {
+                    TRY(c->uwork.ensure(uN * sizeof(double2)));
+                    TRY(to_user_grid(c, src, c->uwork.as<double2>()));
+                    src = c->uwork.as<double2>();
+                }
+                TCG_CUDA(cudaMemcpyAsync(to[q] + 2 * (size_t)s * uN, src, uN * sizeof(double2), cudaMemcpyDeviceToHost,
+                                         c->stream));
+            }
         TCG_CUDA(cudaStreamSynchronize(c->stream));
     }
     return TCG_OK;

@@ -51,7 +51,7 @@ static int validate_system(const tcg_system_desc *s)
     return TCG_OK;
 }
 
-// Pencil table of the pruned transforms (36^3 path).  A pair density
+// Pencil table of the pruned transforms.  A pair density
 // conj(a_q(r)) b_k(r) of two orbitals on the plane-wave spheres of q and k
 // has Fourier components G = G1 - G2 with |k + G1| <= R_k and |q + G2| <= R_q,
 // so it vanishes outside the ball |G + k - q| < R_k + R_q; for every
@@ -59,13 +59,13 @@ static int validate_system(const tcg_system_desc *s)
 // that meet that ball, and lists them first.  Built only when no ball reaches
 // past the grid's Miller range (the support would wrap) and the table stays
 // under 256 MB.
-static int build_prune_table(tcg_ctx *c)
+int tcg::build_prune_table(tcg_ctx *c)
 {
     Host &h = c->h;
     c->prune_ok = false;
     const int n0 = h.n[0], n1 = h.n[1], n2 = h.n[2], np = n0 * n1;
-    const size_t nent = (size_t)h.nk * h.nk_all;
-    if (nent * np * 3 + nent * sizeof(int) + nent * n0 * 8 > ((size_t)256 << 20)) return TCG_OK;
+    const PruneTable pt(h);
+    if (pt.bytes > ((size_t)256 << 20)) return TCG_OK;
     auto cartv = [&](const double *x, double *v) {
         for (int d = 0; d < 3; d++) v[d] = h.recip[0 * 3 + d] * x[0] + h.recip[1 * 3 + d] * x[1] + h.recip[2 * 3 + d] * x[2];
     };
@@ -75,11 +75,11 @@ static int build_prune_table(tcg_ctx *c)
     for (int k = 0; k < h.nk; k++) {
         double kc[3];
         cartv(&h.kvec[3 * h.kall_off[k]], kc);
-        const size_t o = h.gidx_off[h.kall_off[k]];
-        for (int p = 0; p < h.npw[k]; p++) {
-            const int gi = h.gidx_host[o + p];
-            const double m[3] = {(double)signed_m(gi % n0, n0), (double)signed_m((gi / n0) % n1, n1),
-                                 (double)signed_m(gi / np, n2)};
+        for (int p = 0; p < h.npw[k] * h.nspin; p++) {
+            const size_t o = h.gidx_off[(size_t)(p / h.npw[k]) * h.nk_all + h.kall_off[k]];
+            int mi[3];
+            miller_of(h, h.gidx_host[o + p % h.npw[k]], mi);
+            const double m[3] = {(double)mi[0], (double)mi[1], (double)mi[2]};
             double G[3];
             cartv(m, G);
             const double r = sqrt((kc[0] + G[0]) * (kc[0] + G[0]) + (kc[1] + G[1]) * (kc[1] + G[1]) +
@@ -94,13 +94,11 @@ static int build_prune_table(tcg_ctx *c)
                        h.lattice[3 * i + 2] * h.lattice[3 * i + 2]) / (2.0 * PI_D);
     const double *b1 = &h.recip[0], *b2 = &h.recip[3], *b3 = &h.recip[6];
     const double b33 = b3[0] * b3[0] + b3[1] * b3[1] + b3[2] * b3[2];
-    if (n1 > 64) return TCG_OK;                       // column bit masks hold 64 rows
-    const size_t bits_off = (nent * np * 3 + nent * sizeof(int) + 7) & ~(size_t)7;
-    std::vector<unsigned char> tab(bits_off + nent * n0 * sizeof(unsigned long long));
-    unsigned char *mask = tab.data();
-    unsigned short *perm = reinterpret_cast<unsigned short *>(tab.data() + nent * np);
-    int *nact = reinterpret_cast<int *>(tab.data() + nent * np * 3);
-    unsigned long long *bits = reinterpret_cast<unsigned long long *>(tab.data() + bits_off);
+    if (n0 > 64) return TCG_OK;                       // row bit masks hold 64 x
+    std::vector<unsigned char> tab(pt.bytes);
+    unsigned long long *bits = reinterpret_cast<unsigned long long *>(tab.data());
+    int *nact = reinterpret_cast<int *>(tab.data() + pt.nact);
+    unsigned short *perm = reinterpret_cast<unsigned short *>(tab.data() + pt.perm);
     const int zlo = -((n2 - 1) / 2), zhi = n2 / 2;
     for (int ik = 0; ik < h.nk; ik++)
         for (int a = 0; a < h.nk_all; a++) {
@@ -118,8 +116,8 @@ static int build_prune_table(tcg_ctx *c)
             }
             int na = 0;
             std::vector<int> act, inact;
-            for (int y = 0; y < n1; y++)
-                for (int x = 0; x < n0; x++) {
+            for (int x = 0; x < n0; x++)
+                for (int y = 0; y < n1; y++) {
                     const int mx = signed_m(x, n0), my = signed_m(y, n1);
                     double P[3];
                     for (int d = 0; d < 3; d++) P[d] = mx * b1[d] + my * b2[d] + kq[d];
@@ -132,9 +130,8 @@ static int build_prune_table(tcg_ctx *c)
                         const double zl = std::max(ceil(lo), (double)zlo), zh = std::min(floor(hi), (double)zhi);
                         on = zl <= zh;
                     }
-                    mask[e * np + x + n0 * y] = on ? 1 : 0;
-                    if (on) bits[e * n0 + x] |= 1ull << y;
-                    (on ? act : inact).push_back(x + n0 * y);
+                    if (on) bits[e * n1 + y] |= 1ull << x;
+                    (on ? act : inact).push_back(y + n1 * x);
                     na += on;
                 }
             for (size_t i = 0; i < act.size(); i++) perm[e * np + i] = (unsigned short)act[i];
@@ -143,7 +140,7 @@ static int build_prune_table(tcg_ctx *c)
         }
     TRY(up(c->prune_tab, tab.data(), tab.size(), c->stream));
     TCG_CUDA(cudaStreamSynchronize(c->stream));
-    c->prune_nact.assign(nact, nact + nent);
+    c->prune_nact.assign(nact, nact + pt.nent);
     c->prune_ok = true;
     return TCG_OK;
 }
@@ -163,8 +160,8 @@ extern "C" int tcg_ctx_create(const tcg_system_desc *sys, int32_t precision, tcg
     c->prec = precision;
     cudaGetDevice(&c->device);
     Host &h = c->h;
-    for (int d = 0; d < 3; d++) h.n[d] = sys->nr[d];
-    h.N = h.n[0] * h.n[1] * h.n[2];
+    for (int d = 0; d < 3; d++) h.un[d] = h.n[d] = sys->nr[d];
+    h.uN = h.N = h.n[0] * h.n[1] * h.n[2];
     memcpy(h.recip, sys->recip, sizeof h.recip);
     memcpy(h.lattice, sys->lattice, sizeof h.lattice);
     h.omega = sys->omega;
@@ -231,85 +228,50 @@ extern "C" int tcg_ctx_create(const tcg_system_desc *sys, int32_t precision, tcg
         }
     const size_t ngi = off;
     h.gidx_host.assign(sys->gindex, sys->gindex + ngi);
-    std::vector<int> inv((size_t)h.nspin * h.nk_all * h.N, -1);
-    for (int s = 0; s < h.nspin && rc == TCG_OK; s++)
-        for (int a = 0; a < h.nk_all && rc == TCG_OK; a++) {
-            const size_t o = h.gidx_off[(size_t)s * h.nk_all + a];
-            int *im = inv.data() + ((size_t)s * h.nk_all + a) * h.N;
-            for (int p = 0; p < h.npw[h.ik_of_all[a]]; p++) {
-                const int gi = sys->gindex[o + p];
-                if (gi < 0 || gi >= h.N) { rc = fail(TCG_ERR_ARG, "gindex out of range"); break; }
-                if (im[gi] >= 0) { rc = fail(TCG_ERR_ARG, "duplicate gindex within one k-point"); break; }
-                im[gi] = p;
-            }
-        }
-    if (rc != TCG_OK) { delete c; return rc; }
-    // plane-wave -> grid index of every (spin, irreducible k) at isym 0 (one-body terms)
-    std::vector<int> g0;
-    h.g0_off.resize((size_t)h.nspin * h.nk);
-    for (int s = 0; s < h.nspin; s++)
-        for (int k = 0; k < h.nk; k++) {
-            h.g0_off[(size_t)s * h.nk + k] = g0.size();
-            const size_t o = h.gidx_off[(size_t)s * h.nk_all + h.kall_off[k]];
-            g0.insert(g0.end(), sys->gindex + o, sys->gindex + o + h.npw[k]);
-        }
-    // FFT plans
-    GridDesc &g = c->gd;
-    g.n0 = h.n[0]; g.n1 = h.n[1]; g.n2 = h.n[2]; g.N = h.N;
-    for (int d = 0; d < 3; d++)
-        if ((rc = make_axis(h.n[d], g.ax[d])) != TCG_OK) { delete c; return rc; }
     {
-        const double PI = 3.14159265358979323846;
-        std::vector<double2> t64(3 * MAXN);
-        std::vector<float2> t32(3 * MAXN);
-        for (int d = 0; d < 3; d++)
-            for (int j = 0; j < h.n[d]; j++) {
-                long double a = 2.0L * (long double)PI * j / h.n[d];
-                double cr = (double)cosl(a), ci = -(double)sinl(a);
-                t64[d * MAXN + j] = make_double2(cr, ci);
-                t32[d * MAXN + j] = make_float2((float)cr, (float)ci);
+        std::vector<int> seen(h.N, -1);
+        for (int s = 0, id = 0; s < h.nspin && rc == TCG_OK; s++)
+            for (int a = 0; a < h.nk_all && rc == TCG_OK; a++, id++) {
+                const size_t o = h.gidx_off[(size_t)s * h.nk_all + a];
+                for (int p = 0; p < h.npw[h.ik_of_all[a]]; p++) {
+                    const int gi = sys->gindex[o + p];
+                    if (gi < 0 || gi >= h.N) { rc = fail(TCG_ERR_ARG, "gindex out of range"); break; }
+                    if (seen[gi] == id) { rc = fail(TCG_ERR_ARG, "duplicate gindex within one k-point"); break; }
+                    seen[gi] = id;
+                }
             }
-        if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
-            cudaGetLastError();
-            delete c;
-            return fail(TCG_ERR_CUDA, "stream creation failed");
-        }
-        if ((rc = up(c->tw64, t64.data(), t64.size() * sizeof(double2), c->stream)) ||
-            (rc = up(c->tw32, t32.data(), t32.size() * sizeof(float2), c->stream)) ||
-            (rc = up(c->recip, h.recip, sizeof h.recip, c->stream)) ||
-            (rc = up(c->inv, inv.data(), inv.size() * sizeof(int), c->stream)) ||
-            (rc = up(c->phase, sys->phase, ngi * sizeof(double2), c->stream)) ||
-            (rc = up(c->gidx0, g0.data(), g0.size() * sizeof(int), c->stream))) {
-            tcg_ctx_destroy(c);
-            return rc;
-        }
-        g.tw64 = c->tw64.as<const double2>();
-        g.tw32 = c->tw32.as<const float2>();
     }
-    if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
-        tcg_ctx_destroy(c);
-        return fail(TCG_ERR_CUDA, "upload failed");
-    }
-    if (h.n[0] == h.n[1] && h.n[1] == h.n[2]) {
-        const int fastn[] = {12, 16, 24, 32, 36, 40, 48};
-        for (int f : fastn)
-            if (h.n[0] == f) c->fast_n = f;
+    Axis ax;
+    for (int d = 0; d < 3 && rc == TCG_OK; d++) rc = make_axis(h.n[d], ax);
+    if (rc != TCG_OK) { delete c; return rc; }
+    if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaGetLastError();
+        delete c;
+        return fail(TCG_ERR_CUDA, "stream creation failed");
     }
     if (getenv("TCG_GENERIC_PASSES")) c->force_generic = true;
     if (getenv("TCG_NO_PRUNE")) c->no_prune = true;
     if (getenv("TCG_SACC")) c->use_sacc = true;
     if (getenv("TCG_NO_QP_SACC")) c->qp_sacc = false;
     if (getenv("TCG_NO_FUSE")) c->no_fuse = true;
-    if (split_line_grid(c->fast_n) && (rc = build_prune_table(c)) != TCG_OK) {
-        tcg_ctx_destroy(c);
-        return rc;
-    }
     if (const char *e = getenv("TCG_XY_KERNELS"))   // "line" / "pair": override the per-term choice
         c->xy_kernels = !strcmp(e, "line") ? 1 : (!strcmp(e, "pair") ? 2 : (!strcmp(e, "t6") ? 3 : 0));
     if (getenv("TCG_NO_PREFETCH")) c->no_prefetch = true;
     if (const char *e = getenv("TCG_MIN_TARGETS")) c->min_targets = atoi(e);
     if (const char *e = getenv("TCG_Z_KERNELS"))    // "line" / "split": override the per-term choice
         c->z_kernels = !strcmp(e, "line") ? 1 : (!strcmp(e, "split") ? 2 : (!strcmp(e, "t6") ? 3 : (!strcmp(e, "t6r") ? 4 : 0)));
+    h.red_n = choose_reduced(h);
+    if ((rc = make_grid(c, h.un, c->ugd, c->utw64, c->utw32)) ||
+        (rc = up(c->recip, h.recip, sizeof h.recip, c->stream)) ||
+        (rc = up(c->phase, sys->phase, ngi * sizeof(double2), c->stream)) ||
+        (rc = configure_grid(c, h.red_n && c->xy_kernels == 0 && c->z_kernels == 0 && !c->force_generic))) {
+        tcg_ctx_destroy(c);
+        return rc;
+    }
+    if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
+        tcg_ctx_destroy(c);
+        return fail(TCG_ERR_CUDA, "upload failed");
+    }
     *out = c;
     return TCG_OK;
 }
@@ -318,7 +280,7 @@ extern "C" int tcg_ctx_destroy(tcg_ctx *c)
 {
     if (!c) return TCG_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    DBuf *bufs[] = {&c->gpsi, &c->adjw, &c->adjt, &c->prune_tab, &c->VH, &c->V2h, &c->pgw, &c->gidx0, &c->vloc, &c->nlB, &c->nlD, &c->acc1, &c->h1buf,
+    DBuf *bufs[] = {&c->utw64, &c->utw32, &c->ballmap, &c->udens, &c->uvloc, &c->uwork, &c->w3x, &c->gpsi, &c->adjw, &c->adjt, &c->prune_tab, &c->VH, &c->V2h, &c->pgw, &c->gidx0, &c->vloc, &c->nlB, &c->nlD, &c->acc1, &c->h1buf,
                     &c->tw64, &c->tw32, &c->recip, &c->inv, &c->phase, &c->phik, &c->chik, &c->fill,
                     &c->Rocc, &c->Rchi, &c->Rgrad, &c->dens, &c->densT, &c->occfill, &c->Vloc, &c->dnu, &c->dnuT,
                     &c->V3a1, &c->V3b1, &c->V3a2, &c->V3b2, &c->Qt, &c->Bt, &c->accP, &c->qtg, &c->div3b6,
@@ -393,9 +355,10 @@ extern "C" int tcg_set_state(tcg_ctx *c, const tcg_state_desc *st)
     TRY(tcg_set_state_orbitals_only(c, st));
     Host &h = c->h;
     int rc;
-    for (size_t i = 0; i < 4 * (size_t)h.N; i++)
+    for (size_t i = 0; i < 4 * (size_t)h.uN; i++)
         if (!std::isfinite(st->density[i])) return fail(TCG_ERR_NUMERIC, "non-finite density");
-    if ((rc = up(c->dens, st->density, 2 * (size_t)h.N * sizeof(double2), c->stream))) return rc;
+    if ((rc = up(c->udens, st->density, 2 * (size_t)h.uN * sizeof(double2), c->stream))) return rc;
+    TRY(place_state(c));
     rc = c->prec == TCG_PREC_FP64 ? build_occupied<double>(c) : build_occupied<float>(c);
     if (rc) return rc;
     rc = c->prec == TCG_PREC_FP64 ? state_terms<double>(c) : state_terms<float>(c);
@@ -412,6 +375,7 @@ extern "C" int tcg_refresh_state(tcg_ctx *c)
 {
     if (!c) return fail(TCG_ERR_ARG, "null context");
     if (!c->h.have_state) return fail(TCG_ERR_STATE, "no state to refresh");
+    TRY(place_state(c));
     int rc = c->prec == TCG_PREC_FP64 ? build_occupied<double>(c) : build_occupied<float>(c);
     if (rc) return rc;
     rc = c->prec == TCG_PREC_FP64 ? state_terms<double>(c) : state_terms<float>(c);
@@ -552,7 +516,8 @@ extern "C" int tcg_set_forms(tcg_ctx *c, const tcg_forms *f)
     if (!c || !f) return fail(TCG_ERR_ARG, "null argument");
     if (f->xy < 0 || f->xy > 3 || f->z < 0 || f->z > 4 || f->min_targets < 0)
         return fail(TCG_ERR_ARG, "bad kernel form");
-    if (!split_line_grid(c->fast_n) && (f->xy == 3 || f->z >= 3))
+    const int *un = c->h.un;
+    if (!(un[0] == un[1] && un[1] == un[2] && split_line_grid(un[0])) && (f->xy == 3 || f->z >= 3))
         return fail(TCG_ERR_UNSUPPORTED, "split-line kernel forms need a 36^3 or 48^3 grid");
     c->xy_kernels = f->xy;
     c->z_kernels = f->z;
@@ -784,7 +749,19 @@ extern "C" int tcg_density(tcg_ctx *c, const tcg_state_desc *st, double *out)
         TRY(launch(c, k_norms, dim3((unsigned)h.nocc_grids), dim3(256), 0, (int)N, (const double2 *)phi.as<double2>(),
                    (const double2 *)(bitc ? chi.as<double2>() : nullptr), nrm.as<double2>(), bitc ? 1 : 0));
     std::vector<double2> norms(h.nocc_grids);
-    TCG_CUDA(cudaMemcpyAsync(out, dn.p, 2 * N * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
+    const double2 *res = dn.as<double2>();
+    if (h.reduced) {                                   // onto the caller's grid, through G space
+        const size_t uN = h.uN;
+        TRY(c->uwork.ensure(2 * uN * sizeof(double2)));
+        double2 *u = c->uwork.as<double2>();
+        std::vector<void *> gw{dn.as<double2>(), dn.as<double2>() + N}, gu{u, u + uN};
+        TRY((fft3_list<double, -1>(c, gw)));
+        for (int s = 0; s < 2; s++) TRY(to_user_grid(c, dn.as<double2>() + s * N, u + s * uN));
+        TRY((fft3_list<double, +1>(c, gu, &c->ugd)));
+        if (!bitc) TRY(launch(c, k_drop_imag, dim3(148), dim3(256), 0, 2 * uN, u));
+        res = u;
+    }
+    TCG_CUDA(cudaMemcpyAsync(out, res, 2 * (size_t)h.uN * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
     if (h.nocc_grids)
         TCG_CUDA(cudaMemcpyAsync(norms.data(), nrm.p, h.nocc_grids * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
     TCG_CUDA(cudaStreamSynchronize(c->stream));

@@ -58,7 +58,13 @@ struct DBuf {
 
 struct Host {
     // system
-    int n[3] = {0, 0, 0}, N = 0;
+    int un[3] = {0, 0, 0}, uN = 0;          // the caller's FFT grid
+    int n[3] = {0, 0, 0}, N = 0;            // the grid the library works on (workgrid.cuh)
+    int red_n = 0;                          // edge of the smaller work grid this geometry allows (0: none)
+    bool reduced = false;                   // the work grid is red_n^3 instead of the caller's
+    bool hf_wrap = false;                   // pair-density spheres may wrap around the work grid's box (HF)
+    double rmax = 0;                        // largest |k+G| of any plane wave
+    size_t nball = 0;                       // entries of ballmap
     double recip[9], lattice[9], omega = 0;
     int method = 0, nspin = 1, nk = 0, nk_all = 0, num_kpoints = 0;
     std::vector<int> nsym_k, kall_off, ik_of_all, npw;
@@ -69,7 +75,7 @@ struct Host {
     std::vector<int> rotation;              // [nsymop][9]
     std::vector<double> translation;        // [nsymop][3]
     std::vector<size_t> gidx_off;           // [nspin*nk_all] offset in gindex / phase
-    std::vector<int> gidx_host;             // host copy of gindex (pseudopotential set-up)
+    std::vector<int> gidx_host;             // host copy of gindex (on the caller's grid)
     double A[4], F[4];
     bool A_zero = true;
     bool div = false;
@@ -92,10 +98,28 @@ struct Host {
     std::vector<size_t> g0_off;             // [nspin*nk] offset of (s, k) in gidx0
 };
 
-// cubic grid sizes whose pass kernels split each line over several threads
-// (fast::t6::ShapeOf: 36 = 6 x 6, 48 = 4 x 12); only those forms honour
-// pruned transforms
+// cubic grid sizes with compiled pass kernels: split lines (split.cuh) at all of
+// them, one thread or a lane pair per line (fast.cuh) at line_grid's
+#define TCG_FAST_SIZES(X) X(12) X(15) X(16) X(18) X(20) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(45) X(48)
+inline bool fast_grid(int n)
+{
+#define TCG_IS(m) if (n == m) return true;
+    TCG_FAST_SIZES(TCG_IS)
+#undef TCG_IS
+    return false;
+}
+constexpr bool line_grid(int n) { return n == 12 || n == 16 || n == 24 || n == 32 || n == 36 || n == 40 || n == 48; }
+// grids on which tcg_set_forms offers the split-line forms by number
 inline bool split_line_grid(int n) { return n == 36 || n == 48; }
+
+// layout of the pencil table of pruned transforms: bits [nent][n1] u64,
+// counts [nent] int, permutations [nent][n0 n1] u16
+struct PruneTable {
+    size_t nent, np, nact, perm, bytes;
+    explicit PruneTable(const Host &h)
+        : nent((size_t)h.nk * h.nk_all), np((size_t)h.n[0] * h.n[1]), nact(nent * h.n[1] * 8), perm(nact + nent * 4),
+          bytes(perm + nent * np * 2) {}
+};
 
 struct tcg_ctx_impl;
 } // namespace tcg
@@ -107,6 +131,10 @@ struct tcg_ctx {
     tcg::Host h;
     tcg::GridDesc gd;
     // static device data
+    tcg::GridDesc ugd;                      // the caller's grid (gd: the work grid)
+    tcg::DBuf utw64, utw32;
+    tcg::DBuf ballmap;                      // [nball] int2: caller's grid index, work grid index (workgrid.cuh)
+    tcg::DBuf udens, uvloc, uwork;          // density / local pseudopotential / scratch on the caller's grid
     tcg::DBuf tw64, tw32, recip;            // twiddles, reciprocal vectors (9 doubles)
     tcg::DBuf inv;                          // [nspin][nk_all][N] int32
     tcg::DBuf phase;                        // [sum npw] double2
@@ -131,16 +159,15 @@ struct tcg_ctx {
     tcg::DBuf nlD;                          // CSR of D between projector components
     tcg::DBuf acc1, h1buf;                  // one-body accumulators / device copies
     tcg::DBuf gpsi, adjw, adjt;             // energy gradients: occupied block + outputs, pair grids, tables
-    // pruned transforms (36^3 path): per (irreducible k, all-k q) pair, the
+    // pruned transforms: per (irreducible k, all-k q) pair, the
     // (x, y) pencils of the grid that the support of a pair density touches
-    tcg::DBuf prune_tab;                    // masks [nk][nk_all][NP] u8, perms [..][NP] u16, counts [..] i32
+    tcg::DBuf prune_tab;                    // PruneTable
     bool prune_ok = false;                  // table built and usable
     std::vector<int> prune_nact;            // host copy of the table's active-pencil counts
     bool no_prune = false;                  // TCG_NO_PRUNE: full transforms everywhere
-    bool use_sacc = false;                  // TCG_SACC: shared-memory accumulation in the 3a3b6A and fused (2x3A) inverse XY passes
+    bool use_sacc = false;                  // tcg_forms.sacc / .qp_sacc: kept as set, no kernel asks for them
+    bool qp_sacc = true;
     bool no_fuse = false;                   // TCG_NO_FUSE: tc2x and tc3a3b3b4b6 run as separate passes
-    bool qp_sacc = true;                    // TCG_NO_QP_SACC clears: shared-memory accumulation in the
-                                            // occupied-pair inverse XY pass (36^3, FP32)
     tcg::DBuf Qt, Bt;                       // tc3a2a4b2b5 rotated intermediates [nocc_grids][3][N]
     tcg::DBuf accP, qtg;                    // occupied-pair accumulators / gathered q2 grids
     tcg::DBuf div3b6;                       // [nspin][N] fp64 temp_div_3b6 in R space
@@ -149,7 +176,7 @@ struct tcg_ctx {
     tcg::DBuf psi, h2, h3;                  // packed fp64
     tcg::DBuf Rpsi, Rgpsi, acc2, acc3, qsum, tmp, tmp2, aux, items, meta;
     tcg::DBuf rotw, q3b2w, nGw, Ww;           // per-state scratch kept across states (no per-step cudaMalloc / cudaFree)
-    tcg::DBuf ftab;                         // mixed path: FP32 G-space coefficient records of a chunk
+    tcg::DBuf ftab;                         // mixed path: FP32 G-space coefficient planes of a chunk
     tcg::DBuf w3x;                          // [targets][3][N] compute precision: b3 dnu_d psi + b4 qsum_d (3bX input)
     int ftab_nrec = 1;
     int fast_n = 0;                         // cubic grid size with compiled fast kernels (0: generic path)
@@ -167,3 +194,16 @@ struct tcg_ctx {
     struct ProfRec { const void *fn; const char *tag; cudaEvent_t a, b; double bytes; };
     std::vector<ProfRec> prof_recs;
 };
+
+namespace tcg {
+// split-line XY / Z passes in use (the defaults where compiled); sizes without
+// the other forms use them for both or not at all
+inline bool split_form(const tcg_ctx *c, bool xy)
+{
+    const bool fx = c->xy_kernels == 0 || c->xy_kernels == 3, fz = c->z_kernels == 0 || c->z_kernels >= 3;
+    if (!c->fast_n || c->force_generic) return false;
+    return line_grid(c->fast_n) ? (xy ? fx : fz) : (fx && fz);
+}
+inline bool split_xy(const tcg_ctx *c) { return split_form(c, true); }
+inline bool split_z(const tcg_ctx *c) { return split_form(c, false); }
+} // namespace tcg

@@ -31,6 +31,5 @@ template <typename T> using OpTC3BEq = OpTC3B<T, true>;
     TCG_INST(T, OpTC3BEq<T>)           \
     TCG_INST(T, OpTC2X3<T>)            \
     TCG_INST(T, OpTC3X<T>)
-TCG_INST_ALL(float)
-TCG_INST_ALL(double)
+TCG_INST_ALL(TCG_FAST_T)
 } // namespace tcg

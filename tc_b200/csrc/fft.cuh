@@ -14,7 +14,8 @@
 // 1D transforms are self-sorting Stockham, mixed radix {2,3,4,5,8 + generic
 // prime}, ping-ponging between two shared-memory buffers (one barrier per
 // radix stage).  Twiddles are computed in FP64 on the host and staged in
-// shared memory (w[j] = exp(-2 pi i j / n)); the FP32 path rounds them once.
+// shared memory (w[j] = exp(-2 pi i j / n)); the FP32 path rounds them once, to
+// the neighbouring pair of floats whose modulus is closest to 1 (round_twiddle).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -66,14 +67,35 @@ template <typename V, int DIR> __device__ __forceinline__ void dft2(V *v)
     v[0] = cadd(a, b);
     v[1] = csub(a, b);
 }
+// Products with the irrational constants carry the constant's FP32 rounding
+// error (some 2e-8 of it, always of the same sign) as a second term: a transform
+// of a given length would otherwise scale its output by 1 +- 2e-8, and the
+// chains of up to 36 line transforms behind one H psi add these up to more than
+// their random rounding (27^3: gain -2.1e-8 per line transform, 3e-9 with it).
+struct CMul {
+    // x c (+ y d)
+    static __device__ __forceinline__ double mul(double x, double c) { return x * c; }
+    static __device__ __forceinline__ float mul(float x, double c)
+    {
+        const float h = (float)c, l = (float)(c - (double)h);
+        return fmaf(x, h, x * l);
+    }
+    static __device__ __forceinline__ double mul2(double x, double c, double y, double d) { return x * c + y * d; }
+    static __device__ __forceinline__ float mul2(float x, double c, float y, double d)
+    {
+        const float ch = (float)c, cl = (float)(c - (double)ch), dh = (float)d, dl = (float)(d - (double)dh);
+        return fmaf(x, ch, fmaf(y, dh, fmaf(x, cl, y * dl)));
+    }
+};
 template <typename V, int DIR> __device__ __forceinline__ void dft3(V *v)
 {
     using S = decltype(v[0].x);
-    const S h = (S)0.86602540378443864676;   // sin(2 pi / 3)
+    constexpr double h = 0.86602540378443864676;   // sin(2 pi / 3)
     V a = v[0], b = v[1], c = v[2];
     V t1 = cadd(b, c);
     V t2 = {a.x - (S)0.5 * t1.x, a.y - (S)0.5 * t1.y};
-    V t3 = cmuli(cscale(csub(b, c), h), DIR);
+    V d = csub(b, c);
+    V t3 = cmuli(V{CMul::mul(d.x, h), CMul::mul(d.y, h)}, DIR);
     v[0] = cadd(a, t1);
     v[1] = cadd(t2, t3);
     v[2] = csub(t2, t3);
@@ -90,16 +112,18 @@ template <typename V, int DIR> __device__ __forceinline__ void dft4(V *v)
 template <typename V, int DIR> __device__ __forceinline__ void dft5(V *v)
 {
     using S = decltype(v[0].x);
-    const S c1 = (S)0.30901699437494742410, c2 = (S)-0.80901699437494742410;   // cos(2pi/5), cos(4pi/5)
-    const S s1 = (S)0.95105651629515357212, s2 = (S)0.58778525229247312917;    // sin(2pi/5), sin(4pi/5)
+    constexpr double q5 = 0.55901699437494742410;                                // sqrt(5) / 4: cos(2pi/5), cos(4pi/5) = -1/4 +- q5
+    constexpr double s1 = 0.95105651629515357212, s2 = 0.58778525229247312917;   // sin(2pi/5), sin(4pi/5)
     V a = v[0];
     V t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
     V t3 = csub(v[1], v[4]), t4 = csub(v[2], v[3]);
-    V m1 = {a.x + c1 * t1.x + c2 * t2.x, a.y + c1 * t1.y + c2 * t2.y};
-    V m2 = {a.x + c2 * t1.x + c1 * t2.x, a.y + c2 * t1.y + c1 * t2.y};
-    V n1 = cmuli(V{s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y}, DIR);
-    V n2 = cmuli(V{s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y}, DIR);
-    v[0] = cadd(a, cadd(t1, t2));
+    V t = cadd(t1, t2), u = csub(t1, t2);
+    V b = {a.x - (S)0.25 * t.x, a.y - (S)0.25 * t.y};
+    V q = {CMul::mul(u.x, q5), CMul::mul(u.y, q5)};
+    V m1 = cadd(b, q), m2 = csub(b, q);
+    V n1 = cmuli(V{CMul::mul2(t3.x, s1, t4.x, s2), CMul::mul2(t3.y, s1, t4.y, s2)}, DIR);
+    V n2 = cmuli(V{CMul::mul2(t3.x, s2, t4.x, -s1), CMul::mul2(t3.y, s2, t4.y, -s1)}, DIR);
+    v[0] = cadd(a, t);
     v[1] = cadd(m1, n1);
     v[4] = csub(m1, n1);
     v[2] = cadd(m2, n2);
@@ -108,15 +132,15 @@ template <typename V, int DIR> __device__ __forceinline__ void dft5(V *v)
 template <typename V, int DIR> __device__ __forceinline__ void dft8(V *v)
 {
     using S = decltype(v[0].x);
-    const S r = (S)0.70710678118654752440;   // 1/sqrt(2)
+    constexpr double r = 0.70710678118654752440;   // 1/sqrt(2)
     // radix-2 x radix-4 split: even / odd halves
     V e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
     dft4<V, DIR>(e);
     dft4<V, DIR>(o);
     // twiddles w8^k, k = 0..3 : 1, (1 + DIR i) r, DIR i, (-1 + DIR i) r
-    V o1 = {r * (o[1].x - DIR * o[1].y), r * (o[1].y + DIR * o[1].x)};
+    V o1 = {CMul::mul(o[1].x - (S)DIR * o[1].y, r), CMul::mul(o[1].y + (S)DIR * o[1].x, r)};
     V o2 = cmuli(o[2], DIR);
-    V o3 = {r * (-o[3].x - DIR * o[3].y), r * (-o[3].y + DIR * o[3].x)};
+    V o3 = {CMul::mul(-o[3].x - (S)DIR * o[3].y, r), CMul::mul(-o[3].y + (S)DIR * o[3].x, r)};
     v[0] = cadd(e[0], o[0]);
     v[4] = csub(e[0], o[0]);
     v[1] = cadd(e[1], o1);

@@ -160,11 +160,9 @@ static int set_pseudo(tcg_ctx *c, const tcg_pseudo_desc *pp)
             for (int cc = 0; cc < ns; cc++) {
                 const double2 *src = proj + pin + (size_t)(spc_first[is] + cc) * npw;
                 for (int p = 0; p < npw; p++) {
-                    const int gi = h.gidx_host[o + p];
-                    const int m0 = gi % h.n[0], m1 = (gi / h.n[0]) % h.n[1], m2 = gi / (h.n[0] * h.n[1]);
-                    const double mm[3] = {(double)(m0 <= h.n[0] / 2 ? m0 : m0 - h.n[0]),
-                                          (double)(m1 <= h.n[1] / 2 ? m1 : m1 - h.n[1]),
-                                          (double)(m2 <= h.n[2] / 2 ? m2 : m2 - h.n[2])};
+                    int mi[3];
+                    miller_of(h, h.gidx_host[o + p], mi);
+                    const double mm[3] = {(double)mi[0], (double)mi[1], (double)mi[2]};
                     double G[3];
                     for (int d = 0; d < 3; d++)
                         G[d] = h.recip[0 * 3 + d] * mm[0] + h.recip[1 * 3 + d] * mm[1] + h.recip[2 * 3 + d] * mm[2];
@@ -190,9 +188,10 @@ static int set_pseudo(tcg_ctx *c, const tcg_pseudo_desc *pp)
     TRY(up(c->nlD, dbytes.data(), dbytes.size(), c->stream));
     h.have_vloc = pp->vloc != nullptr;
     if (h.have_vloc) {
-        for (int i = 0; i < h.N; i++)
+        for (int i = 0; i < h.uN; i++)
             if (!std::isfinite(pp->vloc[i])) return fail(TCG_ERR_NUMERIC, "non-finite local pseudopotential");
-        TRY(up(c->vloc, pp->vloc, (size_t)h.N * sizeof(double), c->stream));
+        TRY(up(c->uvloc, pp->vloc, (size_t)h.uN * sizeof(double), c->stream));
+        TRY(place_vloc(c));
     }
     TCG_CUDA(cudaStreamSynchronize(c->stream));
     h.have_pseudo = true;

@@ -222,12 +222,15 @@ __global__ void __launch_bounds__(256) k_sphere_z(GridDesc g, const SphereItem *
 }
 
 // In-place XY pass over a list of grids (DIR = +1 backward, -1 forward).
-// Grid pointers of an in-place transform list: a device array, or up to 8
-// pointers passed by value (no upload, no synchronisation for short lists).
+// Grid pointers of an in-place transform list: a device array, evenly spaced
+// grids, or up to 8 pointers passed by value (the last two need no upload and no
+// synchronisation).
 struct GridRefs {
     void *const *dev = nullptr;
+    char *base = nullptr;
+    size_t stride = 0;                       // bytes from grid to grid
     void *inl[8] = {};
-    __device__ void *operator[](int i) const { return dev ? dev[i] : inl[i]; }
+    __device__ void *operator[](int i) const { return base ? base + stride * i : (dev ? dev[i] : inl[i]); }
 };
 
 template <typename T, int DIR>

@@ -3,6 +3,7 @@
 // stage) and the per-apply pipelines.
 #pragma once
 #include "terms.cuh"
+#include "workgrid.cuh"
 
 namespace tcg {
 
@@ -181,49 +182,71 @@ struct Div3b6Item {
     double b6;
 };
 
+// sum over the block (256 threads), the same value in every thread
+__device__ __forceinline__ double2 block_sum256(double2 s)
+{
+    __shared__ double2 part[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    double2 r = part[0];
+#pragma unroll
+    for (int w = 1; w < 8; w++) r = cadd(r, part[w]);
+    return r;
+}
+
+// One CTA per (target, occupied band): the band's factors f b6 (t1 cpi + dot2)
+// (G space) and f b6 cpi (real space), cpi = <chi|psi>, dot2 = <chi|tR|psi>/N.
+// (One CTA per target used to walk its bands in turn: 7 of the 8-atom case's
+// 70 ms, with 96 CTAs of serial sweeps over 48^3 points.)
 template <typename T>
-__global__ void __launch_bounds__(256) k_div3b6(const Div3b6Item *items, int N)
+__global__ void __launch_bounds__(256) k_div3b6_dots(const Div3b6Item *items, int N, int maxocc, double2 *fac)
 {
     using V = typename C2<T>::t;
-    const Div3b6Item it = items[blockIdx.x];
-    __shared__ double2 red[256];
-    const V *Rpsi = (const V *)it.Rpsi;
-    for (int b = 0; b < it.nocc; b++) {
-        const double f = it.fill[b];
-        if (f < 1e-8) continue;
-        const V *chr = (const V *)it.Rchi + (size_t)b * N;
-        const V *phr = (const V *)it.Rphi + (size_t)b * N;
+    const Div3b6Item &it = items[blockIdx.y];
+    const int b = blockIdx.x;
+    if (b >= it.nocc) return;
+    double2 cg = {0, 0}, cr = {0, 0};
+    const double f = it.fill[b];
+    if (!(f < 1e-8)) {
+        const V *Rpsi = (const V *)it.Rpsi, *chr = (const V *)it.Rchi + (size_t)b * N;
         double2 loc = {0, 0};
         for (int p = threadIdx.x; p < it.npw; p += blockDim.x) loc = cadd(loc, cmulc(it.chik[(size_t)b * it.npw + p], it.psi[p]));
-        red[threadIdx.x] = loc;
-        __syncthreads();
-        for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) red[threadIdx.x] = cadd(red[threadIdx.x], red[threadIdx.x + s]);
-            __syncthreads();
-        }
-        const double2 cpi = red[0];
-        __syncthreads();
+        const double2 cpi = block_sum256(loc);
         loc = {0, 0};
         for (int p = threadIdx.x; p < N; p += blockDim.x)
             loc = cadd(loc, cmul(cmulc(to64(chr[p]), to64(Rpsi[p])), it.tR[p]));
-        red[threadIdx.x] = loc;
-        __syncthreads();
-        for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) red[threadIdx.x] = cadd(red[threadIdx.x], red[threadIdx.x + s]);
-            __syncthreads();
+        const double2 dot2 = cscale(block_sum256(loc), 1.0 / (double)N);
+        cg = cadd(cscale(cmul(it.t1, cpi), f * it.b6), cscale(dot2, f * it.b6));
+        cr = cscale(cpi, f * it.b6);
+    }
+    if (threadIdx.x == 0) {
+        double2 *o = fac + ((size_t)blockIdx.y * maxocc + b) * 2;
+        o[0] = cg;
+        o[1] = cr;
+    }
+}
+template <typename T>
+__global__ void __launch_bounds__(256) k_div3b6_add(const Div3b6Item *items, int N, int maxocc, const double2 *fac)
+{
+    using V = typename C2<T>::t;
+    const Div3b6Item &it = items[blockIdx.y];
+    const double2 *fc = fac + (size_t)blockIdx.y * maxocc * 2;
+    const V *phr = (const V *)it.Rphi;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
+        double2 s = {0, 0};
+        for (int b = 0; b < it.nocc; b++) s = cadd(s, cmul(fc[2 * b + 1], to64(phr[(size_t)b * N + p])));
+        acc_add(it.acc + p, cmul(it.tR[p], s), 1.0);
+        if (p < it.npw) {
+            double2 h = it.h[p];
+            for (int b = 0; b < it.nocc; b++) h = cadd(h, cmul(fc[2 * b], it.phik[(size_t)b * it.npw + p]));
+            it.h[p] = h;
         }
-        const double2 dot2 = cscale(red[0], 1.0 / (double)N);
-        __syncthreads();
-        const double2 c1 = cscale(cmul(it.t1, cpi), f * it.b6);
-        const double2 c2 = cscale(dot2, f * it.b6);
-        const double2 *phg = it.phik + (size_t)b * it.npw;
-        for (int p = threadIdx.x; p < it.npw; p += blockDim.x) {
-            double2 hv = cadd(it.h[p], cmul(c1, phg[p]));
-            it.h[p] = cadd(hv, cmul(c2, phg[p]));
-        }
-        const double2 c3 = cscale(cpi, f * it.b6);
-        for (int p = threadIdx.x; p < N; p += blockDim.x) acc_add(it.acc + p, cmul(c3, cmul(it.tR[p], to64(phr[p]))), 1.0);
-        __syncthreads();
     }
 }
 
@@ -234,11 +257,27 @@ struct RotArgs {
     double M[9];
     int tr;
 };
-// scalar: out[idx] += fac * phase * (tr ? conj(in) : in)
-static __global__ void k_rot_scalar(GridDesc g, RotArgs ra, const double2 *in, double2 *out, double fac)
+// One (occupied orbital q2, equivalent k-point) of the rotation stage.
+struct RotItem {
+    RotArgs ra;
+    const double2 *src;      // [nspin + 6][N] G-space intermediates: 3a2 per spin, Q_d, B_d
+    size_t grid;             // its occupied grid
+    double fill;
+};
+// rotated copies of every item (blockIdx.y): scalars S[item][nspin][N],
+//   S[idx] = phase * (tr ? conj(in) : in),
+// and the two vectors R[item][6][N] (Cartesian U^+),
+//   R_d[idx] = +-phase * sum_e M[d][e] (tr ? conj(in_e) : in_e).
+// The whole stage runs over many items per launch (it was some 9 launches per item).
+static __global__ void k_rot(GridDesc g, const RotItem *items, int nspin, double2 *S, double2 *R)
 {
     const double TWOPI = 2.0 * 3.14159265358979323846;
     const int nr[3] = {g.n0, g.n1, g.n2};
+    const size_t N = g.N;
+    const RotItem &it = items[blockIdx.y];
+    const RotArgs &ra = it.ra;
+    double2 *so = S + (size_t)blockIdx.y * nspin * N, *ro = R + (size_t)blockIdx.y * 6 * N;
+    const bool shift = ra.t[0] != 0.0 || ra.t[1] != 0.0 || ra.t[2] != 0.0;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < g.N; p += gridDim.x * blockDim.x) {
         int x, y, z;
         xyz_of(g, p, x, y, z);
@@ -250,86 +289,118 @@ static __global__ void k_rot_scalar(GridDesc g, RotArgs ra, const double2 *in, d
             Gt[i] %= nr[i];
             if (Gt[i] < 0) Gt[i] += nr[i];
         }
-        const double arg = TWOPI * (ra.t[0] * Gt[0] + ra.t[1] * Gt[1] + ra.t[2] * Gt[2]);
-        double sn, cs;
-        sincos(arg, &sn, &cs);
-        const int idx = Gt[0] + Gt[1] * nr[0] + Gt[2] * nr[0] * nr[1];
-        double2 v = in[p];
-        if (ra.tr) v.y = -v.y;
-        const double2 r = cmul(double2{cs, sn}, v);
-        out[idx] = cadd(out[idx], cscale(r, fac));
-    }
-}
-// vector (3 components, Cartesian U^+): out_d[idx] = +-phase * sum_e M[d][e] (tr ? conj(in_e) : in_e)
-static __global__ void k_rot_vec(GridDesc g, RotArgs ra, const double2 *in, double2 *out)
-{
-    const double TWOPI = 2.0 * 3.14159265358979323846;
-    const int nr[3] = {g.n0, g.n1, g.n2};
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < g.N; p += gridDim.x * blockDim.x) {
-        int x, y, z;
-        xyz_of(g, p, x, y, z);
-        const int m[3] = {miller(x, g.n0), miller(y, g.n1), miller(z, g.n2)};
-        int Gt[3];
-        for (int i = 0; i < 3; i++) {
-            Gt[i] = ra.U[0 * 3 + i] * m[0] + ra.U[1 * 3 + i] * m[1] + ra.U[2 * 3 + i] * m[2];
-            if (ra.tr) Gt[i] = -Gt[i];
-            Gt[i] %= nr[i];
-            if (Gt[i] < 0) Gt[i] += nr[i];
-        }
-        const double arg = TWOPI * (ra.t[0] * Gt[0] + ra.t[1] * Gt[1] + ra.t[2] * Gt[2]);
-        double sn, cs;
-        sincos(arg, &sn, &cs);
+        double sn = 0.0, cs = 1.0;
+        if (shift) sincos(TWOPI * (ra.t[0] * Gt[0] + ra.t[1] * Gt[1] + ra.t[2] * Gt[2]), &sn, &cs);
         const double2 ph = {cs, sn};
         const int idx = Gt[0] + Gt[1] * nr[0] + Gt[2] * nr[0] * nr[1];
-        double2 v[3];
-        for (int e = 0; e < 3; e++) {
-            v[e] = in[(size_t)e * g.N + p];
-            if (ra.tr) v[e].y = -v[e].y;
+        for (int s = 0; s < nspin; s++) {
+            double2 v = it.src[(size_t)s * N + p];
+            if (ra.tr) v.y = -v.y;
+            so[(size_t)s * N + idx] = cmul(ph, v);
         }
-        for (int d = 0; d < 3; d++) {
-            double2 s = {0, 0};
-            for (int e = 0; e < 3; e++) s = cadd(s, cscale(v[e], ra.M[d * 3 + e]));
-            s = cmul(ph, s);
-            if (ra.tr) s = cscale(s, -1.0);
-            out[(size_t)d * g.N + idx] = s;
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+            double2 v[3];
+#pragma unroll
+            for (int e = 0; e < 3; e++) {
+                v[e] = it.src[(size_t)(nspin + 3 * w + e) * N + p];
+                if (ra.tr) v[e].y = -v[e].y;
+            }
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                double2 a = {0, 0};
+#pragma unroll
+                for (int e = 0; e < 3; e++) a = cadd(a, cscale(v[e], ra.M[d * 3 + e]));
+                a = cmul(ph, a);
+                if (ra.tr) a = cscale(a, -1.0);
+                ro[(size_t)(3 * w + d) * N + idx] = a;
+            }
         }
     }
 }
-
-// B = -conj(Q) for TC (tc3a2a4b2b5.cpp:662)
-static __global__ void k_negconj(size_t n, const double2 *Q, double2 *B)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        B[i] = {-Q[i].x, Q[i].y};
-}
-
-// qsum3b2[d] += f2 * Bt_d(r) * phi_q2sym(r)  (tc3a2a4b2b5.cpp:811-815)
+// sums over the items in order, one thread per point: V3a2[s] += f S_s (G space),
+// q3b2_d += f B_d(r) phi_q2(r) (tc3a2a4b2b5.cpp:811-815)
 template <typename T>
-__global__ void k_qsum3b2(int N, const double2 *Bt, const typename C2<T>::t *phi, double2 *q, double f2)
+__global__ void k_rot_sums(int N, const RotItem *items, int ni, int nspin, const double2 *S, const double2 *R,
+                           const typename C2<T>::t *Rocc, double2 *V3a2, double2 *q)
 {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x)
-        for (int d = 0; d < 3; d++) acc_add(q + (size_t)d * N + p, cmul(Bt[(size_t)d * N + p], to64(phi[p])), f2);
+    // slot 0 .. nspin - 1: V3a2, nspin .. nspin + 2: q3b2
+    const int slot = blockIdx.y;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
+        double2 *o = slot < nspin ? V3a2 + (size_t)slot * N + p : q + (size_t)(slot - nspin) * N + p;
+        double2 a = *o;
+        for (int i = 0; i < ni; i++) {
+            const double f = items[i].fill;
+            const double2 v = slot < nspin ? S[((size_t)i * nspin + slot) * N + p]
+                                           : cmul(R[((size_t)i * 6 + 3 + slot - nspin) * N + p],
+                                                  to64(Rocc[items[i].grid * N + p]));
+            a = {a.x + f * v.x, a.y + f * v.y};
+        }
+        *o = a;
+    }
+}
+// R-space vectors to compute precision: R[item][0..2] -> Qt[grid], [3..5] -> Bt[grid]
+template <typename T>
+__global__ void k_rot_store(int N, const RotItem *items, const double2 *R, typename C2<T>::t *Qt, typename C2<T>::t *Bt)
+{
+    using V = typename C2<T>::t;
+    const double2 *r = R + (size_t)blockIdx.y * 6 * N;
+    const size_t o = items[blockIdx.y].grid * 3 * N;
+    const int n3 = 3 * N;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n3; p += gridDim.x * blockDim.x) {
+        Qt[o + p] = from64<V>(r[p]);
+        Bt[o + p] = from64<V>(r[n3 + p]);
+    }
 }
 
-// 3a2 divergence correction (tc3a2a4b2b5.cpp:496-573) for one q2 target:
+// B = -conj(Q) for TC (tc3a2a4b2b5.cpp:662), target blockIdx.y of nacc grids each
+static __global__ void k_negconj(int N, int nacc, int nspin, double2 *acc)
+{
+    double2 *Q = acc + ((size_t)blockIdx.y * nacc + nspin) * N, *B = Q + 3 * (size_t)N;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * N; i += gridDim.x * blockDim.x) B[i] = {-Q[i].x, Q[i].y};
+}
+
+// copies of listed grids, blockIdx.y: out[i] = in[idx[i]]
+template <typename V> __global__ void k_pick_grids(int N, const int *idx, const V *in, V *out)
+{
+    const V *s = in + (size_t)idx[blockIdx.y] * N;
+    V *d = out + (size_t)blockIdx.y * N;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) d[i] = s[i];
+}
+
+struct Div3a2Item {
+    size_t pair0;            // first of its ni pair items
+    const double *f1;        // [ni]
+    double dcorr;
+    double2 *Tq;
+    int ni;
+};
+// 3a2 divergence correction (tc3a2a4b2b5.cpp:496-573) for the q2 targets (blockIdx.y):
 // T_xr(0)  -= 4pi A_x (A_x dcorr + u(0; sq, x)) f1 phiphi(0) phij(0)
 // T_xr(G)  -= 4pi A_x f1 u(G; sq, x) (phiphi(G) phij(0) + phiphi(0) phij(G))
 template <typename T>
-__global__ void k_div3a2(GridDesc g, RecipC rc, Jastrow J, int sq, int nspin, int ni, const typename C2<T>::t *pf,
-                         const double *f1, double A0, double A1, double dcorr, double2 *Tq)
+__global__ void k_div3a2(GridDesc g, int tr, RecipC rc, Jastrow J, int sq, int nspin, const Div3a2Item *items, size_t pair0,
+                         const typename C2<T>::t *pairs, double A0, double A1)
 {
+    const Div3a2Item &dt = items[blockIdx.y];
+    const typename C2<T>::t *pf = pairs + (dt.pair0 - pair0) * 2 * g.N;
+    const double *f1 = dt.f1;
+    const double dcorr = dt.dcorr;
+    double2 *Tq = dt.Tq;
+    const int ni = dt.ni;
     using V = typename C2<T>::t;
     const double zero[3] = {0, 0, 0};
     const double FOURPI = 4.0 * 3.14159265358979323846;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < g.N; p += gridDim.x * blockDim.x) {
         int x, y, z;
         xyz_of(g, p, x, y, z);
+        const size_t pt = tr ? (size_t)y + (size_t)g.n1 * (x + (size_t)g.n0 * z) : (size_t)p;   // in the pair grids
         double G[3];
         gvec(rc.R, g, x, y, z, zero, G);
         for (int i1 = 0; i1 < ni; i1++) {
             const V *pp = pf + (size_t)i1 * 2 * g.N;     // [2][N]: phiphi, phij
             const double2 a0 = to64(pp[0]), b0 = to64(pp[g.N]);
-            const double2 ap = to64(pp[p]), bp = to64(pp[g.N + p]);
+            const double2 ap = to64(pp[pt]), bp = to64(pp[g.N + pt]);
             for (int xs = 0; xs < 2; xs++) {
                 const int xr = nspin == 1 ? 0 : xs;
                 const double Ax = xs == 0 ? A0 : A1;
@@ -436,6 +507,7 @@ struct ChunkPlan {
     const double *kq;
     const int *pent;         // [nTB*nSB] pencil-table entry of each (target k, source q) pair
     double pfrac;            // mean active-pencil fraction over the chunk's items
+    int pmax;                // most active pencils of any of its pairs
 };
 
 // Plan (target range x source range) chunks; kq = tcart[tkey] - scart[skey].
@@ -448,7 +520,7 @@ static int plan_chunks(tcg_ctx *c, DBuf &meta, int ntg, const std::vector<int> &
     if (ntg == 0 || nsrc == 0) return TCG_OK;
     int nt_c = std::min(ntg, std::max(1, min_t));
     if ((size_t)nt_c > max_items) nt_c = (int)std::max<size_t>(1, max_items);
-    int ns_c = (int)std::max<size_t>(1, std::min<size_t>(nsrc, max_items / nt_c));
+    int ns_c = (int)std::max<size_t>(1, std::min<size_t>(std::min(nsrc, 64), max_items / nt_c));   // sl::MAXSRC
     // grow the target range if all sources fit
     if (ns_c == nsrc) nt_c = (int)std::min<size_t>(ntg, std::max<size_t>(nt_c, max_items / nsrc));
     std::vector<unsigned char> host;
@@ -499,8 +571,11 @@ static int plan_chunks(tcg_ctx *c, DBuf &meta, int ntg, const std::vector<int> &
             for (int a = 0; a < p.nTB; a++)
                 for (int b = 0; b < p.nSB; b++) pent[(size_t)a * p.nSB + b] = tk[a] * c->h.nk_all + sk[b];
             p.pfrac = 1.0;
+            p.pmax = c->h.n[0] * c->h.n[1];
             if (c->prune_ok) {
                 double sum = 0;
+                p.pmax = 0;
+                for (int e : pent) p.pmax = std::max(p.pmax, c->prune_nact[e]);
                 for (int i = 0; i < p.nt; i++)
                     for (int j = 0; j < p.ns; j++) sum += c->prune_nact[pent[(size_t)tb[i] * p.nSB + sb[j]]];
                 p.pfrac = sum / ((double)p.nt * p.ns * c->h.n[0] * c->h.n[1]);
@@ -547,17 +622,10 @@ static size_t max_items_for(const tcg_ctx *c, int nslots, size_t vbytes)
     return std::min<size_t>(65535, std::max<size_t>(1, budget / per));   // grid.y limit
 }
 
-// Algorithmic bytes per pass launch: a 3D FFT of N points moves 2 N s bytes
-// (one read + one write of the grid); each of the two passes of a
-// transform is credited half of it, N s per grid.
 // Fast-path launcher, defined in fast_launch.cuh and instantiated per grid
 // size in fast_inst.cu (one translation unit per N).
 template <typename T, int N, class Op>
 int run_chunk_fast(tcg_ctx *c, const Op &op, int items, int nt, bool do_xyf, bool do_xyi);
-
-// Algorithmic bytes per pass launch: a 3D FFT of N points moves 2 N s bytes
-// (one read + one write of the grid); each of the two passes of a
-// transform is credited half of it, N s per grid.
 
 // Algorithmic bytes per pass launch: a 3D FFT of N points moves 2 N s bytes
 // (one read + one write of the grid); each of the two passes of a
@@ -567,15 +635,11 @@ static int run_chunk(tcg_ctx *c, const Op &op, int items, int nt, bool do_xyf = 
 {
     using V = typename C2<T>::t;
     const GridDesc &g = c->gd;
-    if (c->fast_n && !c->force_generic) {
+    if (c->fast_n && !c->force_generic && (line_grid(c->fast_n) || (split_xy(c) && split_z(c)))) {
         switch (c->fast_n) {
-        case 12: return run_chunk_fast<T, 12, Op>(c, op, items, nt, do_xyf, do_xyi);
-        case 16: return run_chunk_fast<T, 16, Op>(c, op, items, nt, do_xyf, do_xyi);
-        case 24: return run_chunk_fast<T, 24, Op>(c, op, items, nt, do_xyf, do_xyi);
-        case 32: return run_chunk_fast<T, 32, Op>(c, op, items, nt, do_xyf, do_xyi);
-        case 36: return run_chunk_fast<T, 36, Op>(c, op, items, nt, do_xyf, do_xyi);
-        case 40: return run_chunk_fast<T, 40, Op>(c, op, items, nt, do_xyf, do_xyi);
-        case 48: return run_chunk_fast<T, 48, Op>(c, op, items, nt, do_xyf, do_xyi);
+#define TCG_CASE(n) case n: return run_chunk_fast<T, n, Op>(c, op, items, nt, do_xyf, do_xyi);
+        TCG_FAST_SIZES(TCG_CASE)
+#undef TCG_CASE
         default: break;
         }
     }
@@ -605,48 +669,49 @@ static void op_common(tcg_ctx *c, Op &op, const ChunkPlan &p, int nsl, int ntab)
     op.m.sb = p.sb;
     op.m.kq = p.kq;
     op.m.tab = c->aux.as<double>();
-    op.m.ftab = c->ftab.as<float4>();
+    op.m.ftab = c->ftab.as<float>();
     op.m.nSB = p.nSB;
     op.m.ntab = ntab;
     op.m.nrec = c->ftab_nrec;
-    // pruning: 36^3 or 48^3 grid, table built, split-line Z and inverse XY
-    // passes (k_z_t6 / k_z_t6r read only the active pencils, k_xyi_t6 zeroes
-    // the others; the forward XY pass may write more than the active ones)
+    // pruning: table built, split-line XY and Z passes (the Z pass reads only the
+    // active pencils, the inverse XY pass zeroes the others)
     const int np = c->h.n[0] * c->h.n[1];
     op.m.np = np;
-    op.m.prune = (c->prune_ok && !c->no_prune && split_line_grid(c->fast_n) && !c->force_generic &&
-                  (c->xy_kernels == 0 || c->xy_kernels == 3) && (c->z_kernels == 0 || c->z_kernels >= 3) &&
-                  (Op::BLI | Op::BLO) != 0) ? 1 : 0;
+    op.m.tr = split_xy(c) ? 1 : 0;
+    op.m.prune = (c->prune_ok && !c->no_prune && op.m.tr && split_z(c) && (Op::BLI | Op::BLO) != 0) ? 1 : 0;
     op.m.pent = p.pent;
     op.m.pfrac = op.m.prune ? p.pfrac : 1.0;
-    const size_t nent = (size_t)c->h.nk * c->h.nk_all;
-    op.m.pmask = c->prune_tab.as<const unsigned char>();
-    op.m.pperm = reinterpret_cast<const unsigned short *>(c->prune_tab.as<const unsigned char>() + nent * np);
-    op.m.pnact = reinterpret_cast<const int *>(c->prune_tab.as<const unsigned char>() + nent * np * 3);
-    op.m.pbits = reinterpret_cast<const unsigned long long *>(
-        c->prune_tab.as<const unsigned char>() + ((nent * np * 3 + nent * sizeof(int) + 7) & ~(size_t)7));
+    op.m.pmax = op.m.prune ? p.pmax : np;
+    const PruneTable pt(c->h);
+    const unsigned char *tb = c->prune_tab.as<const unsigned char>();
+    op.m.pperm = reinterpret_cast<const unsigned short *>(tb + pt.perm);
+    op.m.pnact = reinterpret_cast<const int *>(tb + pt.nact);
+    op.m.pbits = reinterpret_cast<const unsigned long long *>(tb);
     memcpy(op.rc.R, c->h.recip, sizeof op.rc.R);
     op.invN = 1.0 / (double)c->h.N;
 }
 
-// Jastrow tables of one chunk: FP64 columns for the FP64 path, FP32
-// coefficient records (nrec per grid point) for the mixed path
+// Jastrow tables of one chunk: FP64 columns for the FP64 path, FP32 coefficient
+// planes for the mixed path (nx: branches x2 carried by TAB_U_SX / TAB_U_QX)
 template <typename T>
-static int gen_tables(tcg_ctx *c, const ChunkPlan &p, int mode, int s, int nrec = 1)
+static int gen_tables(tcg_ctx *c, const ChunkPlan &p, int mode, int s, int nx = 1)
 {
     const int npair = p.nTB * p.nSB;
+    const int tr = split_xy(c) ? 1 : 0;
+    const HFGrid hg{c->h.hf_wrap ? 1 : 0, {c->h.un[0], c->h.un[1], c->h.un[2]}};
     RecipC rc;
     memcpy(rc.R, c->h.recip, sizeof rc.R);
     if constexpr (sizeof(T) == 4) {
-        TRY(c->ftab.ensure((size_t)npair * c->h.N * nrec * sizeof(float4)));
+        const int nrec = mode == TAB_HF ? 1 : (mode == TAB_TC2X ? 4 : 3 * nx);
+        TRY(c->ftab.ensure((size_t)npair * c->h.N * nrec * sizeof(float)));
         c->ftab_nrec = nrec;
-        return launch(c, k_ftables, dim3(148 * 4), dim3(256), 0, c->gd, rc, make_jastrow(c->h), mode, s, nrec, npair,
-                      p.kq, 1.0 / (double)c->h.N, c->ftab.as<float4>());
+        return launch(c, k_ftables, dim3(148 * 4), dim3(256), 0, c->gd, rc, make_jastrow(c->h), mode, tr, hg, s, nrec,
+                      npair, p.kq, 1.0 / (double)c->h.N, c->ftab.as<float>());
     } else {
-        const int ntab = mode == TAB_U_SS ? 1 : 2;
+        const int ntab = mode == TAB_U_SS || mode == TAB_HF ? 1 : 2;
         TRY(c->aux.ensure((size_t)npair * c->h.N * ntab * sizeof(double)));
-        return launch(c, k_tables, dim3(148 * 4), dim3(256), 0, c->gd, rc, make_jastrow(c->h), mode, s, npair, p.kq,
-                      c->aux.as<double>());
+        return launch(c, k_tables, dim3(148 * 4), dim3(256), 0, c->gd, rc, make_jastrow(c->h), mode, tr, hg, s, npair, p.kq,
+                      1.0 / (double)c->h.N, c->aux.as<double>());
     }
 }
 
@@ -824,8 +889,9 @@ static int run_hf2x(tcg_ctx *c, const Targets &Tg, double2 *acc)
                         max_items_for(c, 1, sizeof(V)), min_targets(c), plan));
         for (const ChunkPlan &p : plan) {
             TRY(c->tmp.ensure((size_t)p.nt * p.ns * N * sizeof(V)));
+            TRY(gen_tables<T>(c, p, TAB_HF, s));
             OpHF2X<T> op;
-            op_common<T>(c, op, p, 1, 0);
+            op_common<T>(c, op, p, 1, 1);
             op.Rpsi = c->Rpsi.as<V>() + (size_t)(TR.t0 + p.t0) * N;
             op.Rocc = c->Rocc.as<V>() + (S.base + p.s0) * N;
             op.acc = acc + (size_t)(TR.t0 + p.t0) * N;
@@ -902,8 +968,6 @@ static int tc3_stage_ab(tcg_ctx *c, const Targets &Tg, const TRange &TR, const S
         a.tmp2 = c->tmp2.as<V>();
         a.s = s;
         a.b3 = b3;
-        a.sacc_on = c->use_sacc ? 1 : 0;
-        a.sacc_n = OA::SACC;
         TRY((run_chunk<T, OA>(c, a, (int)items, p.nt)));
         OB b;
         op_common<T>(c, b, p, nsl, 2);
@@ -964,13 +1028,16 @@ static int tc2x_tc3_stage_ab(tcg_ctx *c, const TRange &TR, const Sources &S, int
         x.Qt = c->Qt.as<V>() + (S.base + p.s0) * 3 * N;
         x.acc3 = acc + (size_t)(TR.t0 + p.t0) * N;
         x.fa4 = band_fa4(h);
-        x.sacc_on = c->use_sacc ? 1 : 0;
-        x.sacc_n = band ? 4 : 3;
         TRY((run_chunk<T, OX>(c, x, (int)items, p.nt)));
-        // 3b6B reads du from 3a3b6A's table layout (TAB_U_SX, one record for equal channels)
-        TRY(gen_tables<T>(c, p, TAB_U_SX, s, 1));
         OB b;
         op_common<T>(c, b, p, nsl, 2);
+        if (split_z(c)) {               // du stands in tc2x's tables too (planes 1-3, column u)
+            b.c0 = 1;
+            b.col = 1;
+        } else {
+            TRY(gen_tables<T>(c, p, TAB_U_SX, s, 1));
+            op_common<T>(c, b, p, nsl, 2);
+        }
         b.Rocc = x.Rocc;
         b.acc = acc + (size_t)(TR.t0 + p.t0) * N;
         b.tmp2 = x.tmp2;
@@ -1051,9 +1118,20 @@ static int run_tc3a3b3b4b6(tcg_ctx *c, const Targets &Tg, const ApplyArgs &A, do
                 it.b6 = b6;
                 di.push_back(it);
             }
-            TRY(c->items.ensure(di.size() * sizeof(Div3b6Item)));
-            TCG_CUDA(cudaMemcpyAsync(c->items.p, di.data(), di.size() * sizeof(Div3b6Item), cudaMemcpyHostToDevice, c->stream));
-            TRY(launch(c, k_div3b6<T>, dim3((unsigned)di.size()), dim3(256), 0, (const Div3b6Item *)c->items.p, (int)N));
+            int maxocc = 0;
+            for (const Div3b6Item &it : di) maxocc = std::max(maxocc, it.nocc);
+            const size_t nd = di.size(), ib = (nd * sizeof(Div3b6Item) + 15) / 16 * 16;
+            TRY(c->items.ensure(ib + nd * maxocc * 2 * sizeof(double2)));
+            double2 *fac = reinterpret_cast<double2 *>(c->items.as<char>() + ib);
+            TCG_CUDA(cudaMemcpyAsync(c->items.p, di.data(), nd * sizeof(Div3b6Item), cudaMemcpyHostToDevice, c->stream));
+            for (size_t d0 = 0; d0 < nd && maxocc; d0 += 65535) {
+                const unsigned nb = (unsigned)std::min<size_t>(65535, nd - d0);
+                const Div3b6Item *it = c->items.as<Div3b6Item>() + d0;
+                double2 *fd = fac + d0 * maxocc * 2;
+                TRY(launch(c, k_div3b6_dots<T>, dim3(maxocc, nb), dim3(256), 0, it, (int)N, maxocc, fd));
+                TRY(launch(c, k_div3b6_add<T>, dim3((unsigned)std::min<size_t>(32, (N + 255) / 256), nb), dim3(256), 0, it,
+                           (int)N, maxocc, (const double2 *)fd));
+            }
             TCG_CUDA(cudaStreamSynchronize(c->stream));
         }
         // stage C: 3b4 (:651-770); after the fused first stage also 3b3 and,
@@ -1132,10 +1210,6 @@ static int qp_pairs(tcg_ctx *c, int sq, int ntq, const std::vector<int> &tkey, c
         op.nacc = nacc;
         op.nspin = h.nspin;
         op.sq = sq;
-        // the chunk's sources summed in FP32 shared-memory planes, one FP64
-        // red.add per accumulator point at the end (in place of one per source)
-        op.sacc_on = c->qp_sacc ? 1 : 0;
-        op.sacc_n = nacc;
         TRY((run_chunk<T, OQ>(c, op, (int)items, p.nt)));
     }
     return TCG_OK;
@@ -1204,15 +1278,17 @@ static int qp_partial(tcg_ctx *c, int rank, int nranks)
         Sources S = sources_of(c, sq);
         const int nsrc = (int)S.key.size();
         const int lo = (int)((int64_t)nsrc * rank / nranks), hi = (int)((int64_t)nsrc * (rank + 1) / nranks);
-        // target grids are not contiguous in Rocc (isym > 0 grids in between):
+        // target grids need not be contiguous in Rocc (isym > 0 grids in between):
         // gather them into a contiguous copy
         TRY(c->qtg.ensure((size_t)ntq * 2 * N * sizeof(V)));
-        for (int i = 0; i < ntq; i++) {
-            TCG_CUDA(cudaMemcpyAsync(c->qtg.as<V>() + (size_t)i * N, c->Rocc.as<V>() + (size_t)Q.grid[i] * N,
-                                     N * sizeof(V), cudaMemcpyDeviceToDevice, c->stream));
-            const V *chsrc = bitc ? c->Rchi.as<V>() : c->Rocc.as<V>();
-            TCG_CUDA(cudaMemcpyAsync(c->qtg.as<V>() + (size_t)(ntq + i) * N, chsrc + (size_t)Q.grid[i] * N,
-                                     N * sizeof(V), cudaMemcpyDeviceToDevice, c->stream));
+        TRY(c->items.ensure(ntq * sizeof(int)));
+        TCG_CUDA(cudaMemcpyAsync(c->items.p, Q.grid.data(), ntq * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+        for (int i0 = 0; i0 < ntq; i0 += 65535) {
+            const unsigned nb = (unsigned)std::min(65535, ntq - i0);
+            for (int w = 0; w < (bitc ? 2 : 1); w++)
+                TRY(launch(c, k_pick_grids<V>, dim3((unsigned)std::min<size_t>(16, (N + 255) / 256), nb), dim3(256), 0, (int)N,
+                           (const int *)(c->items.as<int>() + i0), (const V *)(w ? c->Rchi.as<V>() : c->Rocc.as<V>()),
+                           c->qtg.as<V>() + (size_t)(w * ntq + i0) * N));
         }
         double2 *accP = c->accP.as<double2>() + aoff[sq] * N;
         const bool eqq = h.A[sq * 2 + 0] == h.A[sq * 2 + 1] && h.F[sq * 2 + 0] == h.F[sq * 2 + 1];
@@ -1252,8 +1328,11 @@ static int qp_finish(tcg_ctx *c)
     TRY(c->V3b2.ensure((size_t)ns * N * sizeof(double2)));
     TRY(launch(c, k_zero, dim3(pblocks), dim3(256), 0, c->V3a2.as<double2>(), (size_t)ns * N));
     TRY(launch(c, k_zero, dim3(pblocks), dim3(256), 0, c->V3b2.as<double2>(), (size_t)ns * N));
-    DBuf &rot = c->rotw;              // fp64 work: 6 grids
-    TRY(rot.ensure(6 * N * sizeof(double2)));
+    // fp64 work of the rotations: 6 + nspin grids per item, at most 1 GiB (as far as one item fits)
+    const size_t per = (size_t)(6 + ns) * N * sizeof(double2);
+    const size_t ng = std::max<size_t>(1, std::min<size_t>({h.nocc_grids, ((size_t)1 << 30) / per, (size_t)65535}));
+    DBuf &rot = c->rotw;
+    TRY(rot.ensure(ng * per));
     DBuf &q3b2 = c->q3b2w;
     TRY(q3b2.ensure(3 * N * sizeof(double2)));
     for (int sq = 0; sq < ns; sq++) {
@@ -1265,36 +1344,32 @@ static int qp_finish(tcg_ctx *c)
         double2 *accP = c->accP.as<double2>() + aoff[sq] * N;
         // B = -conj(Q) for TC, then forward FFTs of all accumulators
         if (!bitc)
-            for (int i = 0; i < ntq; i++)
-                TRY(launch(c, k_negconj, dim3(pblocks), dim3(256), 0, 3 * N,
-                           (const double2 *)(accP + ((size_t)i * nacc + ns) * N), accP + ((size_t)i * nacc + ns + 3) * N));
-        {
-            std::vector<void *> grids;
-            for (int i = 0; i < ntq; i++)
-                for (int sl = 0; sl < nacc; sl++) grids.push_back(accP + ((size_t)i * nacc + sl) * N);
-            TRY((fft3_list<double, -1>(c, grids)));
-        }
-        // 3a2 divergence correction: pair transforms at q1 = q2 (:496-573)
+            for (int i0 = 0; i0 < ntq; i0 += 65535)
+                TRY(launch(c, k_negconj, dim3(pblocks, (unsigned)std::min(65535, ntq - i0)), dim3(256), 0, (int)N, nacc, ns,
+                           accP + (size_t)i0 * nacc * N));
+        TRY((fft3_strided<double, -1>(c, accP, (size_t)ntq * nacc)));
+        // 3a2 divergence correction: pair transforms at q1 = q2 (:496-573), the
+        // targets of as many k-points at a time as the chunk budget holds
         if (h.div && !h.A_zero) {
-            for (int iq2 = 0; iq2 < h.nk; iq2++) {
-                const int no = h.nocc[sq * h.nk + iq2];
-                if (no == 0) continue;
-                const size_t g0 = h.occ_off[(size_t)sq * h.nk_all + h.kall_off[iq2]];
-                const int items = no * no;
-                std::vector<int> idx(4 * (size_t)items);
-                for (int i2 = 0; i2 < no; i2++)
-                    for (int i1 = 0; i1 < no; i1++) {
-                        const int it = i2 * no + i1;
-                        idx[0 * items + it] = (int)(g0 + i1);   // chi_q1 (bra of phiphi)
-                        idx[1 * items + it] = (int)(g0 + i2);   // phi_q2
-                        idx[2 * items + it] = (int)(g0 + i2);   // chi_q2 (bra of phij)
-                        idx[3 * items + it] = (int)(g0 + i1);   // phi_q1
-                    }
-                TRY(c->aux.ensure(idx.size() * sizeof(int)));
-                TCG_CUDA(cudaMemcpyAsync(c->aux.p, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-                TRY(c->tmp.ensure((size_t)items * 2 * N * sizeof(V)));
+            const size_t maxp = max_items_for(c, 2, sizeof(V));
+            std::vector<Div3a2Item> dv;
+            std::vector<int> idx[4];
+            size_t base0 = 0;              // first pair of the pending batch
+            int t0 = 0;                    // first target of the pending batch
+            auto flush = [&]() -> int {
+                const size_t np = idx[0].size();
+                if (np == 0) return TCG_OK;
+                const size_t ob = (np * 4 * sizeof(int) + 15) / 16 * 16;
+                TRY(c->aux.ensure(ob + dv.size() * sizeof(Div3a2Item)));
+                for (int q = 0; q < 4; q++)
+                    TCG_CUDA(cudaMemcpyAsync(c->aux.as<int>() + q * np, idx[q].data(), np * sizeof(int), cudaMemcpyHostToDevice,
+                                             c->stream));
+                Div3a2Item *dd = reinterpret_cast<Div3a2Item *>(c->aux.as<char>() + ob);
+                TCG_CUDA(cudaMemcpyAsync(dd, dv.data(), dv.size() * sizeof(Div3a2Item), cudaMemcpyHostToDevice, c->stream));
+                TRY(c->tmp.ensure(np * 2 * N * sizeof(V)));
                 OpPairFwd<T> op;
                 op.m = ChunkMeta{};
+                op.m.tr = split_xy(c) ? 1 : 0;
                 op.g = g;
                 op.tmp = c->tmp.as<V>();
                 op.nsl = 2;
@@ -1304,37 +1379,54 @@ static int qp_finish(tcg_ctx *c)
                 const V *chi = bitc ? c->Rchi.as<V>() : c->Rocc.as<V>();
                 op.A0 = chi; op.B0 = c->Rocc.as<V>(); op.A1 = chi; op.B1 = c->Rocc.as<V>();
                 op.ia0 = c->aux.as<int>();
-                op.ib0 = op.ia0 + items;
-                op.ia1 = op.ia0 + 2 * items;
-                op.ib1 = op.ia0 + 3 * items;
-                TRY((run_chunk<T, OpPairFwd<T>>(c, op, items, 0, true, false)));
+                op.ib0 = op.ia0 + np;
+                op.ia1 = op.ia0 + 2 * np;
+                op.ib1 = op.ia0 + 3 * np;
+                TRY((run_chunk<T, OpPairFwd<T>>(c, op, (int)np, 0, true, false)));
+                for (size_t i0 = 0; i0 < dv.size(); i0 += 65535)
+                    TRY(launch(c, k_div3a2<T>, dim3((unsigned)std::min<size_t>(32, (N + 255) / 256), (unsigned)std::min<size_t>(65535, dv.size() - i0)),
+                               dim3(256), 0, g, op.m.tr, rc, J, sq, ns, (const Div3a2Item *)(dd + i0), base0,
+                               (const V *)c->tmp.as<V>(), h.A[sq * 2 + 0], h.A[sq * 2 + 1]));
+                TCG_CUDA(cudaStreamSynchronize(c->stream));
+                base0 += np;
+                t0 += (int)dv.size();
+                dv.clear();
+                for (auto &v : idx) v.clear();
+                return TCG_OK;
+            };
+            size_t pair = 0;
+            for (int iq2 = 0; iq2 < h.nk; iq2++) {
+                const int no = h.nocc[sq * h.nk + iq2];
+                const size_t g0 = h.occ_off[(size_t)sq * h.nk_all + h.kall_off[iq2]];
                 const double dcorr = 1.0 / std::sqrt(PI_D * h.alpha) * Nk * Om - h.sum_vaux[iq2];
                 for (int i2 = 0; i2 < no; i2++) {
-                    int tq = -1;
-                    for (int i = 0; i < ntq; i++)
-                        if (tgrid[i] == (int)(g0 + i2)) tq = i;
-                    TRY(launch(c, k_div3a2<T>, dim3(pblocks), dim3(256), 0, g, rc, J, sq, ns, no,
-                               (const V *)(c->tmp.as<V>() + (size_t)i2 * no * 2 * N),
-                               c->occfill.as<double>() + g0, h.A[sq * 2 + 0], h.A[sq * 2 + 1], dcorr,
-                               accP + (size_t)tq * nacc * N));
+                    if (!dv.empty() && idx[0].size() + no > maxp) TRY(flush());
+                    Div3a2Item it;
+                    it.pair0 = pair;
+                    it.f1 = c->occfill.as<double>() + g0;
+                    it.dcorr = dcorr;
+                    it.Tq = accP + (size_t)(t0 + dv.size()) * nacc * N;   // targets come in this order (qp_targets)
+                    it.ni = no;
+                    dv.push_back(it);
+                    for (int i1 = 0; i1 < no; i1++, pair++) {
+                        idx[0].push_back((int)(g0 + i1));   // chi_q1 (bra of phiphi)
+                        idx[1].push_back((int)(g0 + i2));   // phi_q2
+                        idx[2].push_back((int)(g0 + i2));   // chi_q2 (bra of phij)
+                        idx[3].push_back((int)(g0 + i1));   // phi_q1
+                    }
                 }
-                TCG_CUDA(cudaStreamSynchronize(c->stream));
             }
+            TRY(flush());
         }
         // rotations to every equivalent q2, 3a2 / 3b2 accumulation, Qt / Bt (:576-644, :668-817)
-        std::vector<double> hfill((size_t)ntq);
+        std::vector<RotItem> items;
         for (int i = 0; i < ntq; i++) {
             const int iq2 = tkey[i];
             const int i2 = tgrid[i] - (int)h.occ_off[(size_t)sq * h.nk_all + h.kall_off[iq2]];
-            hfill[i] = h.filling[fill_off(h, sq, iq2) + i2];
-        }
-        for (int i = 0; i < ntq; i++) {
-            const int iq2 = tkey[i];
-            const int i2 = tgrid[i] - (int)h.occ_off[(size_t)sq * h.nk_all + h.kall_off[iq2]];
-            const double f2 = hfill[i];
             for (int isym = 0; isym < h.nsym_k[iq2]; isym++) {
                 const int a2 = h.kall_off[iq2] + isym;
-                RotArgs ra;
+                RotItem it{};
+                RotArgs &ra = it.ra;
                 const int *U = &h.rotation[9 * h.rot_index[a2]];
                 memcpy(ra.U, U, sizeof ra.U);
                 memcpy(ra.t, &h.translation[3 * h.rot_index[a2]], sizeof ra.t);
@@ -1353,25 +1445,28 @@ static int qp_finish(tcg_ctx *c)
                         for (int k = 0; k < 3; k++) s_ += T1[r * 3 + k] * h.lattice[k * 3 + q];
                         ra.M[r * 3 + q] = s_ / (2 * PI_D);
                     }
-                for (int s = 0; s < ns; s++)
-                    TRY(launch(c, k_rot_scalar, dim3(pblocks), dim3(256), 0, g, ra,
-                               (const double2 *)(accP + ((size_t)i * nacc + s) * N), c->V3a2.as<double2>() + (size_t)s * N, f2));
-                double2 *R = rot.as<double2>();
-                TRY(launch(c, k_rot_vec, dim3(pblocks), dim3(256), 0, g, ra,
-                           (const double2 *)(accP + ((size_t)i * nacc + ns) * N), R));
-                TRY(launch(c, k_rot_vec, dim3(pblocks), dim3(256), 0, g, ra,
-                           (const double2 *)(accP + ((size_t)i * nacc + ns + 3) * N), R + 3 * N));
-                std::vector<void *> grids;
-                for (int d = 0; d < 6; d++) grids.push_back(R + (size_t)d * N);
-                TRY((fft3_list<double, +1>(c, grids)));
-                const size_t gq = h.occ_off[(size_t)sq * h.nk_all + a2] + i2;
-                TRY(launch(c, k_qsum3b2<T>, dim3(pblocks), dim3(256), 0, (int)N, (const double2 *)(R + 3 * N),
-                           (const V *)(c->Rocc.as<V>() + gq * N), q3b2.as<double2>(), f2));
-                TRY(launch(c, k_to_prec<T>, dim3(pblocks), dim3(256), 0, (const double2 *)R, c->Qt.as<V>() + gq * 3 * N, 3 * N));
-                TRY(launch(c, k_to_prec<T>, dim3(pblocks), dim3(256), 0, (const double2 *)(R + 3 * N),
-                           c->Bt.as<V>() + gq * 3 * N, 3 * N));
+                it.src = accP + (size_t)i * nacc * N;
+                it.grid = h.occ_off[(size_t)sq * h.nk_all + a2] + i2;
+                it.fill = h.filling[fill_off(h, sq, iq2) + i2];
+                items.push_back(it);
             }
         }
+        TRY(c->items.ensure(items.size() * sizeof(RotItem)));
+        TCG_CUDA(cudaMemcpyAsync(c->items.p, items.data(), items.size() * sizeof(RotItem), cudaMemcpyHostToDevice, c->stream));
+        for (size_t i0 = 0; i0 < items.size(); i0 += ng) {
+            const size_t n = std::min(ng, items.size() - i0);
+            const RotItem *dit = c->items.as<RotItem>() + i0;
+            double2 *R = rot.as<double2>(), *S = R + ng * 6 * N;
+            const unsigned gx = (unsigned)std::min<size_t>(64, (N + 255) / 256);
+            TRY(launch(c, k_rot, dim3(gx, (unsigned)n), dim3(256), 0, g, dit, ns, S, R));
+            TRY((fft3_strided<double, +1>(c, R, 6 * n)));
+            TRY(launch(c, k_rot_sums<T>, dim3((unsigned)std::min<size_t>(148 * 4, (N + 255) / 256), ns + 3), dim3(256), 0, (int)N,
+                       dit, (int)n, ns, (const double2 *)S, (const double2 *)R, (const V *)c->Rocc.as<V>(),
+                       c->V3a2.as<double2>(), q3b2.as<double2>()));
+            TRY(launch(c, k_rot_store<T>, dim3(gx, (unsigned)n), dim3(256), 0, (int)N, dit, (const double2 *)R,
+                       c->Qt.as<V>(), c->Bt.as<V>()));
+        }
+        TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->items is reused below
         // 3b2 local potential (:922-958): V3b2[s](r) += IFFT[ sum_d G_d u' FFT(qsum3b2_d) ]
         {
             std::vector<void *> grids;
@@ -1508,15 +1603,26 @@ static int state_terms(tcg_ctx *c)
     memcpy(rc.R, h.recip, sizeof rc.R);
     const unsigned pblocks = (unsigned)std::min<size_t>(148 * 8, (N + 255) / 256);
     if (h.method == TCG_METHOD_HF) {
-        // Hartree potential of hf2h (calc_hamiltonian_hf2h.cpp:40-51)
-        TRY(c->VH.ensure(N * sizeof(double2)));
-        TRY(launch(c, k_zero, dim3(pblocks), dim3(256), 0, c->VH.as<double2>(), N));
-        TRY(launch(c, k_add, dim3(pblocks), dim3(256), 0, N, (const double2 *)c->dens.as<double2>(), c->VH.as<double2>()));
-        TRY(launch(c, k_add, dim3(pblocks), dim3(256), 0, N, (const double2 *)(c->dens.as<double2>() + N),
-                   c->VH.as<double2>()));
-        std::vector<void *> gv{c->VH.p};
-        TRY((fft3_list<double, -1>(c, gv)));
-        TRY(launch(c, k_hartree_g, dim3(pblocks), dim3(256), 0, g, rc, c->VH.as<double2>()));
+        // Hartree potential of hf2h (calc_hamiltonian_hf2h.cpp:40-51), formed on
+        // the caller's grid; a smaller work grid takes its components G - G' of
+        // plane-wave pairs, all that V psi on the sphere sees
+        const size_t uN = h.uN;
+        TRY(c->VH.ensure(std::max(N, uN) * sizeof(double2)));
+        double2 *vu = c->VH.as<double2>();
+        if (h.reduced) {
+            TRY(c->uwork.ensure(uN * sizeof(double2)));
+            vu = c->uwork.as<double2>();
+        }
+        TRY(launch(c, k_zero, dim3(pblocks), dim3(256), 0, vu, uN));
+        TRY(launch(c, k_add, dim3(pblocks), dim3(256), 0, uN, (const double2 *)c->udens.as<double2>(), vu));
+        TRY(launch(c, k_add, dim3(pblocks), dim3(256), 0, uN, (const double2 *)(c->udens.as<double2>() + uN), vu));
+        std::vector<void *> gv{vu};
+        TRY((fft3_list<double, -1>(c, gv, &c->ugd)));
+        TRY(launch(c, k_hartree_g, dim3(pblocks), dim3(256), 0, c->ugd, rc, vu));
+        if (h.reduced) {
+            TRY(to_work_grid(c, vu, c->VH.as<double2>()));
+            gv[0] = c->VH.p;
+        }
         TRY((fft3_list<double, +1>(c, gv)));
         TCG_CUDA(cudaStreamSynchronize(c->stream));
         return TCG_OK;

@@ -102,10 +102,10 @@ static int sphere_to_r(tcg_ctx *c, const std::vector<SphereItem> &items)
 
 // In-place full 3D FFT of a list of grids (DIR -1: forward with 1/N).
 template <typename T, int DIR>
-static int fft3_list(tcg_ctx *c, const std::vector<void *> &grids)
+static int fft3_list(tcg_ctx *c, const std::vector<void *> &grids, const GridDesc *on = nullptr)
 {
     using V = typename C2<T>::t;
-    const GridDesc &g = c->gd;
+    const GridDesc &g = on ? *on : c->gd;
     if (grids.empty()) return TCG_OK;
     const size_t n = grids.size();
     const int ntiles = (g.n0 * g.n1 + ZTC - 1) / ZTC;
@@ -127,6 +127,25 @@ static int fft3_list(tcg_ctx *c, const std::vector<void *> &grids)
         TRY(launch(c, k_z_inplace<T, DIR>, dim3(ntiles, nb), dim3(256), smem_z<V>(g, 0), g, gr, scale));
     }
     TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->items is reused by the next caller
+    return TCG_OK;
+}
+
+// The same for n evenly spaced grids of N points.
+template <typename T, int DIR>
+static int fft3_strided(tcg_ctx *c, typename C2<T>::t *first, size_t n)
+{
+    using V = typename C2<T>::t;
+    const GridDesc &g = c->gd;
+    const int ntiles = (g.n0 * g.n1 + ZTC - 1) / ZTC;
+    const double scale = DIR < 0 ? 1.0 / (double)g.N : 1.0;
+    for (size_t b0 = 0; b0 < n; b0 += 65535) {
+        const unsigned nb = (unsigned)std::min<size_t>(65535, n - b0);
+        GridRefs gr;
+        gr.base = reinterpret_cast<char *>(first + b0 * g.N);
+        gr.stride = (size_t)g.N * sizeof(V);
+        TRY(launch(c, k_xy_inplace<T, DIR>, dim3(g.n2, nb), dim3(256), smem_xy<V>(g), g, gr));
+        TRY(launch(c, k_z_inplace<T, DIR>, dim3(ntiles, nb), dim3(256), smem_z<V>(g, 0), g, gr, scale));
+    }
     return TCG_OK;
 }
 
@@ -168,19 +187,21 @@ struct ChunkMeta {
     const int *sb;          // [ns]
     const double *kq;       // [nTB*nSB][3]
     const double *tab;      // [nTB*nSB][N][ntab]            (FP64 path)
-    const float4 *ftab;     // [nTB*nSB][N][nrec] coefficients (mixed path)
+    const float *ftab;      // [nTB*nSB][nrec][N] coefficients (mixed path), one plane per component
     int nSB, ntab, nrec;
-    // pruning of band-limited grids (prune != 0): per pair its entry in the
-    // context's pencil table; pmask[entry][x + n0 y] = 1 where the pair
-    // density's support meets pencil (x, y); pperm lists the active pencils
-    // first, pnact counts them
+    // G-side planes y fastest (split-line XY passes, split.cuh): grids between
+    // the XY and Z passes and the coefficient tables
+    int tr;
+    // pruning (prune != 0): per pair its entry in the context's pencil table of
+    // the pencils (x, y) that the ball |G + k - q| < R_k + R_q meets; pperm lists
+    // the active pencils y + n1 x first, pnact counts them
     const int *pent;        // [nTB*nSB]
-    const unsigned char *pmask;
     const unsigned short *pperm;
     const int *pnact;
-    const unsigned long long *pbits;   // [entry][x]: bit y set where pencil (x, y) is active
+    const unsigned long long *pbits;   // [entry][y]: bit x set where pencil (x, y) is active
     int np, prune;
     double pfrac;           // mean active-pencil fraction of the chunk's items (host accounting)
+    int pmax;               // most active pencils of its pairs (host: Z-pass grid)
 };
 
 template <typename T>
@@ -194,23 +215,6 @@ struct OpBase {
     // 36^3 once the plane copies were made division-free) or lines split over
     // lane pairs (half the registers, one shuffle per element)
     static constexpr bool XYF_PAIR = false, XYI_PAIR = false;
-    // forward XY pass in split lines by default also in FP32 where a whole
-    // line per thread spills (48^3)
-    static constexpr bool XYF_SPLIT48 = false;
-    // split-line inverse XY pass at 36^3: resident CTAs per SM beyond the
-    // default four (a register cap the op's work fits without spilling)
-    static constexpr int XYI_MINB_EXTRA = 0;
-    // the same for the register-resident split-line Z pass (k_z_t6r)
-    static constexpr int ZR_MINB_EXTRA = 0;
-    // split-line Z pass in shared memory (k_z_t6): the input plane that holds
-    // the inverse transform of each output, valid when every output after the
-    // first reads input 0 only in zmix (-1: a plane of its own)
-    static constexpr int ZO_ALIAS = -1;
-    static constexpr int Z_MINB_EXTRA = 0;    // k_z_t6 as XYI_MINB_EXTRA
-    // split-line Z pass (36^3, 48^3): transformed inputs kept in registers
-    // (one exchange per transform, fewer resident CTAs); measured faster for
-    // three inputs
-    static constexpr bool ZREG = false;
     GridDesc g;
     V *tmp;
     int nsl;                // tmp slots per item
@@ -240,45 +244,66 @@ struct OpBase {
     // xyi_extra(tj, item, b, p, v) (other accumulators of the op)
     static constexpr bool RACC_EXTRA = false;
     __device__ void xyi_extra(int, int, int, size_t, const V *) const {}
-    // split-line inverse XY pass (k_xyi_t6), FP32: SACC > 0 accumulates the chunk's
-    // sources in SACC shared-memory planes per CTA (xyi_sterm picks the slot
-    // of output b, -1 for none) and adds them to the FP64 accumulators once
-    // at the end (xyi_sflush), instead of one FP64 red.add per source
-    static constexpr int SACC = 0;           // most slots an op uses (compile-time bound)
-    int sacc_on = 0;                         // runtime switch of the SACC path
-    int sacc_n = 0;                          // slots in use when on (<= SACC; sizes the shared memory)
-    __device__ int xyi_slot(int) const { return -1; }
-    __device__ V xyi_sterm(int, int, int, size_t, V v) const { return v; }
-    __device__ void xyi_sflush(int, int, size_t, V) const {}
-    // SACC_GROUP: the op defines xyi_sgroup(tj, item, b0, p, vals[GS], add),
-    // the contributions of an output group to the slots (add(slot, value));
-    // otherwise output b0 goes to slot xyi_slot(b0) as xyi_sterm (sacc_group)
-    static constexpr bool SACC_GROUP = false;
+    // ---- split-line passes (split.cuh)
+    // Inverse XY: the sums over the sources that an output group feeds, at most
+    // NACC of them, made with at most NOPS operand grids of the source
+    // (xyi_operand(k, b0, si), null where unused): xyi_add(si, b0, vals[GS], o,
+    // add) calls add(slot, value) for the group b0's contributions at a point,
+    // xyi_put(tj, b0, slot, p, sum) adds a finished sum to its accumulator.
+    static constexpr int NACC = 1, NOPS = 1;
+    __device__ const V *xyi_operand(int, int, int) const { return nullptr; }
+    template <class F> __device__ void xyi_add(int, int, const V *, const V *, F &&) const {}
+    __device__ void xyi_put(int, int, int, size_t, V) const {}
+    // Forward XY: operands that all inputs of an item share (xyf_pre), read once
+    // and handed to xyf_with in place of xyf_load.
+    static constexpr int NPRE = 0;
+    __device__ V xyf_pre(int, int, size_t) const { return czero<V>(); }
+    __device__ V xyf_with(int, int, size_t, const V *) const { return czero<V>(); }
+    // Z: output ZMO = sum over f >= ZM0 of zmixc(f) X_f, the others zoutc(o) X_zsrc(o);
+    // inputs f < ZK stay in registers.  The same combination as zmix.
+    static constexpr int ZK = 1, ZMO = 0, ZM0 = 0;
+    __device__ int zsrc(int) const { return 0; }
+    __device__ T zmixc(int, int, int, int, int) const { return (T)0; }
+    __device__ T zoutc(int, int, int, int, int) const { return (T)0; }
+    // (k - q + G)_d u(G)/N, column col of the FP64 tables
+    __device__ double du64(int item, int d, int ncol, int col, int x, int y, int z) const
+    {
+        double G[3];
+        gvec(rc.R, g, x, y, z, kq_of(item), G);
+        const double u = __ldg(&tab_of(item)[(size_t)ncol * pidx(x, y, z) + col]) * invN;
+        return (d == 0 ? G[0] : (d == 1 ? G[1] : G[2])) * u;
+    }
     __device__ bool regacc_grid(int) const { return false; }
     __device__ V xyi_term(int, int, int, size_t, const V *v) const { return v[0]; }
     __device__ void xyi_flush(int, size_t, V) const {}
     __device__ int pair_id(int item) const { return m.tb[item / ns] * m.nSB + m.sb[item % ns]; }
     __device__ const double *kq_of(int item) const { return m.kq + 3 * pair_id(item); }
     __device__ const double *tab_of(int item) const { return m.tab + (size_t)pair_id(item) * g.N * m.ntab; }
-    // mixed path: record r of the coefficient table at grid point p
-    __device__ float4 fco(int item, size_t p, int r) const
+    // mixed path: plane r of the coefficient table at grid point p.  (One plane
+    // per component: an output that needs one of them reads 4 bytes per point,
+    // not a record of 16, from tables that stay in L2.)
+    __device__ float fco(int item, size_t p, int r) const
     {
-        return __ldg(&m.ftab[((size_t)pair_id(item) * g.N + p) * m.nrec + r]);
+        return __ldg(&m.ftab[((size_t)pair_id(item) * m.nrec + r) * g.N + p]);
     }
     static constexpr bool FT = sizeof(T) == 4;   // mixed path: FP32 coefficient tables
-    __device__ static float comp(const float4 &c, int d) { return d == 0 ? c.x : (d == 1 ? c.y : (d == 2 ? c.z : c.w)); }
-    __device__ size_t pidx(int x, int y, int z) const { return (size_t)x + (size_t)g.n0 * (y + (size_t)g.n1 * z); }
-    // Band-limited inputs (bit f of BLI) and outputs (bit o of BLO): pair
-    // densities conj(a_q) b_k of two orbitals of the plane-wave spheres of q
-    // and k, and G-space multiples of them, vanish outside the ball
-    // |G + k - q| < R_k + R_q.  With m.prune set, the pass kernels skip
-    // their pencils outside it (XYF stores, Z loads / transforms / stores,
-    // XYI loads read as zero); values there are zero up to round-off.
+    // index of G-space point (x, y, z) in the grids between the passes and the tables
+    __device__ size_t pidx(int x, int y, int z) const
+    {
+        return m.tr ? (size_t)y + (size_t)g.n1 * (x + (size_t)g.n0 * z) : (size_t)x + (size_t)g.n0 * (y + (size_t)g.n1 * z);
+    }
+    // Inputs (bit f of BLI) and outputs (bit o of BLO) of which only the pencils
+    // inside the ball |G + k - q| < R_k + R_q are needed; with m.prune set, the
+    // pass kernels skip the others (XYF stores, Z loads / transforms / stores,
+    // XYI loads read as zero).  Two kinds: pair densities conj(a_q) b_k of two
+    // orbitals of the plane-wave spheres of q and k and their G-space multiples,
+    // which vanish outside it; and grids X of terms phi_q(r) X(r) (or with
+    // grad phi_q) that are only gathered on the sphere of k, since a component G
+    // of X reaches k + G' only through q + G' - G inside the sphere of q.
     static constexpr unsigned BLI = 0, BLO = 0;
     __device__ int pent_of(int item) const { return m.pent[pair_id(item)]; }
-    __device__ bool pact(int item, int xy) const { return m.pmask[(size_t)pent_of(item) * m.np + xy] != 0; }
-    // active rows y of column x of the item's pair (bit y)
-    __device__ unsigned long long pcol(int item, int x) const { return m.pbits[(size_t)pent_of(item) * g.n0 + x]; }
+    // active x of row y of the item's pair (bit x)
+    __device__ unsigned long long pcol(int item, int y) const { return m.pbits[(size_t)pent_of(item) * g.n1 + y]; }
 };
 
 // =================================================================== hf2x ==
@@ -286,7 +311,7 @@ template <typename T>
 struct OpHF2X : OpBase<T> {
     using V = typename C2<T>::t;
     static constexpr const char *NAME = "hf2x";
-    static constexpr unsigned BLI = 1, BLO = 1;           // conj(phi_q) psi_k and its multiple
+    static constexpr unsigned BLI = 1, BLO = 1;
     static constexpr bool REGACC = true;
     __device__ bool regacc_grid(int) const { return true; }
     __device__ V xyi_term(int, int item, int, size_t p, const V *v) const
@@ -295,6 +320,18 @@ struct OpHF2X : OpBase<T> {
         return cscale(cmul(v[0], __ldg(&Rocc[(size_t)si * this->g.N + p])), (decltype(v[0].x))fill[si]);
     }
     __device__ void xyi_flush(int tj, size_t p, V s) const { acc_red(acc + (size_t)tj * this->g.N + p, to64(s), 1.0); }
+    __device__ const V *xyi_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
+    template <class F> __device__ void xyi_add(int si, int, const V *v, const V *o, F &&add) const
+    {
+        add(0, cscale(cmul(v[0], o[0]), (T)(fill[si])));
+    }
+    __device__ T zmixc(int item, int, int x, int y, int z) const
+    {
+        const size_t p = this->pidx(x, y, z);
+        if constexpr (OpBase<T>::FT) return this->fco(item, p, 0);
+        else return __ldg(&this->tab_of(item)[p]);
+    }
+    __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     static constexpr int NF = 1, NB = 1;
     const V *Rpsi, *Rocc;     // chunk's first target / source
     double2 *acc;
@@ -306,11 +343,10 @@ struct OpHF2X : OpBase<T> {
     }
     __device__ V zmix(int item, int, int x, int y, int z, const V *in) const
     {
-        double G[3];
-        gvec(this->rc.R, this->g, x, y, z, this->kq_of(item), G);
-        const double t = G[0] * G[0] + G[1] * G[1] + G[2] * G[2];
-        const double v = t < 1e-8 ? 0.0 : this->invN / t;   // 1/|k-q+G|^2 (hf2x.cpp:93-104), 1/N folded in
-        return cscale(in[0], (decltype(in[0].x))v);
+        // 1/|k-q+G|^2 (hf2x.cpp:93-104) with the 1/N of the forward transform (TAB_HF)
+        const size_t p = (size_t)this->pair_id(item) * this->g.N + this->pidx(x, y, z);
+        if constexpr (OpBase<T>::FT) return cscale(in[0], __ldg(this->m.ftab + p));
+        else return cscale(in[0], __ldg(this->m.tab + p));
     }
     __device__ void xyi_accum(int tj, int item, int, size_t p, const V *v) const
     {
@@ -324,10 +360,8 @@ template <typename T>
 struct OpTC2X : OpBase<T> {
     using V = typename C2<T>::t;
     static constexpr const char *NAME = "tc2x";
-    static constexpr unsigned BLI = 0xF, BLO = 0xF;       // conj(chi_q) psi_k, conj(chi_q) grad psi_k
+    static constexpr unsigned BLI = 0xF, BLO = 0xF;
     static constexpr bool ZSPLIT = false;     // one thread per z-line measured faster here
-    static constexpr int ZO_ALIAS = 1;        // outputs 1-3 read input 0 only (zmix)
-    static constexpr int Z_MINB_EXTRA = 1;    // five CTAs of 38 KB at 36^3
     static constexpr bool REGACC = true;
     __device__ bool regacc_grid(int) const { return true; }
     __device__ V xyi_term(int, int item, int b, size_t p, const V *v) const
@@ -338,6 +372,30 @@ struct OpTC2X : OpBase<T> {
         return cscale(cmul(v[0], o), (decltype(v[0].x))(b == 0 ? fill[si] : -fill[si]));
     }
     __device__ void xyi_flush(int tj, size_t p, V s) const { acc_red(acc + (size_t)tj * this->g.N + p, to64(s), 1.0); }
+    __device__ const V *xyi_operand(int, int b, int si) const
+    {
+        return b == 0 ? Rocc + (size_t)si * this->g.N : Rgrad + ((size_t)si * 3 + (b - 1)) * this->g.N;
+    }
+    template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
+    {
+        add(0, cscale(cmul(v[0], o[0]), (T)(b == 0 ? fill[si] : -fill[si])));
+    }
+    static constexpr int NPRE = 1;
+    __device__ V xyf_pre(int item, int, size_t p) const { return __ldg(&Rchi[(size_t)(item % this->ns) * this->g.N + p]); }
+    __device__ V xyf_with(int item, int f, size_t p, const V *w) const
+    {
+        const size_t N = this->g.N, tj = item / this->ns;
+        return cmulc(w[0], f == 0 ? __ldg(&Rpsi[tj * N + p]) : __ldg(&Rgpsi[(tj * 3 + (f - 1)) * N + p]));
+    }
+    // coefficient planes: V_2body, du_0, du_1, du_2
+    __device__ T zmixc(int item, int f, int x, int y, int z) const
+    {
+        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), f);
+        else if (f == 0) return __ldg(&this->tab_of(item)[2 * this->pidx(x, y, z)]) * this->invN;
+        else return this->du64(item, f - 1, 2, 1, x, y, z);
+    }
+    __device__ T zoutc(int item, int o, int x, int y, int z) const { return zmixc(item, o, x, y, z); }
+    __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     static constexpr int NF = 4, NB = 4;
     const V *Rpsi, *Rgpsi;        // [nt][N], [nt][3][N]
     const V *Rocc, *Rchi, *Rgrad; // [ns][N], [ns][N], [ns][3][N]
@@ -355,18 +413,18 @@ struct OpTC2X : OpBase<T> {
     {
         using S = decltype(in[0].x);
         if constexpr (OpBase<T>::FT) {
-            const float4 c = this->fco(item, this->pidx(x, y, z), 0);
+            const size_t p = this->pidx(x, y, z);
+            V r = cscale(in[0], this->fco(item, p, o));
             if (o == 0) {
-                V r = cscale(in[0], c.x);
-                r = cadd(r, cscale(in[1], c.y));
-                r = cadd(r, cscale(in[2], c.z));
-                return cadd(r, cscale(in[3], c.w));
+                r = cadd(r, cscale(in[1], this->fco(item, p, 1)));
+                r = cadd(r, cscale(in[2], this->fco(item, p, 2)));
+                r = cadd(r, cscale(in[3], this->fco(item, p, 3)));
             }
-            return cscale(in[0], this->comp(c, o));
+            return r;
         }
         double G[3];
         gvec(this->rc.R, this->g, x, y, z, this->kq_of(item), G);
-        const size_t p = (size_t)x + (size_t)this->g.n0 * (y + (size_t)this->g.n1 * z);
+        const size_t p = this->pidx(x, y, z);
         const double *tab = this->tab_of(item);
         const double u = tab[2 * p + 1] * this->invN;
         if (o == 0) {   // [2a_x] rho V_2body + [2b_x2] sum_d rho_d du_d   (tc2x.cpp:378-386)
@@ -387,24 +445,77 @@ struct OpTC2X : OpBase<T> {
 };
 
 // Jastrow tables per (tb, sb): modes select the columns
-enum TabMode { TAB_TC2X = 0, TAB_U_SX = 1, TAB_U_SS = 2, TAB_U_QX = 3 };
+enum TabMode { TAB_TC2X = 0, TAB_U_SX = 1, TAB_U_SS = 2, TAB_U_QX = 3, TAB_HF = 4 };
 // TAB_TC2X : [V_2body(s,s), u(s,s)]                         (tc2x.cpp:266-276)
 // TAB_U_SX : [u(G; 0, s), u(G; 1, s)]                        (tc3a3b3b4b6.cpp:208-217)
 // TAB_U_SS : [u(G; s, s)]                                    (tc3a3b3b4b6.cpp:679-686)
 // TAB_U_QX : [u(G; s, 0), u(G; s, 1)]                        (tc3a2a4b2b5.cpp:244-253)
-static __global__ void k_tables(GridDesc g, RecipC rc, Jastrow J, int mode, int s, int npair, const double *kq, double *tab)
+// TAB_HF   : [1/(N |G|^2), 0 where |G|^2 < 1e-8]             (hf2x.cpp:93-104)
+// Points in the order of the grids between the passes (tr: y fastest in a plane).
+__device__ __forceinline__ void xyz_tab(const GridDesc &g, int tr, size_t p, int &x, int &y, int &z)
 {
-    const int ntab = mode == TAB_U_SS ? 1 : 2;
+    if (tr) {
+        y = (int)(p % g.n1);
+        x = (int)((p / g.n1) % g.n0);
+        z = (int)(p / ((size_t)g.n0 * g.n1));
+    } else xyz_of(g, p, x, y, z);
+}
+// wrap: the pair densities' sphere reaches past the work grid's box
+// (workgrid.cuh), so a grid point stands for the image of G under the grid's
+// periods that lies in it (the shortest k - q + G); the value is the one the
+// caller's grid un has at that component.
+struct HFGrid {
+    int wrap, un[3];
+};
+__device__ __forceinline__ double hf_kernel(const double *q, const double *R, const GridDesc &g, const HFGrid &hg, int x, int y,
+                                            int z, double invN)
+{
+    int m[3] = {miller(x, g.n0), miller(y, g.n1), miller(z, g.n2)};
+    if (hg.wrap) {
+        double best = 1e300;
+        int b[3] = {0, 0, 0};
+        for (int i = 0; i < 27; i++) {
+            const int s[3] = {m[0] + (i % 3 - 1) * g.n0, m[1] + (i / 3 % 3 - 1) * g.n1, m[2] + (i / 9 - 1) * g.n2};
+            double v = 0;
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const double c = q[d] + R[d] * s[0] + R[3 + d] * s[1] + R[6 + d] * s[2];
+                v += c * c;
+            }
+            if (v < best) {
+                best = v;
+                for (int d = 0; d < 3; d++) b[d] = s[d];
+            }
+        }
+        for (int d = 0; d < 3; d++) {
+            int u = b[d] % hg.un[d];
+            if (u < 0) u += hg.un[d];
+            m[d] = miller(u, hg.un[d]);
+        }
+    }
+    double t = 0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const double c = q[d] + R[d] * m[0] + R[3 + d] * m[1] + R[6 + d] * m[2];
+        t += c * c;
+    }
+    return t < 1e-8 ? 0.0 : invN / t;
+}
+static __global__ void k_tables(GridDesc g, RecipC rc, Jastrow J, int mode, int tr, HFGrid hg, int s, int npair,
+                                const double *kq, double invN, double *tab)
+{
+    const int ntab = mode == TAB_U_SS || mode == TAB_HF ? 1 : 2;
     const size_t total = (size_t)npair * g.N;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const int pr = (int)(i / g.N);
         const size_t p = i % g.N;
         int x, y, z;
-        xyz_of(g, p, x, y, z);
+        xyz_tab(g, tr, p, x, y, z);
         double G[3];
         gvec(rc.R, g, x, y, z, kq + 3 * pr, G);
         double *o = tab + i * ntab;
-        if (mode == TAB_TC2X) { o[0] = J.tc2body(G, s, s); o[1] = J.uk(G, s, s); }
+        if (mode == TAB_HF) o[0] = hf_kernel(kq + 3 * pr, rc.R, g, hg, x, y, z, invN);
+        else if (mode == TAB_TC2X) { o[0] = J.tc2body(G, s, s); o[1] = J.uk(G, s, s); }
         else if (mode == TAB_U_SX) { o[0] = J.uk(G, 0, s); o[1] = J.uk(G, 1, s); }
         else if (mode == TAB_U_SS) { o[0] = J.uk(G, s, s); }
         else { o[0] = J.uk(G, s, 0); o[1] = J.uk(G, s, 1); }
@@ -412,37 +523,39 @@ static __global__ void k_tables(GridDesc g, RecipC rc, Jastrow J, int mode, int 
 }
 
 // FP32 coefficient tables of the mixed path, evaluated in FP64 and rounded
-// once; G = k - q + G_p, all include the 1/N of the forward transform:
-//   TAB_TC2X : {V_2body(s,s), G_0 u, G_1 u, G_2 u} / N       with u = u(G; s, s)
-//   TAB_U_SX : record r = {G_d u(G; x_r, s)} / N, x_r = r (nrec 2) or s (nrec 1)
-//   TAB_U_SS : {G_d u(G; s, s)} / N
-//   TAB_U_QX : record r = {G_d u(G; s, x_r)} / N, x_r = r (nrec 2) or s (nrec 1)
-static __global__ void k_ftables(GridDesc g, RecipC rc, Jastrow J, int mode, int s, int nrec, int npair,
-                                 const double *kq, double invN, float4 *tab)
+// once; G = k - q + G_p, all include the 1/N of the forward transform; a pair's
+// planes of N points each:
+//   TAB_TC2X : V_2body(s,s), G_0 u, G_1 u, G_2 u     with u = u(G; s, s)
+//   TAB_U_SX : G_d u(G; x, s), plane 3 x + d (3 planes: x = s alone)
+//   TAB_U_SS : G_d u(G; s, s)
+//   TAB_U_QX : G_d u(G; s, x), plane 3 x + d (3 planes: x = s alone)
+//   TAB_HF   : 1 / |G|^2
+static __global__ void k_ftables(GridDesc g, RecipC rc, Jastrow J, int mode, int tr, HFGrid hg, int s, int nrec, int npair,
+                                 const double *kq, double invN, float *tab)
 {
     const size_t total = (size_t)npair * g.N;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const int pr = (int)(i / g.N);
         const size_t p = i % g.N;
         int x, y, z;
-        xyz_of(g, p, x, y, z);
-        double G[3];
-        gvec(rc.R, g, x, y, z, kq + 3 * pr, G);
-        float4 *o = tab + i * nrec;
-        if (mode == TAB_TC2X) {
-            const double u = J.uk(G, s, s) * invN;
-            o[0] = make_float4((float)(J.tc2body(G, s, s) * invN), (float)(G[0] * u), (float)(G[1] * u),
-                               (float)(G[2] * u));
+        xyz_tab(g, tr, p, x, y, z);
+        float *o = tab + (size_t)pr * nrec * g.N + p;
+        if (mode == TAB_HF) {
+            o[0] = (float)hf_kernel(kq + 3 * pr, rc.R, g, hg, x, y, z, invN);
             continue;
         }
-        for (int r = 0; r < nrec; r++) {
-            const int xr = nrec == 1 ? s : r;
-            double u;
-            if (mode == TAB_U_SX) u = J.uk(G, xr, s);
-            else if (mode == TAB_U_QX) u = J.uk(G, s, xr);
-            else u = J.uk(G, s, s);
-            u *= invN;
-            o[r] = make_float4((float)(G[0] * u), (float)(G[1] * u), (float)(G[2] * u), 0.f);
+        double G[3];
+        gvec(rc.R, g, x, y, z, kq + 3 * pr, G);
+        int r0 = 0;
+        if (mode == TAB_TC2X) {
+            o[0] = (float)(J.tc2body(G, s, s) * invN);
+            r0 = 1;
+        }
+        const int nx = (nrec - r0) / 3;
+        for (int x2 = 0; x2 < nx; x2++) {
+            const int xr = nx == 1 ? s : x2;
+            const double u = (mode == TAB_U_SX ? J.uk(G, xr, s) : (mode == TAB_U_QX ? J.uk(G, s, xr) : J.uk(G, s, s))) * invN;
+            for (int d = 0; d < 3; d++) o[(size_t)(r0 + 3 * x2 + d) * g.N] = (float)(G[d] * u);
         }
     }
 }
@@ -459,10 +572,7 @@ struct OpTC3A : OpBase<T> {
     static constexpr const char *NAME = "3a3b6A";
     static constexpr int NX = EQ ? 1 : 2;     // spin branches of x2 carried
     static constexpr int NF = 4, NB = 1 + 3 * NX;
-    static constexpr int ZO_ALIAS = 1;        // outputs 1.. read input 0 only (zmix)
-    // input 0 = conj(chi_q) psi_k and outputs 1.. = its multiples; inputs 1-3
-    // carry dnu (their products alias over the whole grid), output 0 mixes them
-    static constexpr unsigned BLI = 1, BLO = ((1u << NB) - 1) & ~1u;
+    static constexpr unsigned BLI = 0xF, BLO = (1u << NB) - 1;
     static constexpr bool REFWD = true;
     static constexpr bool ZSPLIT = false;    // one thread per z-line measured faster here
     // accumulation through xyi_accum (FP64 red.add per source), so that the
@@ -506,18 +616,16 @@ struct OpTC3A : OpBase<T> {
         if constexpr (OpBase<T>::FT) {
             const size_t p = this->pidx(x, y, z);
             if (o == 0) {
-                const float4 c = this->fco(item, p, EQ ? 0 : s);
-                V r = cscale(in[1], c.x);
-                r = cadd(r, cscale(in[2], c.y));
-                return cadd(r, cscale(in[3], c.z));
+                const int r0 = EQ ? 0 : 3 * s;
+                V r = cscale(in[1], this->fco(item, p, r0));
+                r = cadd(r, cscale(in[2], this->fco(item, p, r0 + 1)));
+                return cadd(r, cscale(in[3], this->fco(item, p, r0 + 2)));
             }
-            const int xs = EQ ? s : (o - 1) / 3, d = (o - 1) % 3;
-            const float4 c = this->fco(item, p, EQ ? 0 : xs);
-            return cscale(in[0], (float)fill[item % this->ns] * this->comp(c, d));
+            return cscale(in[0], (float)fill[item % this->ns] * this->fco(item, p, o - 1));   // plane 3 xs + d
         }
         double G[3];
         gvec(this->rc.R, this->g, x, y, z, this->kq_of(item), G);
-        const size_t p = (size_t)x + (size_t)this->g.n0 * (y + (size_t)this->g.n1 * z);
+        const size_t p = this->pidx(x, y, z);
         const double *tab = this->tab_of(item) + 2 * p;
         if (o == 0) {   // [3b3] sum_d du[s]_d FFT(dnu_phi_d conj chi) (:286-295)
             const double u = tab[s] * this->invN;
@@ -547,25 +655,39 @@ struct OpTC3A : OpBase<T> {
         const int xs = EQ ? 0 : (b - 1) / 3;
         return cmul(v, __ldg(&densT[(size_t)xs * this->g.N + p]));   // orbital * n_s2 (:332)
     }
-    // shared-memory accumulation (k_xyi_t6, FP32): slot 0 = acc, 1 + d = qsum_d
-    static constexpr int SACC = 4;
-    __device__ int xyi_slot(int b) const
+    // one sum per output: b3 f v phi_q (b = 0), v phi_q of the branch x = s
+    __device__ const V *xyi_operand(int, int b, int si) const
     {
-        if (b == 0) return 0;
-        const int xs = EQ ? s : (b - 1) / 3;
-        return xs == s ? 1 + (b - 1) % 3 : -1;
+        return regacc_grid(b) ? Rocc + (size_t)si * this->g.N : nullptr;
     }
-    __device__ V xyi_sterm(int, int item, int b, size_t p, V v) const
+    template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
     {
-        const int si = item % this->ns;
-        const V t = cmul(v, __ldg(&Rocc[(size_t)si * this->g.N + p]));
-        return b == 0 ? cscale(t, (decltype(t.x))(fill[si] * b3)) : t;
+        if (regacc_grid(b)) add(0, cscale(cmul(v[0], o[0]), b == 0 ? (T)(fill[si] * b3) : (T)1));
     }
-    __device__ void xyi_sflush(int tj, int slot, size_t p, V sum) const
+    __device__ void xyi_put(int tj, int b, int, size_t p, V sum) const
+    {
+        if (regacc_grid(b)) xyi_flush_b(tj, b, p, sum);
+    }
+    static constexpr int NPRE = 2;
+    __device__ V xyf_pre(int item, int k, size_t p) const
     {
         const size_t N = this->g.N;
-        if (slot == 0) acc_red(acc + (size_t)tj * N + p, to64(sum), 1.0);
-        else acc_red(qsum + ((size_t)tj * 3 + (slot - 1)) * N + p, to64(sum), 1.0);
+        return k == 0 ? __ldg(&Rchi[(size_t)(item % this->ns) * N + p]) : __ldg(&Rpsi[(size_t)(item / this->ns) * N + p]);
+    }
+    __device__ V xyf_with(int, int f, size_t p, const V *w) const
+    {
+        return cmulc(w[0], f > 0 ? cmul(__ldg(&dnu[(size_t)(f - 1) * this->g.N + p]), w[1]) : w[1]);
+    }
+    static constexpr int ZM0 = 1;
+    __device__ T branch_du(int item, int xs, int d, int x, int y, int z) const
+    {
+        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), (EQ ? 0 : 3 * xs) + d);
+        else return this->du64(item, d, 2, xs, x, y, z);
+    }
+    __device__ T zmixc(int item, int f, int x, int y, int z) const { return branch_du(item, s, f - 1, x, y, z); }
+    __device__ T zoutc(int item, int o, int x, int y, int z) const
+    {
+        return (T)fill[item % this->ns] * branch_du(item, EQ ? s : (o - 1) / 3, (o - 1) % 3, x, y, z);
     }
     __device__ V *refwd_grid(int item, int b) const { return tmp2 + ((size_t)item * 3 * NX + (b - 1)) * this->g.N; }
 };
@@ -575,10 +697,9 @@ template <typename T, bool EQ = false>
 struct OpTC3B : OpBase<T> {
     using V = typename C2<T>::t;
     static constexpr const char *NAME = "3b6B";
-    static constexpr bool ZREG = true;
-    static constexpr int ZR_MINB_EXTRA = EQ ? 2 : 0;   // 64 registers without spills for one spin channel
     static constexpr int NX = EQ ? 1 : 2;
     static constexpr int NF = 3 * NX, NB = 1;
+    static constexpr unsigned BLI = (1u << NF) - 1, BLO = 1;
     static constexpr bool REGACC = true;
     __device__ bool regacc_grid(int) const { return true; }
     __device__ V xyi_term(int, int item, int, size_t p, const V *v) const
@@ -587,6 +708,20 @@ struct OpTC3B : OpBase<T> {
         return cscale(cmul(v[0], __ldg(&Rocc[(size_t)si * this->g.N + p])), (decltype(v[0].x))b6);
     }
     __device__ void xyi_flush(int tj, size_t p, V s) const { acc_red(acc + (size_t)tj * this->g.N + p, to64(s), 1.0); }
+    __device__ const V *xyi_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
+    template <class F> __device__ void xyi_add(int si, int, const V *v, const V *o, F &&add) const
+    {
+        add(0, cscale(cmul(v[0], o[0]), (T)(b6)));
+    }
+    // in the coefficient planes / columns of tc3a3b3b4b6's tables, or after tc2x's
+    // V_2body plane (c0 = 1) and in its u column (col = 1) in the shared pass
+    int c0 = 0, col = -1;
+    __device__ T zmixc(int item, int f, int x, int y, int z) const
+    {
+        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), c0 + f);
+        else return this->du64(item, f % 3, 2, col >= 0 ? col : (EQ ? s : f / 3), x, y, z);
+    }
+    __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     const V *Rocc;
     double2 *acc;
     V *tmp2;
@@ -601,16 +736,15 @@ struct OpTC3B : OpBase<T> {
             V r = czero<V>();
 #pragma unroll
             for (int xs = 0; xs < NX; xs++) {
-                const float4 c = this->fco(item, p, xs);
-                r = cadd(r, cscale(in[3 * xs], c.x));
-                r = cadd(r, cscale(in[3 * xs + 1], c.y));
-                r = cadd(r, cscale(in[3 * xs + 2], c.z));
+                r = cadd(r, cscale(in[3 * xs], this->fco(item, p, 3 * xs)));
+                r = cadd(r, cscale(in[3 * xs + 1], this->fco(item, p, 3 * xs + 1)));
+                r = cadd(r, cscale(in[3 * xs + 2], this->fco(item, p, 3 * xs + 2)));
             }
             return r;
         }
         double G[3];
         gvec(this->rc.R, this->g, x, y, z, this->kq_of(item), G);
-        const size_t p = (size_t)x + (size_t)this->g.n0 * (y + (size_t)this->g.n1 * z);
+        const size_t p = this->pidx(x, y, z);
         const double *tab = this->tab_of(item) + 2 * p;
         V r = czero<V>();
 #pragma unroll
@@ -633,7 +767,6 @@ template <typename T>
 struct OpTC3C : OpBase<T> {
     using V = typename C2<T>::t;
     static constexpr const char *NAME = "3b4C";
-    static constexpr bool ZREG = true;
     static constexpr bool REGACC = true;
     __device__ bool regacc_grid(int) const { return true; }
     __device__ V xyi_term(int, int item, int, size_t p, const V *v) const
@@ -642,7 +775,19 @@ struct OpTC3C : OpBase<T> {
         return cscale(cmul(v[0], __ldg(&Rocc[(size_t)si * this->g.N + p])), (decltype(v[0].x))(b4 * fill[si]));
     }
     __device__ void xyi_flush(int tj, size_t p, V s) const { acc_red(acc + (size_t)tj * this->g.N + p, to64(s), 1.0); }
+    __device__ const V *xyi_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
+    template <class F> __device__ void xyi_add(int si, int, const V *v, const V *o, F &&add) const
+    {
+        add(0, cscale(cmul(v[0], o[0]), (T)(b4 * fill[si])));
+    }
+    __device__ T zmixc(int item, int f, int x, int y, int z) const
+    {
+        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), f);
+        else return this->du64(item, f, 1, 0, x, y, z);
+    }
+    __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     static constexpr int NF = 3, NB = 1;
+    static constexpr unsigned BLI = 7, BLO = 1;
     const V *Rocc, *Rchi;
     const double2 *qsum;      // [nt][3][N]
     double2 *acc;
@@ -658,14 +803,14 @@ struct OpTC3C : OpBase<T> {
     {
         using S = decltype(in[0].x);
         if constexpr (OpBase<T>::FT) {
-            const float4 c = this->fco(item, this->pidx(x, y, z), 0);
-            V r = cscale(in[0], c.x);
-            r = cadd(r, cscale(in[1], c.y));
-            return cadd(r, cscale(in[2], c.z));
+            const size_t p = this->pidx(x, y, z);
+            V r = cscale(in[0], this->fco(item, p, 0));
+            r = cadd(r, cscale(in[1], this->fco(item, p, 1)));
+            return cadd(r, cscale(in[2], this->fco(item, p, 2)));
         }
         double G[3];
         gvec(this->rc.R, this->g, x, y, z, this->kq_of(item), G);
-        const size_t p = (size_t)x + (size_t)this->g.n0 * (y + (size_t)this->g.n1 * z);
+        const size_t p = this->pidx(x, y, z);
         const double u = this->tab_of(item)[p] * this->invN;
         V r = cscale(in[0], (S)(G[0] * u));
         r = cadd(r, cscale(in[1], (S)(G[1] * u)));
@@ -690,9 +835,7 @@ struct OpTC3X : OpBase<T> {
     using V = typename C2<T>::t;
     static constexpr const char *NAME = "3bX";
     static constexpr int NF = 3, NB = 1;
-    static constexpr bool ZREG = true;
-    static constexpr bool XYF_SPLIT48 = true;    // measured faster at 48^3 (three operand grids per point)
-    static constexpr int ZR_MINB_EXTRA = 2;      // 64 registers without spills
+    static constexpr unsigned BLI = 7, BLO = 1;
     static constexpr bool REGACC = true;
     __device__ bool regacc_grid(int) const { return true; }
     const V *Rpsi, *Rocc, *Rchi;  // [nt][N], [ns][N], [ns][N]
@@ -714,14 +857,14 @@ struct OpTC3X : OpBase<T> {
     {
         using S = decltype(in[0].x);
         if constexpr (OpBase<T>::FT) {
-            const float4 c = this->fco(item, this->pidx(x, y, z), 0);
-            V r = cscale(in[0], c.x);
-            r = cadd(r, cscale(in[1], c.y));
-            return cadd(r, cscale(in[2], c.z));
+            const size_t p = this->pidx(x, y, z);
+            V r = cscale(in[0], this->fco(item, p, 0));
+            r = cadd(r, cscale(in[1], this->fco(item, p, 1)));
+            return cadd(r, cscale(in[2], this->fco(item, p, 2)));
         }
         double G[3];
         gvec(this->rc.R, this->g, x, y, z, this->kq_of(item), G);
-        const size_t p = (size_t)x + (size_t)this->g.n0 * (y + (size_t)this->g.n1 * z);
+        const size_t p = this->pidx(x, y, z);
         const double u = this->tab_of(item)[p] * this->invN;
         V r = cscale(in[0], (S)(G[0] * u));
         r = cadd(r, cscale(in[1], (S)(G[1] * u)));
@@ -733,6 +876,30 @@ struct OpTC3X : OpBase<T> {
         return cscale(cmul(v[0], __ldg(&Rocc[(size_t)si * this->g.N + p])), (decltype(v[0].x))fill[si]);
     }
     __device__ void xyi_flush(int tj, size_t p, V s) const { acc_red(acc + (size_t)tj * this->g.N + p, to64(s), 1.0); }
+    __device__ const V *xyi_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
+    template <class F> __device__ void xyi_add(int si, int, const V *v, const V *o, F &&add) const
+    {
+        add(0, cscale(cmul(v[0], o[0]), (T)(fill[si])));
+    }
+    static constexpr int NPRE = 2;
+    __device__ V xyf_pre(int item, int k, size_t p) const
+    {
+        const size_t N = this->g.N;
+        return k == 0 ? __ldg(&Rchi[(size_t)(item % this->ns) * N + p]) : __ldg(&Rpsi[(size_t)(item / this->ns) * N + p]);
+    }
+    __device__ V xyf_with(int item, int f, size_t p, const V *w) const
+    {
+        const size_t N = this->g.N;
+        V r = cmulc(w[0], __ldg(&W[((size_t)(item / this->ns) * 3 + f) * N + p]));
+        if (Bt) r = cadd(r, cscale(cmul(__ldg(&Bt[((size_t)(item % this->ns) * 3 + f) * N + p]), w[1]), (T)b5));
+        return r;
+    }
+    __device__ T zmixc(int item, int f, int x, int y, int z) const
+    {
+        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), f);
+        else return this->du64(item, f, 1, 0, x, y, z);
+    }
+    __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     __device__ void xyi_accum(int tj, int item, int, size_t p, const V *v) const
     {
         const int si = item % this->ns;
@@ -751,7 +918,7 @@ struct OpQP : OpBase<T> {
     static constexpr const char *NAME = "qp";
     static constexpr int NX = EQ ? 1 : 2;
     static constexpr int NF = BITC ? 2 : 1, NB = (BITC ? 6 : 3) * NX, GS = BITC ? 2 : 1;
-    static constexpr unsigned BLI = (1u << NF) - 1, BLO = (1u << NB) - 1;   // pair densities of occupied orbitals
+    static constexpr unsigned BLI = (1u << NF) - 1, BLO = (1u << NB) - 1;
     const V *Rq2, *Rq2c;          // targets phi_q2(r), chi_q2(r)  [nt][N]
     const V *Rocc, *Rchi;         // sources phi_q1, chi_q1        [ns][N]
     double2 *acc;                 // [nt][nacc][N]: 3a2[nspin], 3a4[3], 3b5[3]
@@ -771,12 +938,11 @@ struct OpQP : OpBase<T> {
             int xs, d, w;
             if (BITC) { w = o & 1; xs = (o >> 1) / 3; d = (o >> 1) % 3; }
             else { w = 0; xs = o / 3; d = o % 3; }
-            const float4 c = this->fco(item, this->pidx(x, y, z), EQ ? 0 : xs);
-            return cscale(in[w], this->comp(c, d));
+            return cscale(in[w], this->fco(item, this->pidx(x, y, z), (EQ ? 0 : 3 * xs) + d));
         }
         double G[3];
         gvec(this->rc.R, this->g, x, y, z, this->kq_of(item), G);
-        const size_t p = (size_t)x + (size_t)this->g.n0 * (y + (size_t)this->g.n1 * z);
+        const size_t p = this->pidx(x, y, z);
         const double *tab = this->tab_of(item) + 2 * p;
         int xs, d, w;
         if (BITC) { w = o & 1; xs = (o >> 1) / 3; d = (o >> 1) % 3; }
@@ -784,40 +950,56 @@ struct OpQP : OpBase<T> {
         if (EQ) xs = sq;
         return cscale(in[w], (S)(G[d] * tab[xs] * this->invN));   // du[x]_d * phiphi (:378, :385)
     }
-    // shared-memory accumulation (k_xyi_t6, FP32): slot a = accumulator a of
-    // the target (3a2 per spin, 3a4_d, 3b5_d), the same sums as xyi_accum
-    static constexpr int SACC = 8;
-    static constexpr bool SACC_GROUP = true;
-    template <class F>
-    __device__ void xyi_sgroup(int, int item, int b, size_t p, const V *v, F &&add) const
+    // a group's sums: 0 = 3a2 of its branch x2, 1 = 3a4_d, 2 = 3b5_d (x2 = sq)
+    static constexpr int NACC = BITC ? 3 : 2;
+    __device__ void branch(int b, int &xs, int &d) const
     {
-        using S = decltype(v[0].x);
-        const size_t N = this->g.N;
-        const int si = item % this->ns;
-        const S f1 = (S)fill[si];
-        int xs, d;
         if (BITC) { xs = (b >> 1) / 3; d = (b >> 1) % 3; }
         else { xs = b / 3; d = b % 3; }
         if (EQ) xs = sq;
+    }
+    static constexpr int NOPS = BITC ? 2 : 1;
+    __device__ const V *xyi_operand(int k, int b, int si) const
+    {
+        int xs, d;
+        branch(b, xs, d);
+        return xs == sq ? (k == 0 ? Rocc : Rchi) + (size_t)si * this->g.N : nullptr;
+    }
+    template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
+    {
+        const T f1 = (T)fill[si];
+        int xs, d;
+        branch(b, xs, d);
         const V o1 = v[0];
-        V c3a2;
-        if constexpr (BITC) c3a2 = cmulc(v[1], o1);
-        else c3a2 = V{o1.x * o1.x + o1.y * o1.y, (S)0};
-        if (EQ) {
-            if (nspin == 1) add(0, cscale(c3a2, -2 * f1));
-            else { add(0, cscale(c3a2, -f1)); add(1, cscale(c3a2, -f1)); }
-        } else {
-            add(nspin == 1 ? 0 : xs, cscale(c3a2, -f1));
-        }
+        if constexpr (BITC) add(0, cscale(cmulc(v[1], o1), -f1));                            // (:392-394)
+        else add(0, V{-f1 * (o1.x * o1.x + o1.y * o1.y), (T)0});                             // (:404-406)
         if (xs == sq) {
-            add(nspin + d, cscale(cmul(v[0], __ldg(&Rocc[(size_t)si * N + p])), f1));
-            if constexpr (BITC)
-                add(nspin + 3 + d, cscale(cmul(cconj(v[1]), cconj(__ldg(&Rchi[(size_t)si * N + p]))), -f1));
+            add(1, cscale(cmul(o1, o[0]), f1));
+            if constexpr (BITC) add(2, cscale(cconj(cmul(v[1], o[1])), -f1));                // (:428-430)
         }
     }
-    __device__ void xyi_sflush(int tj, int slot, size_t p, V sum) const
+    static constexpr int ZK = NF, ZMO = -1;
+    __device__ int zsrc(int o) const { return BITC ? o & 1 : 0; }
+    __device__ T zoutc(int item, int o, int x, int y, int z) const
     {
-        acc_red(acc + ((size_t)tj * nacc + slot) * this->g.N + p, to64(sum), 1.0);
+        const int w = BITC ? o >> 1 : o, xs = EQ ? sq : w / 3, d = w % 3;
+        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), (EQ ? 0 : 3 * xs) + d);
+        else return this->du64(item, d, 2, xs, x, y, z);
+    }
+    __device__ void xyi_put(int tj, int b, int slot, size_t p, V sum) const
+    {
+        const size_t N = this->g.N;
+        double2 *A = acc + (size_t)tj * nacc * N + p;
+        int xs, d;
+        branch(b, xs, d);
+        if (slot == 0) {
+            // EQ: one branch stands for both, twice into slot 0 (unpolarised) or into 0 and 1
+            if (EQ && nspin == 1) acc_red(A, to64(sum), 2.0);
+            else if (EQ) { acc_red(A, to64(sum), 1.0); acc_red(A + N, to64(sum), 1.0); }
+            else acc_red(A + (size_t)(nspin == 1 ? 0 : xs) * N, to64(sum), 1.0);
+        } else if (xs == sq) {
+            acc_red(A + (size_t)(nspin + (slot == 2 ? 3 : 0) + d) * N, to64(sum), 1.0);
+        }
     }
     __device__ void xyi_accum(int tj, int item, int b, size_t p, const V *v) const
     {
@@ -867,7 +1049,6 @@ struct OpTC2X3 : OpTC2X<T> {
     static constexpr const char *NAME = "2x3A";
     static constexpr bool REFWD = true;
     static constexpr bool RACC_EXTRA = true;
-    static constexpr int XYI_MINB_EXTRA = 1;     // 56 registers, no spills: 2x3A:xyi 638 -> 586 ms on C3
     const V *densT;               // [N] n_0 + n_1 (compute precision)
     double2 *qsum;                // [nt][3][N]
     V *tmp2;                      // [items][3][N] re-forwarded grids
@@ -901,25 +1082,36 @@ struct OpTC2X3 : OpTC2X<T> {
         OpTC2X<T>::xyi_accum(tj, item, b, p, v);
         xyi_extra(tj, item, b, p, v);
     }
-    // optional shared-memory accumulation of the extra sums (k_xyi_t6, FP32;
-    // tc2x's own sum stays in registers): slots 0-2 qsum_d, 3 the band part
-    static constexpr int SACC = 4;
-    static constexpr bool SACC_GROUP = true;
-    template <class F>
-    __device__ void xyi_sgroup(int, int item, int b, size_t p, const V *v, F &&add) const
-    {
-        if (b == 0) return;
-        const int si = item % this->ns;
-        using S = decltype(v[0].x);
-        const S f = (S)this->fill[si];
-        add(b - 1, cscale(cmul(v[0], __ldg(&this->Rocc[(size_t)si * this->g.N + p])), f));
-        if (band) add(3, cscale(cmul(__ldg(&Qt[((size_t)si * 3 + (b - 1)) * this->g.N + p]), v[0]), (S)(f * fa4)));
-    }
-    __device__ void xyi_sflush(int tj, int slot, size_t p, V sum) const
+    // an output's sums: 0 = tc2x's, 1 = qsum_d, 2 = the band part (the last two for b > 0)
+    static constexpr int NACC = 3;
+    static constexpr int NOPS = 3;           // phi_q, grad_d phi_q, Q_d
+    __device__ const V *xyi_operand(int k, int b, int si) const
     {
         const size_t N = this->g.N;
-        if (slot < 3) acc_red(qsum + ((size_t)tj * 3 + slot) * N + p, to64(sum), 1.0);
-        else acc_red(acc3 + (size_t)tj * N + p, to64(sum), 1.0);
+        if (k == 0) return this->Rocc + (size_t)si * N;
+        if (b == 0) return nullptr;
+        if (k == 1) return this->Rgrad + ((size_t)si * 3 + (b - 1)) * N;
+        return band ? Qt + ((size_t)si * 3 + (b - 1)) * N : nullptr;
+    }
+    template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
+    {
+        const T f = (T)this->fill[si];
+        const V w = cscale(v[0], f);
+        if (b == 0) {
+            add(0, cmul(w, o[0]));
+            return;
+        }
+        add(0, cscale(cmul(w, o[1]), (T)-1));
+        add(1, cmul(w, o[0]));
+        if (band) add(2, cmul(w, o[2]));
+    }
+    __device__ void xyi_put(int tj, int b, int slot, size_t p, V sum) const
+    {
+        const size_t N = this->g.N;
+        if (slot == 0) acc_red(this->acc + (size_t)tj * N + p, to64(sum), 1.0);
+        else if (b == 0) return;
+        else if (slot == 1) acc_red(qsum + ((size_t)tj * 3 + (b - 1)) * N + p, to64(sum), 1.0);
+        else if (band) acc_red(acc3 + (size_t)tj * N + p, to64(sum), fa4);
     }
 };
 
@@ -930,6 +1122,9 @@ struct OpPairFwd : OpBase<T> {
     static constexpr const char *NAME = "pairfwd";
     static constexpr int NF = 2, NB = 2;
     static constexpr bool ZINV = false;
+    static constexpr int ZK = 2, ZMO = -1;
+    __device__ int zsrc(int o) const { return o; }
+    __device__ T zoutc(int, int, int, int, int) const { return (T)this->invN; }
     const V *A0, *B0, *A1, *B1;   // item i: conj(A0_i) B0_i, conj(A1_i) B1_i, pointers per item via strides
     const int *ia0, *ib0, *ia1, *ib1;   // per item grid indices; results: tmp slots 0, 1 (G space)
     __device__ V xyf_load(int item, int f, int, int, int, size_t p) const
@@ -950,9 +1145,7 @@ template <typename T>
 struct OpBand : OpBase<T> {
     using V = typename C2<T>::t;
     static constexpr const char *NAME = "band";
-    // input 0 = conj(chi_q2) psi_k and outputs 0-2 = its multiples; inputs 1-3
-    // carry the rotated intermediates Bt (whole grid), output 3 mixes them
-    static constexpr unsigned BLI = 1, BLO = 7;
+    static constexpr unsigned BLI = 0xF, BLO = 0xF;
     static constexpr bool ZSPLIT = false;     // one thread per z-line measured faster here
     static constexpr bool REGACC = true;
     __device__ bool regacc_grid(int) const { return true; }
@@ -964,6 +1157,34 @@ struct OpBand : OpBase<T> {
         return cscale(cmul(v[0], __ldg(&Rocc[(size_t)si * N + p])), (decltype(v[0].x))(fb5 * fill[si]));
     }
     __device__ void xyi_flush(int tj, size_t p, V s) const { acc_red(acc + (size_t)tj * this->g.N + p, to64(s), 1.0); }
+    __device__ const V *xyi_operand(int, int b, int si) const
+    {
+        return b < 3 ? Qt + ((size_t)si * 3 + b) * this->g.N : Rocc + (size_t)si * this->g.N;
+    }
+    template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
+    {
+        const V w = cmul(v[0], o[0]);
+        add(0, b < 3 ? w : cscale(w, (T)(fb5 * fill[si])));
+    }
+    static constexpr int NPRE = 1;
+    __device__ V xyf_pre(int item, int, size_t p) const { return __ldg(&Rpsi[(size_t)(item / this->ns) * this->g.N + p]); }
+    __device__ V xyf_with(int item, int f, size_t p, const V *w) const
+    {
+        const size_t N = this->g.N, si = item % this->ns;
+        return f == 0 ? cmulc(__ldg(&Rchi[si * N + p]), w[0]) : cmul(__ldg(&Bt[(si * 3 + (f - 1)) * N + p]), w[0]);
+    }
+    static constexpr int ZMO = 3, ZM0 = 1;
+    __device__ T du(int item, int d, int x, int y, int z) const
+    {
+        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), d);
+        else return this->du64(item, d, 1, 0, x, y, z);
+    }
+    __device__ T zmixc(int item, int f, int x, int y, int z) const { return du(item, f - 1, x, y, z); }
+    __device__ T zoutc(int item, int o, int x, int y, int z) const
+    {
+        return (T)(fill[item % this->ns] * fa4) * du(item, o, x, y, z);
+    }
+    __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     static constexpr int NF = 4, NB = 4;
     const V *Rpsi;                // [nt][N]
     const V *Rocc, *Rchi;         // phi_q2sym, chi_q2sym [ns][N]
@@ -983,15 +1204,15 @@ struct OpBand : OpBase<T> {
     {
         using S = decltype(in[0].x);
         if constexpr (OpBase<T>::FT) {
-            const float4 c = this->fco(item, this->pidx(x, y, z), 0);
-            if (o < 3) return cscale(in[0], (float)(fill[item % this->ns] * fa4) * this->comp(c, o));
-            V r = cscale(in[1], c.x);
-            r = cadd(r, cscale(in[2], c.y));
-            return cadd(r, cscale(in[3], c.z));
+            const size_t p = this->pidx(x, y, z);
+            if (o < 3) return cscale(in[0], (float)(fill[item % this->ns] * fa4) * this->fco(item, p, o));
+            V r = cscale(in[1], this->fco(item, p, 0));
+            r = cadd(r, cscale(in[2], this->fco(item, p, 1)));
+            return cadd(r, cscale(in[3], this->fco(item, p, 2)));
         }
         double G[3];
         gvec(this->rc.R, this->g, x, y, z, this->kq_of(item), G);
-        const size_t p = (size_t)x + (size_t)this->g.n0 * (y + (size_t)this->g.n1 * z);
+        const size_t p = this->pidx(x, y, z);
         const double u = this->tab_of(item)[p] * this->invN;
         if (o < 3) {    // f2 a4 phiphi du0_d  (:867-872)
             const double f2 = fill[item % this->ns];
