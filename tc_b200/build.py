@@ -1,6 +1,6 @@
 """Build step of the CUDA library libtcg_b200.so (in-tree, sm_100a).
 
-api.cu (C-ABI, orchestration, generic kernels), subspace.cu (the dense
+api.cu (C-ABI, orchestration, generic kernels), cube.cu (on-chip hf2x), subspace.cu (the dense
 Davidson subspace step on cuBLAS / cuSOLVER) and one instance of fast_inst.cu
 per compiled cubic grid size and precision are compiled in parallel into tc_b200/_build/
 and linked into tc_b200/libtcg_b200.so.
@@ -33,6 +33,7 @@ def stale():
 
 def _units():
     units = [(os.path.join(SRC, "api.cu"), os.path.join(OBJ, "api.o"), []),
+             (os.path.join(SRC, "cube.cu"), os.path.join(OBJ, "cube.o"), []),
              (os.path.join(SRC, "subspace.cu"), os.path.join(OBJ, "subspace.o"), [])]
     for t in ("double", "float"):                 # the longest units first
         for n in reversed(FAST_SIZES):

@@ -280,7 +280,7 @@ extern "C" int tcg_ctx_destroy(tcg_ctx *c)
 {
     if (!c) return TCG_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    DBuf *bufs[] = {&c->utw64, &c->utw32, &c->ballmap, &c->udens, &c->uvloc, &c->uwork, &c->w3x, &c->gpsi, &c->adjw, &c->adjt, &c->prune_tab, &c->VH, &c->V2h, &c->pgw, &c->gidx0, &c->vloc, &c->nlB, &c->nlD, &c->acc1, &c->h1buf,
+    DBuf *bufs[] = {&c->hftab, &c->utw64, &c->utw32, &c->ballmap, &c->udens, &c->uvloc, &c->uwork, &c->w3x, &c->gpsi, &c->adjw, &c->adjt, &c->prune_tab, &c->VH, &c->V2h, &c->pgw, &c->gidx0, &c->vloc, &c->nlB, &c->nlD, &c->acc1, &c->h1buf,
                     &c->tw64, &c->tw32, &c->recip, &c->inv, &c->phase, &c->phik, &c->chik, &c->fill,
                     &c->Rocc, &c->Rchi, &c->Rgrad, &c->dens, &c->densT, &c->occfill, &c->Vloc, &c->dnu, &c->dnuT,
                     &c->V3a1, &c->V3b1, &c->V3a2, &c->V3b2, &c->Qt, &c->Bt, &c->accP, &c->qtg, &c->div3b6,

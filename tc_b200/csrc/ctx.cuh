@@ -179,6 +179,10 @@ struct tcg_ctx {
     tcg::DBuf ftab;                         // mixed path: FP32 G-space coefficient planes of a chunk
     tcg::DBuf w3x;                          // [targets][3][N] compute precision: b3 dnu_d psi + b4 qsum_d (3bX input)
     int ftab_nrec = 1;
+    tcg::DBuf hftab;                        // hf2x on chip (cube.cuh): kernel of every (irreducible k, all-k q) pair
+    bool hftab_ok = false;                  // built for the current work grid
+    std::vector<double2> htw64;             // host copies of the work grid's axis-0 twiddles
+    std::vector<float2> htw32;
     int fast_n = 0;                         // cubic grid size with compiled fast kernels (0: generic path)
     bool force_generic = false;             // use the generic pass kernels even if fast_n is set
     int xy_kernels = 0;                     // fast XY passes: 0 default, 1 all line, 2 all lane-pair, 3 split lines (36^3, 48^3)

@@ -62,6 +62,16 @@ __global__ void k_dot3(int N, const double2 *a, const typename C2<T>::t *b, doub
     }
 }
 
+// acc += the splits' sums of the on-chip hf2x, in order
+template <typename V> __global__ void cube_sum(size_t n, int nsplit, const V *part, double2 *acc)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        double2 s = acc[i];
+        for (int k = 0; k < nsplit; k++) s = cadd(s, to64(part[(size_t)k * n + i]));
+        acc[i] = s;
+    }
+}
+
 // per-target input part of the combined 3b3 + 3b4 + 3b5 transform (OpTC3X):
 // W[t][d] = b3 dnu_d psi_t + b4 qsum[t][d], once per target instead of once
 // per (target, source) pair
@@ -874,10 +884,105 @@ static TRange targets_of(const tcg_ctx *c, const Targets &T, int s)
 }
 
 // ================================================================= terms ==
+// hf2x with the pair on chip (cube.cuh, instantiated in cube.cu): sums of nt
+// targets over ns sources into part, `splits` of them, each over `per` sources.
+// TCG_ERR_UNSUPPORTED where the grid has no such kernel.
+template <typename T> struct CubeCall {
+    using V = typename C2<T>::t;
+    const V *Rpsi, *Rocc;
+    const double *fill;
+    const T *tab;
+    const int *tb, *sb;
+    int nSB, ns, per, nt, splits;
+    V *part;
+};
+template <typename T> int hf_cube(tcg_ctx *c, const CubeCall<T> &call);
+template <typename T> bool hf_cube_has(int n);
+
+// The kernel 1 / |k - q + G|^2 of every (irreducible k, all-k q) pair depends on
+// the geometry alone: laid out once per context (and work grid), if it stays
+// below 1 GiB.
+template <typename T>
+static int hf_cube_table(tcg_ctx *c, bool &ok)
+{
+    const Host &h = c->h;
+    const size_t npair = (size_t)h.nk * h.nk_all;
+    ok = false;
+    if (!split_xy(c) || !split_z(c) || !hf_cube_has<T>(c->fast_n) || npair * h.N * sizeof(T) > ((size_t)1 << 30)) return TCG_OK;
+    ok = true;
+    if (c->hftab_ok) return TCG_OK;
+    std::vector<double> kq(3 * npair);
+    for (int k = 0; k < h.nk; k++)
+        for (int a = 0; a < h.nk_all; a++) {
+            double kc[3], qc[3];
+            cart(h, &h.kvec[3 * h.kall_off[k]], kc);
+            cart(h, &h.kvec[3 * a], qc);
+            for (int d = 0; d < 3; d++) kq[3 * ((size_t)k * h.nk_all + a) + d] = kc[d] - qc[d];
+        }
+    TRY(c->hftab.ensure(npair * h.N * sizeof(T)));
+    TRY(up(c->meta, kq.data(), kq.size() * sizeof(double), c->stream));
+    RecipC rc;
+    memcpy(rc.R, h.recip, sizeof rc.R);
+    const HFGrid hg{h.hf_wrap ? 1 : 0, {h.un[0], h.un[1], h.un[2]}};
+    const double invN = 1.0 / (double)h.N;
+    if constexpr (sizeof(T) == 4)
+        TRY(launch(c, k_ftables, dim3(148 * 8), dim3(256), 0, c->gd, rc, make_jastrow(h), (int)TAB_HF, 1, hg, 0, 1, (int)npair,
+                   (const double *)c->meta.p, invN, c->hftab.as<float>()));
+    else
+        TRY(launch(c, k_tables, dim3(148 * 8), dim3(256), 0, c->gd, rc, make_jastrow(h), (int)TAB_HF, 1, hg, 0, (int)npair,
+                   (const double *)c->meta.p, invN, c->hftab.as<double>()));
+    TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->meta is reused
+    c->hftab_ok = true;
+    return TCG_OK;
+}
+
+template <typename T>
+static int run_hf2x_cube(tcg_ctx *c, const Targets &Tg, double2 *acc)
+{
+    using V = typename C2<T>::t;
+    const Host &h = c->h;
+    const size_t N = h.N;
+    for (int s = 0; s < h.nspin; s++) {
+        TRange TR = targets_of(c, Tg, s);
+        Sources S = sources_of(c, s);
+        const int ns = (int)S.key.size();
+        if (TR.n == 0 || ns == 0) continue;
+        CubeCall<T> a;
+        a.nt = TR.n;
+        a.ns = ns;
+        // about 8 CTAs per SM in all (a partly filled last round then costs
+        // little), at least 4 sources each, at most 1 GiB of partial sums
+        int splits = std::max(1, std::min((148 * 8 + TR.n - 1) / TR.n, (ns + 3) / 4));
+        splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ((size_t)1 << 30) / (TR.n * N * sizeof(V))));
+        a.per = (ns + splits - 1) / splits;
+        a.splits = (ns + a.per - 1) / a.per;
+        std::vector<int> idx(TR.key);
+        idx.insert(idx.end(), S.key.begin(), S.key.end());
+        TRY(up(c->meta, idx.data(), idx.size() * sizeof(int), c->stream));
+        TRY(c->tmp.ensure((size_t)a.splits * TR.n * N * sizeof(V)));
+        a.Rpsi = c->Rpsi.as<V>() + (size_t)TR.t0 * N;
+        a.Rocc = c->Rocc.as<V>() + S.base * N;
+        a.fill = c->occfill.as<double>() + S.base;
+        a.tab = c->hftab.as<T>();
+        a.tb = c->meta.as<int>();
+        a.sb = a.tb + TR.n;
+        a.nSB = h.nk_all;
+        a.part = c->tmp.as<V>();
+        TRY(hf_cube<T>(c, a));
+        TRY(launch(c, cube_sum<V>, dim3((unsigned)std::min<size_t>(148 * 8, (TR.n * N + 255) / 256)), dim3(256), 0,
+                   (size_t)TR.n * N, a.splits, (const V *)a.part, acc + (size_t)TR.t0 * N));
+        TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->meta is reused
+    }
+    return TCG_OK;
+}
+
 template <typename T>
 static int run_hf2x(tcg_ctx *c, const Targets &Tg, double2 *acc)
 {
     PhaseScope ps_(c, "ap:2x");
+    bool on_chip;
+    TRY(hf_cube_table<T>(c, on_chip));
+    if (on_chip) return run_hf2x_cube<T>(c, Tg, acc);
     using V = typename C2<T>::t;
     const Host &h = c->h;
     const size_t N = h.N;

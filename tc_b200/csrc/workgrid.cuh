@@ -232,6 +232,10 @@ static int make_grid(tcg_ctx *c, const int *n, GridDesc &g, DBuf &tw64, DBuf &tw
     TCG_CUDA(cudaStreamSynchronize(c->stream));
     g.tw64 = tw64.as<const double2>();
     g.tw32 = tw32.as<const float2>();
+    if (&g == &c->gd) {
+        c->htw64.assign(t64.begin(), t64.begin() + n[0]);
+        c->htw32.assign(t32.begin(), t32.begin() + n[0]);
+    }
     return TCG_OK;
 }
 
@@ -322,6 +326,7 @@ static int configure_grid(tcg_ctx *c, bool reduced)
         TCG_CUDA(cudaStreamSynchronize(c->stream));
         h.hf_wrap = h.method == TCG_METHOD_HF;
     }
+    c->hftab_ok = false;
     c->prune_ok = false;
     if (c->fast_n) TRY(build_prune_table(c));
     return place_vloc(c);
