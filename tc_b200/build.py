@@ -16,7 +16,7 @@ SRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 FAST_SIZES = (12, 15, 16, 18, 20, 24, 25, 27, 30, 32, 36, 40, 45, 48)     # ctx.cuh: TCG_FAST_SIZES
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-CFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
+CFLAGS = ARCH + ["-O3", "-lineinfo", "-compress-mode=size", "-std=c++17", "-Xcompiler", "-fPIC"]
 
 
 def sources():
@@ -36,6 +36,7 @@ def _units():
              (os.path.join(SRC, "cube.cu"), os.path.join(OBJ, "cube.o"), []),
              (os.path.join(SRC, "subspace.cu"), os.path.join(OBJ, "subspace.o"), [])]
     for t in ("double", "float"):                 # the longest units first
+        units.append((os.path.join(SRC, "any_inst.cu"), os.path.join(OBJ, f"any_{t}.o"), [f"-DTCG_FAST_T={t}"]))
         for n in reversed(FAST_SIZES):
             units.append((os.path.join(SRC, "fast_inst.cu"), os.path.join(OBJ, f"fast_{n}_{t}.o"),
                           [f"-DTCG_FAST_N={n}", f"-DTCG_FAST_T={t}"]))

@@ -112,6 +112,33 @@ constexpr bool line_grid(int n) { return n == 12 || n == 16 || n == 24 || n == 3
 // grids on which tcg_set_forms offers the split-line forms by number
 inline bool split_line_grid(int n) { return n == 36 || n == 48; }
 
+namespace sl {
+// run-time shape of the split-line passes on other grids (anygrid.cuh): n = a b
+// along each axis, row stride and size of an XY buffer
+struct AnyShape {
+    int n[3], a[3], b[3], rs, ps;
+};
+constexpr int MAXTHR = 9 * 64;       // threads of an XY pass: a (<= 9) per line, 64 lines
+
+inline bool any_shape(const int *n, size_t vbytes, AnyShape &s)
+{
+    for (int d = 0; d < 3; d++) {
+        s.n[d] = n[d];
+        s.a[d] = 0;
+        for (int a = 9; a >= 2; a--)
+            if (n[d] <= 64 && n[d] % a == 0 && n[d] / a <= a && n[d] / a >= 2) { s.a[d] = a; s.b[d] = n[d] / a; }
+        if (!s.a[d]) return false;
+    }
+    const int m = n[0] > n[1] ? n[0] : n[1];
+    s.rs = m | 1;
+    s.ps = s.rs * m;
+    const int thr = s.a[1] * n[0] > s.a[0] * n[1] ? s.a[1] * n[0] : s.a[0] * n[1];
+    // the inverse XY pass with three sums per point, the Z pass with six inputs
+    return vbytes * (n[0] + n[1] + 2 * (size_t)s.ps + 3 * (size_t)s.b[1] * thr) <= 227 * 1024 &&
+           vbytes * (size_t)n[2] * (1 + 6 * 32) <= 227 * 1024;
+}
+} // namespace sl
+
 // layout of the pencil table of pruned transforms: bits [nent][n1] u64,
 // counts [nent] int, permutations [nent][n0 n1] u16
 struct PruneTable {
@@ -184,6 +211,8 @@ struct tcg_ctx {
     std::vector<double2> htw64;             // host copies of the work grid's axis-0 twiddles
     std::vector<float2> htw32;
     int fast_n = 0;                         // cubic grid size with compiled fast kernels (0: generic path)
+    bool any_ok = false;                    // split-line passes with the run-time shape `any` (fast_n == 0)
+    tcg::sl::AnyShape any;
     bool force_generic = false;             // use the generic pass kernels even if fast_n is set
     int xy_kernels = 0;                     // fast XY passes: 0 default, 1 all line, 2 all lane-pair, 3 split lines (36^3, 48^3)
     bool no_prefetch = false;               // fast XYI: no prefetch of the next plane set
@@ -205,7 +234,8 @@ namespace tcg {
 inline bool split_form(const tcg_ctx *c, bool xy)
 {
     const bool fx = c->xy_kernels == 0 || c->xy_kernels == 3, fz = c->z_kernels == 0 || c->z_kernels >= 3;
-    if (!c->fast_n || c->force_generic) return false;
+    if (c->force_generic) return false;
+    if (!c->fast_n) return c->any_ok && fx && fz;
     return line_grid(c->fast_n) ? (xy ? fx : fz) : (fx && fz);
 }
 inline bool split_xy(const tcg_ctx *c) { return split_form(c, true); }

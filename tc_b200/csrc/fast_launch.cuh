@@ -22,9 +22,18 @@ int run_chunk_fast(tcg_ctx *c, const Op &op, int items, int nt, bool do_xyf, boo
     const bool slx = split_xy(c), slz = split_z(c);
     using SH = sl::Shape<N, sl::ShapeOf<N>::A, sl::ShapeOf<N>::B>;
     const int nref = Op::REFWD ? Op::NB - 1 : 0;
-    if (slx && do_xyf)
-        TRY(launch_tagged(c, tagname(Op::NAME, "xyf"), (double)items * nf_eff * gb, sl::k_xyf<T, Op, SH>, dim3(np_f),
-                          dim3(SH::THREADS), sl::smem_xyf<V, SH>(), op, items));
+    if (slx && do_xyf) {
+        const double by = (double)items * nf_eff * gb;
+        if constexpr (Op::NSO == 0) {
+            TRY(launch_tagged(c, tagname(Op::NAME, "xyf"), by, sl::k_xyf_items<T, Op, SH>, dim3(np_f), dim3(SH::THREADS),
+                              sl::smem_xyf<V, SH, Op>(), op, items));
+        } else {
+            // sources per CTA: at least 8 CTAs per SM and round of 4 where the chunk has them
+            const int parts = std::max(1, std::min(op.ns, (148 * 8 * 4 + np_i - 1) / np_i)), per = (op.ns + parts - 1) / parts;
+            TRY(launch_tagged(c, tagname(Op::NAME, "xyf"), by, sl::k_xyf<T, Op, SH>, dim3(np_i, (op.ns + per - 1) / per),
+                              dim3(SH::THREADS), sl::smem_xyf<V, SH, Op>(), op, nt, per));
+        }
+    }
     auto z_split = [&]() -> int {
         // pencils nobody needs get no CTA
         const unsigned fi = (1u << Op::NF) - 1, fo = (1u << Op::NB) - 1;

@@ -33,7 +33,12 @@ namespace sl {
 template <int N_, int A_, int B_> struct Shape {
     static constexpr int N = N_, A = A_, B = B_;
     static constexpr int PAD = N_ + ((N_ % 2 == 0) ? 1 : 0);   // odd row stride: rows across lanes conflict-free
-    static constexpr int THREADS = A_ * N_;      // XY passes: one plane per CTA
+    // XY passes: one plane per CTA, A groups of LP lanes.  A group of N lanes
+    // that ends inside a half-warp would share its shared-memory accesses with the
+    // next group's row, two to a bank (30: every second access took a third
+    // wavefront), so it is padded to a half-warp or warp where that is close.
+    static constexpr int LP = N_ <= 16 ? 16 : (N_ <= 32 ? 32 : N_);
+    static constexpr int THREADS = A_ * LP;
     static constexpr int ZTHREADS = A_ * 32;     // Z pass: 32 pencils per CTA
     static_assert(N_ == A_ * B_ && A_ >= B_ && N_ <= 64, "two-step lines; pencil masks hold 64 bits");
 };
@@ -102,9 +107,37 @@ template <typename V, int DIR> __device__ __forceinline__ void dft9(V *v)
         v[k + 6] = w[2];
     }
 }
+template <typename V, int DIR> __device__ __forceinline__ void dft7(V *v)
+{
+    using S = decltype(v[0].x);
+    // cos, sin of 2 pi j / 7
+    constexpr double c[4] = {1.0, 0.62348980185873353053, -0.22252093395631440429, -0.90096886790241912624};
+    constexpr double w[4] = {0.0, 0.78183148246802980871, 0.97492791218182360702, 0.43388373911755812048};
+    V t[4], d[4], a = v[0];
+#pragma unroll
+    for (int k = 1; k < 4; k++) {
+        t[k] = cadd(v[k], v[7 - k]);
+        d[k] = csub(v[k], v[7 - k]);
+    }
+    v[0] = cadd(cadd(a, t[1]), cadd(t[2], t[3]));
+    auto sum3 = [](S x, double p, S y, double q, S z, double r) { return CMul::mul2(x, p, y, q) + CMul::mul(z, r); };
+#pragma unroll
+    for (int j = 1; j < 4; j++) {
+        // j k mod 7 folded to 1..3; the sine changes sign beyond
+        const int i1 = j, i2 = 2 * j % 7 > 3 ? 7 - 2 * j % 7 : 2 * j % 7, i3 = 3 * j % 7 > 3 ? 7 - 3 * j % 7 : 3 * j % 7;
+        const double g2 = 2 * j % 7 > 3 ? -1.0 : 1.0, g3 = 3 * j % 7 > 3 ? -1.0 : 1.0;
+        const V m = {a.x + sum3(t[1].x, c[i1], t[2].x, c[i2], t[3].x, c[i3]),
+                     a.y + sum3(t[1].y, c[i1], t[2].y, c[i2], t[3].y, c[i3])};
+        const V n = cmuli(V{sum3(d[1].x, w[i1], d[2].x, g2 * w[i2], d[3].x, g3 * w[i3]),
+                            sum3(d[1].y, w[i1], d[2].y, g2 * w[i2], d[3].y, g3 * w[i3])}, DIR);
+        v[j] = cadd(m, n);
+        v[7 - j] = csub(m, n);
+    }
+}
 template <typename V, int R, int DIR> __device__ __forceinline__ void dft(V *v)
 {
     if constexpr (R == 6) dft6<V, DIR>(v);
+    else if constexpr (R == 7) dft7<V, DIR>(v);
     else if constexpr (R == 9) dft9<V, DIR>(v);
     else fast::dftR<V, R, DIR>(v);
 }
@@ -145,25 +178,26 @@ template <typename V, class S>
 __device__ __forceinline__ void plane_fwd(V *b0, V *b1, int t, int l, V (&u)[S::B], const Tw<V, S::B> &tw, V (&v)[S::A])
 {
     constexpr int A = S::A, B = S::B, PAD = S::PAD;
-    if (t < A) {
+    const bool on = S::LP == S::N || l < S::N;
+    if (on) {
         step1<V, B, -1>(u, tw);
         put<V, A, B>(b0 + l, PAD, t, u);
     }
     __syncthreads();
-    if (t < B) {
+    if (on && t < B) {
         step2<V, A, B, -1>(b0 + l, PAD, t, v);          // ky = t + B m at x = l
 #pragma unroll
         for (int m = 0; m < A; m++) b1[(t + B * m) * PAD + l] = v[m];
     }
     __syncthreads();
-    if (t < A) {
+    if (on) {
 #pragma unroll
         for (int m = 0; m < B; m++) u[m] = b1[l * PAD + t + A * m];   // x = t + A m at ky = l
         step1<V, B, -1>(u, tw);
         put<V, A, B>(b0 + l, PAD, t, u);
     }
     __syncthreads();
-    if (t < B) step2<V, A, B, -1>(b0 + l, PAD, t, v);
+    if (on && t < B) step2<V, A, B, -1>(b0 + l, PAD, t, v);
 }
 // Inverse XY transform.  In: u[m] = F(kx = t + B m, ky = l), t < B.
 // Out: v[m] = f(x = l, y = t + A m), t < A.
@@ -171,73 +205,58 @@ template <typename V, class S>
 __device__ __forceinline__ void plane_inv(V *b0, V *b1, int t, int l, V (&u)[S::A], const Tw<V, S::A> &tw, V (&v)[S::B])
 {
     constexpr int A = S::A, B = S::B, PAD = S::PAD;
-    if (t < B) {
+    const bool on = S::LP == S::N || l < S::N;
+    if (on && t < B) {
         step1<V, A, +1>(u, tw);
         put<V, B, A>(b0 + l, PAD, t, u);
     }
     __syncthreads();
-    if (t < A) {
+    if (on) {
         step2<V, B, A, +1>(b0 + l, PAD, t, v);          // x = t + A m at ky = l
 #pragma unroll
         for (int m = 0; m < B; m++) b1[l * PAD + t + A * m] = v[m];
     }
     __syncthreads();
-    if (t < B) {
+    if (on && t < B) {
 #pragma unroll
         for (int m = 0; m < A; m++) u[m] = b1[(t + B * m) * PAD + l];   // ky = t + B m at x = l
         step1<V, A, +1>(u, tw);
         put<V, B, A>(b0 + l, PAD, t, u);
     }
     __syncthreads();
-    if (t < A) step2<V, B, A, +1>(b0 + l, PAD, t, v);
+    if (on) step2<V, B, A, +1>(b0 + l, PAD, t, v);
 }
 
 // --------------------------------------------------------------- XYF --------
 // One (item, z) plane per CTA: pair products -> forward XY -> tmp (y fastest).
-// Planes of equal z are neighbours in the grid, so that the operand planes
-// (shared by many items) stay in L1 / L2; the operands that every input of the
-// item uses (Op::NPRE of them) are read once.
+// For ops without a target / source structure (Op::NSO == 0).
 template <typename T, class Op, class S>
-__global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, sizeof(T) == 4 ? 56 + 2 * Op::NPRE * S::B : 104))
-    k_xyf(Op op, int items)
+__global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, sizeof(T) == 4 ? 56 : 104)) k_xyf_items(Op op, int items)
 {
     using V = typename C2<T>::t;
-    constexpr int N = S::N, A = S::A, B = S::B, PS = S::N * S::PAD, NP = Op::NPRE;
+    constexpr int N = S::N, A = S::A, B = S::B, PS = S::N * S::PAD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V *b0 = reinterpret_cast<V *>(smem_raw), *b1 = b0 + PS;
-    const int t = threadIdx.x / N, l = threadIdx.x % N;
+    const int t = threadIdx.x / S::LP, l = threadIdx.x % S::LP;
+    const bool on = S::LP == N || l < N;
     const int z = blockIdx.x / items, item = blockIdx.x % items;
-    const size_t pz = (size_t)z * N * N, p0 = pz + (size_t)t * N + l;
-    V pre[NP ? NP : 1][B];
-#pragma unroll
-    for (int k = 0; k < NP; k++)
-#pragma unroll
-        for (int m = 0; m < B; m++) pre[k][m] = op.xyf_pre(item, k, p0 + (size_t)A * m * N);
+    const size_t pz = (size_t)z * N * N;
     Tw<V, B> tw;
     tw.load(op.g, t);
-    unsigned long long bits = ~0ull;
-    if (Op::BLI != 0 && op.m.prune) bits = op.pcol(item, l);   // kx mask of row ky = l
-#pragma unroll 1
     for (int f = 0; f < Op::NF; f++) {
         V u[B], v[A];
+        if (on) {
 #pragma unroll
-        for (int m = 0; m < B; m++) {
-            if constexpr (NP > 0) {
-                V w[NP];
-#pragma unroll
-                for (int k = 0; k < NP; k++) w[k] = pre[k][m];
-                u[m] = op.xyf_with(item, f, p0 + (size_t)A * m * N, w);
-            } else {
-                u[m] = op.xyf_load(item, f, l, t + A * m, z, p0 + (size_t)A * m * N);
+            for (int m = 0; m < B; m++) {
+                const int y = t + A * m;
+                u[m] = op.xyf_load(item, f, l, y, z, pz + (size_t)y * N + l);
             }
         }
         plane_fwd<V, S>(b0, b1, t, l, u, tw, v);
-        if (t < B) {
+        if (on && t < B) {
             V *dst = op.tmp_grid(item, f) + pz + l;
-            const bool bl = (Op::BLI >> f) & 1;
 #pragma unroll
-            for (int m = 0; m < A; m++)
-                if (!bl || ((bits >> (t + B * m)) & 1)) dst[(size_t)(t + B * m) * N] = v[m];
+            for (int m = 0; m < A; m++) dst[(size_t)(t + B * m) * N] = v[m];
         }
         V *s = b0;
         b0 = b1;
@@ -245,35 +264,116 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, sizeof(T) == 
     }
 }
 
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int K> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(K) : "memory"); }
+
+// One (target, z) plane per CTA, looping over `per` of the chunk's sources (part
+// blockIdx.y): the target's operand planes are read again for every source from
+// L1, the source's own (at most Op::NSO per input) are copied ahead, one input
+// while the previous one is transformed, into slots that belong to the reading
+// thread.  With a CTA per pair every operand came from L2 for every pair (3bX:xyf
+// at 30^3: 7 TB/s of it).
+template <typename T, class Op, class S>
+__global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, sizeof(T) == 4 ? 64 : 104)) k_xyf(Op op, int nt, int per)
+{
+    using V = typename C2<T>::t;
+    constexpr int N = S::N, A = S::A, B = S::B, PS = S::N * S::PAD, NO = Op::NSO;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    V *b0 = reinterpret_cast<V *>(smem_raw), *b1 = b0 + PS;
+    V *ops = b1 + PS + threadIdx.x;              // [NO][B][THREADS]
+    const int t = threadIdx.x / S::LP, l = threadIdx.x % S::LP;
+    const bool on = S::LP == N || l < N;
+    const int z = blockIdx.x / nt, tj = blockIdx.x % nt;
+    const size_t pz = (size_t)z * N * N, p0 = pz + (size_t)t * N + l;
+    const int s0 = blockIdx.y * per, s1 = min(op.nsrc(tj), s0 + per);
+    Tw<V, B> tw;
+    tw.load(op.g, t);
+    auto fetch = [&](int si, int f) {
+        if (on) {
+#pragma unroll
+            for (int k = 0; k < NO; k++) {
+                const V *src = op.xyf_operand(k, f, si);
+                if (src) {
+#pragma unroll
+                    for (int m = 0; m < B; m++) fast::cp_async_elem(ops + (k * B + m) * S::THREADS, src + p0 + (size_t)A * m * N);
+                }
+            }
+        }
+        cp_commit();
+    };
+    fetch(s0, 0);
+#pragma unroll 1
+    for (int si = s0; si < s1; si++) {
+        const int item = op.item_of(tj, si);
+        unsigned long long bits = ~0ull;
+        if (Op::BLI != 0 && op.m.prune && on) bits = op.pcol(item, l);   // kx mask of row ky = l
+        bits >>= t;
+#pragma unroll 1
+        for (int f = 0; f < Op::NF; f++) {
+            V u[B], v[A];
+            cp_wait<0>();
+            if (on) {
+#pragma unroll
+                for (int m = 0; m < B; m++) {
+                    V o[NO];
+#pragma unroll
+                    for (int k = 0; k < NO; k++) o[k] = ops[(k * B + m) * S::THREADS];
+                    u[m] = op.xyf_pair(tj, f, p0 + (size_t)A * m * N, o);
+                }
+            }
+            if (f + 1 < Op::NF) fetch(si, f + 1);
+            else if (si + 1 < s1) fetch(si + 1, 0);
+            plane_fwd<V, S>(b0, b1, t, l, u, tw, v);
+            if (on && t < B) {
+                V *dst = op.tmp_grid(item, f) + pz + (size_t)t * N + l;
+                const bool bl = (Op::BLI >> f) & 1;
+#pragma unroll
+                for (int m = 0; m < A; m++)
+                    if (!bl || ((bits >> (B * m)) & 1)) dst[(size_t)B * m * N] = v[m];
+            }
+            V *s = b0;
+            b0 = b1;
+            b1 = s;
+        }
+    }
+}
+template <typename V, class S, class Op> __host__ inline size_t smem_xyf()
+{
+    return sizeof(V) * (2 * (size_t)S::N * S::PAD + (size_t)Op::NSO * S::B * S::THREADS);
+}
+
 // --------------------------------------------------------------- XYI --------
 // One (target, z) plane per CTA.  The outputs b (in groups of GS) run outside,
 // the chunk's sources inside, and a group's sums over the sources (at most
 // Op::NACC of them: xyi_add) stay with the thread that owns the points, in
-// registers in FP32 and in shared memory in FP64; each reaches the FP64
-// accumulators once per group and chunk (xyi_put).
+// registers; each reaches the FP64 accumulators once per group and chunk
+// (xyi_put).
 // What bounds the pass is the latency of its operands (phi_q, grad phi_q, Q_q at
 // the plane: read by every target, so from L2): loaded where they are used, they
 // stalled each step for longer than its transforms took (issue slots 27% busy,
-// 10.7 of 14 stall cycles long_scoreboard for 2x3A:xyi at 30^3).  In FP32 they and
-// the next step's G plane are therefore copied asynchronously into slots of
-// shared memory that belong to the reading thread alone, so a thread waits for
-// its own copies and the passes' barriers stay the only ones.
+// 10.7 of 14 stall cycles long_scoreboard for 2x3A:xyi at 30^3, 45.8 ms of the
+// 27-k case).  They and the next step's G plane are therefore copied
+// asynchronously into slots of shared memory that belong to the reading thread
+// alone, so a thread waits for its own copies and the passes' barriers stay the
+// only ones (20.9 ms, with registers for three sums and no spills; 24.2 with one
+// CTA more and spills).  FP64 planes beyond 32^2 leave no room for the slots:
+// there operands are loaded in place and the sums live in shared memory.
 // GS > 1: the first GS - 1 outputs of a group wait in registers.
 constexpr int MAXSRC = 64;           // sources per chunk (plan_chunks): rows of pencil masks in shared memory
 
 template <class Op, class S, typename V> struct Lay {
     static constexpr int B = S::B;
-    static constexpr bool STG = sizeof(V) == 8;          // FP32: staged operands, sums in registers
+    static constexpr bool STG = sizeof(V) == 8 || S::N <= 32;     // staged operands, sums in registers
     static constexpr size_t PLANES = sizeof(V) * 2 * (size_t)S::N * S::PAD;
     static constexpr size_t ACC = STG ? 0 : sizeof(V) * (size_t)Op::NACC * B * S::THREADS;
     static constexpr size_t OPS = STG ? sizeof(V) * (size_t)Op::NOPS * B * S::THREADS : 0;
     static constexpr size_t GPL = STG ? sizeof(V) * (size_t)S::N * S::N : 0;
     static constexpr size_t TOTAL = PLANES + ACC + OPS + GPL;
-    // FP32: 80 registers (4 CTAs of 180 threads) with three sums per point, 64 with one
-    static constexpr int REGS = STG ? 50 + 2 * Op::NACC * B : 112;
+    // registers: in FP32 96 (3 CTAs of 6 warps) with three sums per point, 72 with one
+    static constexpr int REGS = sizeof(V) == 8 ? 66 + 2 * Op::NACC * B : (STG ? 108 + 4 * Op::NACC * B : 112);
 };
 template <class Op, class S, typename V> struct Acc {
-    static constexpr bool SM = sizeof(V) == 16;
+    static constexpr bool SM = !Lay<Op, S, V>::STG;
     static constexpr int B = S::B;
     V r[SM ? 1 : Op::NACC][SM ? 1 : B];
     V *sm;
@@ -283,8 +383,6 @@ template <class Op, class S, typename V> struct Acc {
         else return r[slot][m];
     }
 };
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int K> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(K) : "memory"); }
 
 template <typename T, class Op, class S>
 __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, typename C2<T>::t>::REGS)) k_xyi(Op op, int nt)
@@ -294,7 +392,8 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
     constexpr int N = S::N, A = S::A, B = S::B, PS = S::N * S::PAD, NA = Op::NACC, NO = Op::NOPS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V *b0 = reinterpret_cast<V *>(smem_raw), *b1 = b0 + PS;
-    const int t = threadIdx.x / N, l = threadIdx.x % N;
+    const int t = threadIdx.x / S::LP, l = threadIdx.x % S::LP;
+    const bool on = S::LP == N || l < N;
     const int z = blockIdx.x / nt, tj = blockIdx.x % nt;
     const size_t pz = (size_t)z * N * N, p0 = pz + (size_t)t * N + l;
     const int ns = op.nsrc(tj);
@@ -324,7 +423,7 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
     auto mask = [&](int si, int b) { return prune && ((Op::BLO >> b) & 1) ? sbits[si * N + l] : ~0ull; };
     V nx[L::STG ? 1 : A];
     auto fetch = [&](int si, int b) {
-        if (t < B) {
+        if (on && t < B) {
             const V *src = op.xyi_grid(op.item_of(tj, si), b) + pz + (size_t)t * N + l;
             const unsigned long long bits = mask(si, b) >> t;
 #pragma unroll
@@ -346,12 +445,12 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
         V u[A], v[B];
         if constexpr (L::STG) {
             cp_wait<0>();
-            if (t < B) {
+            if (on && t < B) {
                 const unsigned long long bits = mask(si, bg + q) >> t;
 #pragma unroll
                 for (int m = 0; m < A; m++) u[m] = (bits >> (B * m)) & 1 ? gpl[m * B * N] : czero<V>();
             }
-            if (q == Op::GS - 1) {
+            if (on && q == Op::GS - 1) {
 #pragma unroll
                 for (int k = 0; k < NO; k++) {
                     const V *src = op.xyi_operand(k, bg, si);
@@ -393,7 +492,7 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
         }
         const int item = op.item_of(tj, si);
         if constexpr (L::STG) cp_wait<1>();      // this step's operands; the next G plane may be on its way
-        if (t < A) {
+        if (on) {
 #pragma unroll
             for (int m = 0; m < B; m++) {
                 V vals[Op::GS], o[NO];
@@ -417,7 +516,7 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
         if (Op::REFWD && op.refwd_want(bg)) {   // uniform over the CTA
             // derived plane (orbital x density): forward XY straight from the registers
             V w[A];
-            if (t < A) {
+            if (on) {
 #pragma unroll
                 for (int m = 0; m < B; m++) v[m] = op.refwd_load(tj, item, bg, p0 + (size_t)A * m * N, v[m]);
             }
@@ -427,7 +526,7 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
                 b0 = b1;
                 b1 = s;
             }
-            if (t < B) {
+            if (on && t < B) {
                 V *dst = op.refwd_grid(item, bg) + pz + (size_t)t * N + l;
                 const unsigned long long bits = (prune ? sbits[si * N + l] : ~0ull) >> t;
 #pragma unroll
@@ -436,7 +535,7 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
             }
         }
         if (bn != bg) {                          // the group's last source
-            if (t < A) {
+            if (on) {
 #pragma unroll
                 for (int a = 0; a < NA; a++)
 #pragma unroll
@@ -456,7 +555,6 @@ template <typename V, class S, class Op> __host__ inline size_t smem_xyi(bool pr
 {
     return Lay<Op, S, V>::TOTAL + (prune ? (size_t)ns * S::N * sizeof(unsigned long long) : 0);
 }
-template <typename V, class S> __host__ inline size_t smem_xyf() { return sizeof(V) * 2 * (size_t)S::N * S::PAD; }
 // ----------------------------------------------------------------- Z --------
 // One item and 32 consecutive pencils per CTA, A threads per z-line, one
 // exchange per transform.  The G-space combination is linear: output ZMO (if
@@ -490,7 +588,7 @@ __global__ void __launch_bounds__(S::ZTHREADS, ctas_for(S::ZTHREADS, sizeof(T) =
         if (allin && (Op::BLI & FI) == FI && (Op::BLO & FO) == FO) return;   // uniform over the CTA
     }
     const bool act = slot < N * N;
-    const int x = op.m.tr ? c / N : c % N, y = op.m.tr ? c % N : c / N;
+    const auto zc = op.zctx(item, op.m.tr ? c / N : c % N, op.m.tr ? c % N : c / N, c);
     {
         V u[NF][B];
 #pragma unroll
@@ -523,7 +621,7 @@ __global__ void __launch_bounds__(S::ZTHREADS, ctas_for(S::ZTHREADS, sizeof(T) =
                 if (f >= Op::ZM0) {
 #pragma unroll
                     for (int m = 0; m < A; m++) {
-                        const V w = cscale(X[m], act ? op.zmixc(item, f, x, y, t + B * m) : (T)0);
+                        const V w = cscale(X[m], act ? op.zmixc(zc, f, t + B * m) : (T)0);
                         mix[m] = f == Op::ZM0 ? w : cadd(mix[m], w);
                     }
                 }
@@ -549,7 +647,7 @@ __global__ void __launch_bounds__(S::ZTHREADS, ctas_for(S::ZTHREADS, sizeof(T) =
                 const int k = op.zsrc(o);
 #pragma unroll
                 for (int m = 0; m < A; m++) {
-                    const T w = act ? op.zoutc(item, o, x, y, t + B * m) : (T)0;
+                    const T w = act ? op.zoutc(zc, o, t + B * m) : (T)0;
                     v[m] = cscale(ZK > 1 && k ? K[ZK - 1][m] : K[0][m], w);
                 }
             }

@@ -636,6 +636,9 @@ static size_t max_items_for(const tcg_ctx *c, int nslots, size_t vbytes)
 // size in fast_inst.cu (one translation unit per N).
 template <typename T, int N, class Op>
 int run_chunk_fast(tcg_ctx *c, const Op &op, int items, int nt, bool do_xyf, bool do_xyi);
+// The same for grids without compiled kernels (anygrid.cuh, instantiated in any_inst.cu).
+template <typename T, class Op>
+int run_chunk_any(tcg_ctx *c, const Op &op, int items, int nt, bool do_xyf, bool do_xyi);
 
 // Algorithmic bytes per pass launch: a 3D FFT of N points moves 2 N s bytes
 // (one read + one write of the grid); each of the two passes of a
@@ -653,6 +656,7 @@ static int run_chunk(tcg_ctx *c, const Op &op, int items, int nt, bool do_xyf = 
         default: break;
         }
     }
+    if (!c->fast_n && split_xy(c)) return run_chunk_any<T, Op>(c, op, items, nt, do_xyf, do_xyi);
     const int ntiles = (g.n0 * g.n1 + ZTC - 1) / ZTC;
     const double gb = (double)g.N * sizeof(V);
     if (do_xyf) TRY(launch_tagged(c, tagname(Op::NAME, "xyf"), (double)items * Op::NF * gb, k_xyf<T, Op>, dim3(g.n2, items), dim3(256), smem_xy<V>(g), op));

@@ -254,24 +254,48 @@ struct OpBase {
     __device__ const V *xyi_operand(int, int, int) const { return nullptr; }
     template <class F> __device__ void xyi_add(int, int, const V *, const V *, F &&) const {}
     __device__ void xyi_put(int, int, int, size_t, V) const {}
-    // Forward XY: operands that all inputs of an item share (xyf_pre), read once
-    // and handed to xyf_with in place of xyf_load.
-    static constexpr int NPRE = 0;
-    __device__ V xyf_pre(int, int, size_t) const { return czero<V>(); }
-    __device__ V xyf_with(int, int, size_t, const V *) const { return czero<V>(); }
+    // Forward XY: at most NSO operand grids of the source per input (xyf_operand(k,
+    // f, si), null where unused); xyf_pair(tj, f, p, o) is the input's value from
+    // them and the target's operands, the same as xyf_load.  NSO = 0: xyf_load.
+    static constexpr int NSO = 1;
     // Z: output ZMO = sum over f >= ZM0 of zmixc(f) X_f, the others zoutc(o) X_zsrc(o);
     // inputs f < ZK stay in registers.  The same combination as zmix.
     static constexpr int ZK = 1, ZMO = 0, ZM0 = 0;
     __device__ int zsrc(int) const { return 0; }
-    __device__ T zmixc(int, int, int, int, int) const { return (T)0; }
-    __device__ T zoutc(int, int, int, int, int) const { return (T)0; }
-    // (k - q + G)_d u(G)/N, column col of the FP64 tables
-    __device__ double du64(int item, int d, int ncol, int col, int x, int y, int z) const
+    // what the coefficients of one item and pencil need, looked up once: FP32 its
+    // planes at the pencil, FP64 its table column and k - q + G without the z part
+    struct ZC {
+        const float *ft;
+        const double *td;
+        double q[3];
+        T f;                 // filling of the item's source (ops that use it)
+    };
+    __device__ ZC zctx_base(int item, int x, int y, int c, int ncol) const
     {
-        double G[3];
-        gvec(rc.R, g, x, y, z, kq_of(item), G);
-        const double u = __ldg(&tab_of(item)[(size_t)ncol * pidx(x, y, z) + col]) * invN;
-        return (d == 0 ? G[0] : (d == 1 ? G[1] : G[2])) * u;
+        ZC z;
+        const int pr = pair_id(item);
+        z.f = (T)1;
+        if constexpr (sizeof(T) == 4) z.ft = m.ftab + (size_t)pr * m.nrec * g.N + c;
+        else {
+            z.td = m.tab + ((size_t)pr * g.N + c) * ncol;
+            const int m0 = miller(x, g.n0), m1 = miller(y, g.n1);
+#pragma unroll
+            for (int d = 0; d < 3; d++) z.q[d] = m.kq[3 * pr + d] + rc.R[d] * m0 + rc.R[3 + d] * m1;
+        }
+        return z;
+    }
+    // coefficient plane r at height z (FP32); table column col and
+    // (k - q + G)_d u(G)/N from u in column col (FP64, ncol columns)
+    __device__ T zpl(const ZC &c, int r, int z) const { return (T)__ldg(c.ft + (size_t)r * g.N + (size_t)z * g.n0 * g.n1); }
+    __device__ double zcol(const ZC &c, int ncol, int col, int z) const
+    {
+        return __ldg(c.td + (size_t)z * g.n0 * g.n1 * ncol + col);
+    }
+    __device__ double zdu(const ZC &c, int ncol, int col, int d, int z) const
+    {
+        const double u = zcol(c, ncol, col, z) * invN, m2 = miller(z, g.n2);
+        const double k = d == 0 ? c.q[0] + rc.R[6] * m2 : (d == 1 ? c.q[1] + rc.R[7] * m2 : c.q[2] + rc.R[8] * m2);
+        return k * u;
     }
     __device__ bool regacc_grid(int) const { return false; }
     __device__ V xyi_term(int, int, int, size_t, const V *v) const { return v[0]; }
@@ -325,12 +349,16 @@ struct OpHF2X : OpBase<T> {
     {
         add(0, cscale(cmul(v[0], o[0]), (T)(fill[si])));
     }
-    __device__ T zmixc(int item, int, int x, int y, int z) const
+    __device__ const V *xyf_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
+    __device__ V xyf_pair(int tj, int, size_t p, const V *o) const { return cmulc(o[0], __ldg(&Rpsi[(size_t)tj * this->g.N + p])); }
+    using ZC = typename OpBase<T>::ZC;
+    __device__ ZC zctx(int item, int x, int y, int c) const { return this->zctx_base(item, x, y, c, 1); }
+    __device__ T zmixc(const ZC &c, int, int z) const
     {
-        const size_t p = this->pidx(x, y, z);
-        if constexpr (OpBase<T>::FT) return this->fco(item, p, 0);
-        else return __ldg(&this->tab_of(item)[p]);
+        if constexpr (OpBase<T>::FT) return this->zpl(c, 0, z);
+        else return this->zcol(c, 1, 0, z);
     }
+    __device__ T zoutc(const ZC &, int, int) const { return (T)0; }
     __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     static constexpr int NF = 1, NB = 1;
     const V *Rpsi, *Rocc;     // chunk's first target / source
@@ -380,21 +408,22 @@ struct OpTC2X : OpBase<T> {
     {
         add(0, cscale(cmul(v[0], o[0]), (T)(b == 0 ? fill[si] : -fill[si])));
     }
-    static constexpr int NPRE = 1;
-    __device__ V xyf_pre(int item, int, size_t p) const { return __ldg(&Rchi[(size_t)(item % this->ns) * this->g.N + p]); }
-    __device__ V xyf_with(int item, int f, size_t p, const V *w) const
+    __device__ const V *xyf_operand(int, int, int si) const { return Rchi + (size_t)si * this->g.N; }
+    __device__ V xyf_pair(int tj, int f, size_t p, const V *o) const
     {
-        const size_t N = this->g.N, tj = item / this->ns;
-        return cmulc(w[0], f == 0 ? __ldg(&Rpsi[tj * N + p]) : __ldg(&Rgpsi[(tj * 3 + (f - 1)) * N + p]));
+        const size_t N = this->g.N;
+        return cmulc(o[0], f == 0 ? __ldg(&Rpsi[(size_t)tj * N + p]) : __ldg(&Rgpsi[((size_t)tj * 3 + (f - 1)) * N + p]));
     }
     // coefficient planes: V_2body, du_0, du_1, du_2
-    __device__ T zmixc(int item, int f, int x, int y, int z) const
+    using ZC = typename OpBase<T>::ZC;
+    __device__ ZC zctx(int item, int x, int y, int c) const { return this->zctx_base(item, x, y, c, 2); }
+    __device__ T zmixc(const ZC &c, int f, int z) const
     {
-        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), f);
-        else if (f == 0) return __ldg(&this->tab_of(item)[2 * this->pidx(x, y, z)]) * this->invN;
-        else return this->du64(item, f - 1, 2, 1, x, y, z);
+        if constexpr (OpBase<T>::FT) return this->zpl(c, f, z);
+        else if (f == 0) return this->zcol(c, 2, 0, z) * this->invN;
+        else return this->zdu(c, 2, 1, f - 1, z);
     }
-    __device__ T zoutc(int item, int o, int x, int y, int z) const { return zmixc(item, o, x, y, z); }
+    __device__ T zoutc(const ZC &c, int o, int z) const { return zmixc(c, o, z); }
     __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     static constexpr int NF = 4, NB = 4;
     const V *Rpsi, *Rgpsi;        // [nt][N], [nt][3][N]
@@ -668,27 +697,28 @@ struct OpTC3A : OpBase<T> {
     {
         if (regacc_grid(b)) xyi_flush_b(tj, b, p, sum);
     }
-    static constexpr int NPRE = 2;
-    __device__ V xyf_pre(int item, int k, size_t p) const
+    __device__ const V *xyf_operand(int, int, int si) const { return Rchi + (size_t)si * this->g.N; }
+    __device__ V xyf_pair(int tj, int f, size_t p, const V *o) const
     {
-        const size_t N = this->g.N;
-        return k == 0 ? __ldg(&Rchi[(size_t)(item % this->ns) * N + p]) : __ldg(&Rpsi[(size_t)(item / this->ns) * N + p]);
-    }
-    __device__ V xyf_with(int, int f, size_t p, const V *w) const
-    {
-        return cmulc(w[0], f > 0 ? cmul(__ldg(&dnu[(size_t)(f - 1) * this->g.N + p]), w[1]) : w[1]);
+        V rhs = __ldg(&Rpsi[(size_t)tj * this->g.N + p]);
+        if (f > 0) rhs = cmul(__ldg(&dnu[(size_t)(f - 1) * this->g.N + p]), rhs);
+        return cmulc(o[0], rhs);
     }
     static constexpr int ZM0 = 1;
-    __device__ T branch_du(int item, int xs, int d, int x, int y, int z) const
+    using ZC = typename OpBase<T>::ZC;
+    __device__ ZC zctx(int item, int x, int y, int c) const
     {
-        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), (EQ ? 0 : 3 * xs) + d);
-        else return this->du64(item, d, 2, xs, x, y, z);
+        ZC z = this->zctx_base(item, x, y, c, 2);
+        z.f = (T)fill[item % this->ns];
+        return z;
     }
-    __device__ T zmixc(int item, int f, int x, int y, int z) const { return branch_du(item, s, f - 1, x, y, z); }
-    __device__ T zoutc(int item, int o, int x, int y, int z) const
+    __device__ T branch_du(const ZC &c, int xs, int d, int z) const
     {
-        return (T)fill[item % this->ns] * branch_du(item, EQ ? s : (o - 1) / 3, (o - 1) % 3, x, y, z);
+        if constexpr (OpBase<T>::FT) return this->zpl(c, (EQ ? 0 : 3 * xs) + d, z);
+        else return this->zdu(c, 2, xs, d, z);
     }
+    __device__ T zmixc(const ZC &c, int f, int z) const { return branch_du(c, s, f - 1, z); }
+    __device__ T zoutc(const ZC &c, int o, int z) const { return c.f * branch_du(c, EQ ? s : (o - 1) / 3, (o - 1) % 3, z); }
     __device__ V *refwd_grid(int item, int b) const { return tmp2 + ((size_t)item * 3 * NX + (b - 1)) * this->g.N; }
 };
 
@@ -716,11 +746,15 @@ struct OpTC3B : OpBase<T> {
     // in the coefficient planes / columns of tc3a3b3b4b6's tables, or after tc2x's
     // V_2body plane (c0 = 1) and in its u column (col = 1) in the shared pass
     int c0 = 0, col = -1;
-    __device__ T zmixc(int item, int f, int x, int y, int z) const
+    static constexpr int NSO = 0;             // no forward pass
+    using ZC = typename OpBase<T>::ZC;
+    __device__ ZC zctx(int item, int x, int y, int c) const { return this->zctx_base(item, x, y, c, 2); }
+    __device__ T zmixc(const ZC &c, int f, int z) const
     {
-        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), c0 + f);
-        else return this->du64(item, f % 3, 2, col >= 0 ? col : (EQ ? s : f / 3), x, y, z);
+        if constexpr (OpBase<T>::FT) return this->zpl(c, c0 + f, z);
+        else return this->zdu(c, 2, col >= 0 ? col : (EQ ? s : f / 3), f % 3, z);
     }
+    __device__ T zoutc(const ZC &, int, int) const { return (T)0; }
     __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     const V *Rocc;
     double2 *acc;
@@ -780,11 +814,19 @@ struct OpTC3C : OpBase<T> {
     {
         add(0, cscale(cmul(v[0], o[0]), (T)(b4 * fill[si])));
     }
-    __device__ T zmixc(int item, int f, int x, int y, int z) const
+    __device__ const V *xyf_operand(int, int, int si) const { return Rchi + (size_t)si * this->g.N; }
+    __device__ V xyf_pair(int tj, int f, size_t p, const V *o) const
     {
-        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), f);
-        else return this->du64(item, f, 1, 0, x, y, z);
+        return cmulc(o[0], from64<V>(__ldg(&qsum[((size_t)tj * 3 + f) * this->g.N + p])));
     }
+    using ZC = typename OpBase<T>::ZC;
+    __device__ ZC zctx(int item, int x, int y, int c) const { return this->zctx_base(item, x, y, c, 1); }
+    __device__ T zmixc(const ZC &c, int f, int z) const
+    {
+        if constexpr (OpBase<T>::FT) return this->zpl(c, f, z);
+        else return this->zdu(c, 1, 0, f, z);
+    }
+    __device__ T zoutc(const ZC &, int, int) const { return (T)0; }
     __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     static constexpr int NF = 3, NB = 1;
     static constexpr unsigned BLI = 7, BLO = 1;
@@ -881,24 +923,26 @@ struct OpTC3X : OpBase<T> {
     {
         add(0, cscale(cmul(v[0], o[0]), (T)(fill[si])));
     }
-    static constexpr int NPRE = 2;
-    __device__ V xyf_pre(int item, int k, size_t p) const
+    static constexpr int NSO = 2;
+    __device__ const V *xyf_operand(int k, int f, int si) const
     {
-        const size_t N = this->g.N;
-        return k == 0 ? __ldg(&Rchi[(size_t)(item % this->ns) * N + p]) : __ldg(&Rpsi[(size_t)(item / this->ns) * N + p]);
+        return k == 0 ? Rchi + (size_t)si * this->g.N : (Bt ? Bt + ((size_t)si * 3 + f) * this->g.N : nullptr);
     }
-    __device__ V xyf_with(int item, int f, size_t p, const V *w) const
+    __device__ V xyf_pair(int tj, int f, size_t p, const V *o) const
     {
         const size_t N = this->g.N;
-        V r = cmulc(w[0], __ldg(&W[((size_t)(item / this->ns) * 3 + f) * N + p]));
-        if (Bt) r = cadd(r, cscale(cmul(__ldg(&Bt[((size_t)(item % this->ns) * 3 + f) * N + p]), w[1]), (T)b5));
+        V r = cmulc(o[0], __ldg(&W[((size_t)tj * 3 + f) * N + p]));
+        if (Bt) r = cadd(r, cscale(cmul(o[1], __ldg(&Rpsi[(size_t)tj * N + p])), (T)b5));
         return r;
     }
-    __device__ T zmixc(int item, int f, int x, int y, int z) const
+    using ZC = typename OpBase<T>::ZC;
+    __device__ ZC zctx(int item, int x, int y, int c) const { return this->zctx_base(item, x, y, c, 1); }
+    __device__ T zmixc(const ZC &c, int f, int z) const
     {
-        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), f);
-        else return this->du64(item, f, 1, 0, x, y, z);
+        if constexpr (OpBase<T>::FT) return this->zpl(c, f, z);
+        else return this->zdu(c, 1, 0, f, z);
     }
+    __device__ T zoutc(const ZC &, int, int) const { return (T)0; }
     __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     __device__ void xyi_accum(int tj, int item, int, size_t p, const V *v) const
     {
@@ -980,11 +1024,19 @@ struct OpQP : OpBase<T> {
     }
     static constexpr int ZK = NF, ZMO = -1;
     __device__ int zsrc(int o) const { return BITC ? o & 1 : 0; }
-    __device__ T zoutc(int item, int o, int x, int y, int z) const
+    using ZC = typename OpBase<T>::ZC;
+    __device__ ZC zctx(int item, int x, int y, int c) const { return this->zctx_base(item, x, y, c, 2); }
+    __device__ T zmixc(const ZC &, int, int) const { return (T)0; }
+    __device__ T zoutc(const ZC &c, int o, int z) const
     {
         const int w = BITC ? o >> 1 : o, xs = EQ ? sq : w / 3, d = w % 3;
-        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), (EQ ? 0 : 3 * xs) + d);
-        else return this->du64(item, d, 2, xs, x, y, z);
+        if constexpr (OpBase<T>::FT) return this->zpl(c, (EQ ? 0 : 3 * xs) + d, z);
+        else return this->zdu(c, 2, xs, d, z);
+    }
+    __device__ const V *xyf_operand(int, int f, int si) const { return (f == 0 ? Rchi : Rocc) + (size_t)si * this->g.N; }
+    __device__ V xyf_pair(int tj, int f, size_t p, const V *o) const
+    {
+        return cmulc(o[0], __ldg(&(f == 0 ? Rq2 : Rq2c)[(size_t)tj * this->g.N + p]));
     }
     __device__ void xyi_put(int tj, int b, int slot, size_t p, V sum) const
     {
@@ -1124,7 +1176,11 @@ struct OpPairFwd : OpBase<T> {
     static constexpr bool ZINV = false;
     static constexpr int ZK = 2, ZMO = -1;
     __device__ int zsrc(int o) const { return o; }
-    __device__ T zoutc(int, int, int, int, int) const { return (T)this->invN; }
+    static constexpr int NSO = 0;
+    using ZC = typename OpBase<T>::ZC;
+    __device__ ZC zctx(int, int, int, int) const { return ZC{}; }
+    __device__ T zmixc(const ZC &, int, int) const { return (T)0; }
+    __device__ T zoutc(const ZC &, int, int) const { return (T)this->invN; }
     const V *A0, *B0, *A1, *B1;   // item i: conj(A0_i) B0_i, conj(A1_i) B1_i, pointers per item via strides
     const int *ia0, *ib0, *ia1, *ib1;   // per item grid indices; results: tmp slots 0, 1 (G space)
     __device__ V xyf_load(int item, int f, int, int, int, size_t p) const
@@ -1166,24 +1222,30 @@ struct OpBand : OpBase<T> {
         const V w = cmul(v[0], o[0]);
         add(0, b < 3 ? w : cscale(w, (T)(fb5 * fill[si])));
     }
-    static constexpr int NPRE = 1;
-    __device__ V xyf_pre(int item, int, size_t p) const { return __ldg(&Rpsi[(size_t)(item / this->ns) * this->g.N + p]); }
-    __device__ V xyf_with(int item, int f, size_t p, const V *w) const
+    __device__ const V *xyf_operand(int, int f, int si) const
     {
-        const size_t N = this->g.N, si = item % this->ns;
-        return f == 0 ? cmulc(__ldg(&Rchi[si * N + p]), w[0]) : cmul(__ldg(&Bt[(si * 3 + (f - 1)) * N + p]), w[0]);
+        return f == 0 ? Rchi + (size_t)si * this->g.N : Bt + ((size_t)si * 3 + (f - 1)) * this->g.N;
+    }
+    __device__ V xyf_pair(int tj, int f, size_t p, const V *o) const
+    {
+        const V phj = __ldg(&Rpsi[(size_t)tj * this->g.N + p]);
+        return f == 0 ? cmulc(o[0], phj) : cmul(o[0], phj);
     }
     static constexpr int ZMO = 3, ZM0 = 1;
-    __device__ T du(int item, int d, int x, int y, int z) const
+    using ZC = typename OpBase<T>::ZC;
+    __device__ ZC zctx(int item, int x, int y, int c) const
     {
-        if constexpr (OpBase<T>::FT) return this->fco(item, this->pidx(x, y, z), d);
-        else return this->du64(item, d, 1, 0, x, y, z);
+        ZC z = this->zctx_base(item, x, y, c, 1);
+        z.f = (T)(fill[item % this->ns] * fa4);
+        return z;
     }
-    __device__ T zmixc(int item, int f, int x, int y, int z) const { return du(item, f - 1, x, y, z); }
-    __device__ T zoutc(int item, int o, int x, int y, int z) const
+    __device__ T du(const ZC &c, int d, int z) const
     {
-        return (T)(fill[item % this->ns] * fa4) * du(item, o, x, y, z);
+        if constexpr (OpBase<T>::FT) return this->zpl(c, d, z);
+        else return this->zdu(c, 1, 0, d, z);
     }
+    __device__ T zmixc(const ZC &c, int f, int z) const { return du(c, f - 1, z); }
+    __device__ T zoutc(const ZC &c, int o, int z) const { return c.f * du(c, o, z); }
     __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
     static constexpr int NF = 4, NB = 4;
     const V *Rpsi;                // [nt][N]

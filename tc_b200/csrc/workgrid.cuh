@@ -328,7 +328,8 @@ static int configure_grid(tcg_ctx *c, bool reduced)
     }
     c->hftab_ok = false;
     c->prune_ok = false;
-    if (c->fast_n) TRY(build_prune_table(c));
+    c->any_ok = !c->fast_n && sl::any_shape(h.n, c->prec == TCG_PREC_FP64 ? sizeof(double2) : sizeof(float2), c->any);
+    if (c->fast_n || c->any_ok) TRY(build_prune_table(c));
     return place_vloc(c);
 }
 

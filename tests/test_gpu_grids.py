@@ -1,0 +1,143 @@
+"""The pass kernels at the sizes where they differ, and the choice of the work
+grid, against the oracle.
+
+- every compiled cubic size and run-time shape (uneven grids, cubic sizes without
+  kernels of their own, lengths only the generic passes take), with a cutoff so
+  large for the grid that the library has to work on the grid itself;
+- the smaller work grid: HF where the pair densities wrap around its box, time
+  reversal with k-differences beyond the first cell, TC with a density that is not
+  band limited (the grid of the caller has to be used) and back, density output;
+- the on-chip hf2x at each of its sizes, with several partial sums per target.
+
+Tolerances as in test_gpu_parity.py: FP64 relative 1e-10, mixed 2e-5.
+"""
+import numpy as np
+import pytest
+
+from tc_b200 import abi, synth
+from tc_b200.context import Context
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = {"fp64": 1e-10, "mixed": 2e-5}
+
+
+def rel(a, b):
+    d, m = np.abs(a - b).max(), np.abs(b).max()
+    return d / m if m > 0 else d
+
+
+def check(s, mask, prec):
+    r2, r3 = O.apply(s, mask)
+    with Context(s, prec) as ctx:
+        ctx.set_state()
+        g2, g3 = ctx.apply(mask)
+    assert rel(g2, r2) < TOL[prec]
+    if mask & ~abi.TERMS_H2:
+        assert rel(g3, r3) < TOL[prec]
+
+
+def tight(n, frac=0.21):
+    """cutoff of an fcc Si sphere whose radius is `frac` times the shortest period of
+    the n^3 grid: products of three-body terms fold onto the used components"""
+    b = np.sqrt(3.0) * 2.0 * np.pi / 10.26
+    return 0.5 * (frac * n * b) ** 2
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [12, 15, 16, 18, 20, 24, 25, 27, 30, 32, 36, 40, 45, 48])
+def test_compiled_sizes(n, prec):
+    s = synth.small("BITC", nr=(n, n, n), nk=1, ecut=tight(n), nbands=2, nocc=1, seed=n)
+    check(s, abi.TERMS_TC, prec)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("nr", [(21, 21, 21), (14, 14, 14), (20, 18, 21), (12, 25, 16), (35, 18, 20), (28, 42, 15),
+                                (22, 20, 18), (26, 26, 26)])
+def test_run_time_shapes(nr, prec):
+    n = min(nr)
+    s = synth.small("TC", nr=nr, nk=1, ecut=tight(n, 0.19), nbands=2, nocc=2, seed=n)
+    check(s, abi.TERMS_TC, prec)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_run_time_shape_spin_channels(prec):
+    """unequal Jastrow channels: the separate passes, both branches of x2"""
+    s = synth.small("BITC", nr=(15, 18, 14), nk=1, ecut=2.5, nbands=2, nocc=1, nspin=2, F=np.array([[1.3, 1.0], [1.0, 1.2]]))
+    check(s, abi.TERMS_TC, prec)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,ecut", [(12, 4.0), (15, 7.0), (16, 7.9), (18, 10.0), (20, 12.0)])
+def test_on_chip_exchange(n, ecut, prec):
+    """hf2x work grids of n^3 inside a finer grid; 16 sources"""
+    s = synth.small("HF", nr=(36, 36, 36), nk=2, ecut=ecut, nbands=3, nocc=2, seed=n)
+    check(s, abi.TERM_HF2X, prec)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("method", ["HF", "TC"])
+def test_work_grid_time_reversal(method, prec):
+    """k - q up to 4/3: the pair densities' sphere leaves the box of the caller's
+    grid, whose own representation of those components defines the result"""
+    s = synth.small(method, nr=(16, 16, 16), tr=True, ecut=5.0, nbands=2, nocc=1)
+    check(s, abi.TERMS_HF if method == "HF" else abi.TERMS_TC, prec)
+
+
+def test_density_beyond_the_pair_sphere():
+    """a density with a component outside the pair densities' sphere needs the
+    caller's grid; the next state may go back to the smaller one"""
+    s = synth.small("TC", nr=(32, 32, 32), nk=1, ecut=6.0, nbands=2, nocc=2, seed=4)
+    plain = s.density.copy()
+    z, y, x = np.meshgrid(*[np.arange(32) / 32.0] * 3, indexing="ij")
+    wave = 0.05 * np.abs(plain).max() * np.cos(2 * np.pi * (13 * x + 2 * y - 11 * z)).ravel()
+    with Context(s, "fp64") as ctx:
+        for dens in (plain, plain + wave[None, :], plain):
+            s.density = dens
+            r2, r3 = O.apply(s, abi.TERMS_TC)
+            ctx.set_state()
+            g2, g3 = ctx.apply(abi.TERMS_TC)
+            assert rel(g2, r2) < TOL["fp64"]
+            assert rel(g3, r3) < TOL["fp64"]
+    s.density = plain
+
+
+@pytest.mark.parametrize("method", ["HF", "TC", "BITC"])
+def test_density_from_the_work_grid(method):
+    s = synth.small(method, nr=(32, 32, 32), nk=2, ecut=5.0, nbands=2, nocc=2, seed=6)
+    d0 = O.density(s)
+    with Context(s, "fp64") as ctx:
+        d = ctx.density()
+    assert rel(d, d0) < 1e-12
+
+
+@pytest.mark.parametrize("npw,nbasis,nblock", [(40, 3, 9), (512, 8, 8), (1025, 5, 17), (3073, 1, 3), (5121, 2, 10)])
+def test_expansion_edges(npw, nbasis, nblock):
+    """block Gram-Schmidt at the edges of its register tiles and panels, with a
+    vector that vanishes, against numpy (1e-10)"""
+    import torch
+    from tc_b200.context import davidson_expand
+    rng = np.random.default_rng(npw)
+    V0 = np.linalg.qr(rng.standard_normal((npw, nbasis)) + 1j * rng.standard_normal((npw, nbasis)))[0].T
+    phi = rng.standard_normal((nblock, npw)) + 1j * rng.standard_normal((nblock, npw))
+    H = rng.standard_normal((nblock, npw)) + 1j * rng.standard_normal((nblock, npw))
+    kg2 = rng.uniform(0.1, 20.0, npw)
+    eig = rng.standard_normal(nblock) + 0j
+    if nblock > 2:
+        phi[2], H[2], eig[2] = phi[1], H[1], eig[1]          # the same residual twice: dropped
+    rows = [v for v in V0]
+    for b in range(nblock):
+        x = kg2 / (np.sum(kg2 * np.abs(phi[b]) ** 2) / np.sum(np.abs(phi[b]) ** 2))
+        p = 27 + x * (18 + x * (12 + 8 * x))
+        t = -(p / (p + 16 * x ** 4)) * (H[b] - eig[b] * phi[b])
+        t /= np.linalg.norm(t)
+        for v in rows:
+            t = t - np.vdot(v, t) * v
+        if np.linalg.norm(t) >= 1e-8:
+            rows.append(t / np.linalg.norm(t))
+    V = torch.zeros((nbasis + nblock, npw), dtype=torch.complex128, device="cuda")
+    V[:nbasis] = torch.from_numpy(np.ascontiguousarray(V0)).cuda()
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    n = davidson_expand(V, nbasis, dev(phi), [dev(H)], dev(kg2), eig)
+    assert n == len(rows)
+    assert np.abs(V[:n].cpu().numpy() - np.array(rows)).max() < 1e-10
