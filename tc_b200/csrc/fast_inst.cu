@@ -12,4 +12,5 @@ namespace tcg {
 #define TCG_INST(T, OP) \
     template int run_chunk_fast<T, TCG_FAST_N, OP>(tcg_ctx *, const OP &, int, int, bool, bool);
 TCG_INST_ALL(TCG_FAST_T)
+template struct FastIO<TCG_FAST_T, TCG_FAST_N>;
 } // namespace tcg

@@ -4,6 +4,7 @@
 #include "terms.cuh"
 #include "fast.cuh"
 #include "split.cuh"
+#include "fft_split.cuh"
 
 namespace tcg {
 
@@ -92,6 +93,38 @@ int run_chunk_fast(tcg_ctx *c, const Op &op, int items, int nt, bool do_xyf, boo
     }
     }
     return TCG_OK;
+}
+
+// ---- whole transforms (fft_split.cuh)
+template <int N> using IOShape = sl::Shape<N, sl::ShapeOf<N>::A, sl::ShapeOf<N>::B>;
+template <typename T, int N> int FastIO<T, N>::xy(tcg_ctx *c, const GridDesc &g, const GridRefs &gr, unsigned n, int dir)
+{
+    using V = typename C2<T>::t;
+    using S = IOShape<N>;
+    return launch(c, dir < 0 ? sl::k_xy_io<T, S, -1> : sl::k_xy_io<T, S, +1>, dim3(N, n), dim3(S::THREADS), sl::smem_xy_io<V, S>(), g,
+                  gr);
+}
+template <typename T, int N>
+int FastIO<T, N>::z(tcg_ctx *c, const GridDesc &g, const GridRefs &gr, unsigned n, int dir, double scale)
+{
+    using V = typename C2<T>::t;
+    using S = IOShape<N>;
+    return launch(c, dir < 0 ? sl::k_z_io<T, S, -1> : sl::k_z_io<T, S, +1>, dim3((N * N + 31) / 32, n), dim3(S::ZTHREADS),
+                  sl::smem_z_io<V, S>(), g, gr, (T)scale);
+}
+template <typename T, int N> int FastIO<T, N>::sphere(tcg_ctx *c, const GridDesc &g, const SphereItem *items, unsigned n)
+{
+    using V = typename C2<T>::t;
+    using S = IOShape<N>;
+    return launch(c, sl::k_sphere_io<T, S>, dim3((N * N + 31) / 32, n), dim3(S::ZTHREADS), sl::smem_z_io<V, S>(), g, items,
+                  c->recip.as<const double>());
+}
+template <typename T, int N> int FastIO<T, N>::gather(tcg_ctx *c, const GridDesc &g, const GatherItem *items, unsigned n)
+{
+    if constexpr (sizeof(T) == 8) {
+        using S = IOShape<N>;
+        return launch(c, sl::k_gather_io<S>, dim3((N * N + 31) / 32, n), dim3(S::ZTHREADS), sl::smem_z_io<double2, S>(), g, items);
+    } else return fail(TCG_ERR_UNSUPPORTED, "accumulators are double precision");
 }
 
 } // namespace tcg

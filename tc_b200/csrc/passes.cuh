@@ -177,6 +177,24 @@ struct SphereItem {
     int mode;                // 0 plain, 1..3: multiply by (k+G)_{mode-1}
 };
 
+// value of grid point (column c = x + n0 y, plane z) of a sphere item
+template <typename V>
+__device__ __forceinline__ V sphere_value(const GridDesc &g, const SphereItem &it, const double *recip, int c, int z)
+{
+    const int ip = it.inv[(size_t)z * g.n0 * g.n1 + c];
+    if (ip < 0) return czero<V>();
+    double2 cf = it.coef[ip];
+    if (it.tr) cf.y = -cf.y;
+    cf = cmul(cf, it.phase[ip]);
+    if (it.mode > 0) {
+        const int d = it.mode - 1;
+        const int m0 = miller(c % g.n0, g.n0), m1 = miller(c / g.n0, g.n1), m2 = miller(z, g.n2);
+        const double Gd = recip[0 * 3 + d] * m0 + recip[1 * 3 + d] * m1 + recip[2 * 3 + d] * m2;
+        cf = cscale(cf, it.kc[d] + Gd);
+    }
+    return from64<V>(cf);
+}
+
 // Z pass of a backward transform, loading straight from the sphere.
 template <typename T>
 __global__ void __launch_bounds__(256) k_sphere_z(GridDesc g, const SphereItem *items, const double *recip)
@@ -192,24 +210,7 @@ __global__ void __launch_bounds__(256) k_sphere_z(GridDesc g, const SphereItem *
     const int ncol = min(ZTC, plane - c0);
     for (int e = threadIdx.x; e < tile; e += blockDim.x) {
         const int zz = e / ZTC, cc = e % ZTC;
-        V v = czero<V>();
-        if (cc < ncol) {
-            const int c = c0 + cc;
-            const size_t p = (size_t)zz * plane + c;
-            const int ip = it.inv[p];
-            if (ip >= 0) {
-                double2 cf = it.coef[ip];
-                if (it.tr) cf.y = -cf.y;
-                cf = cmul(cf, it.phase[ip]);
-                if (it.mode > 0) {
-                    const int d = it.mode - 1;
-                    const int m0 = miller(c % g.n0, g.n0), m1 = miller(c / g.n0, g.n1), m2 = miller(zz, g.n2);
-                    const double Gd = recip[0 * 3 + d] * m0 + recip[1 * 3 + d] * m1 + recip[2 * 3 + d] * m2;
-                    cf = cscale(cf, it.kc[d] + Gd);
-                }
-                v = from64<V>(cf);
-            }
-        }
+        const V v = cc < ncol ? sphere_value<V>(g, it, recip, c0 + cc, zz) : czero<V>();
         A[e] = v;
     }
     __syncthreads();

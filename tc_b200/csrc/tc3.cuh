@@ -754,13 +754,12 @@ static int finalize_acc(tcg_ctx *c, const Targets &T, double2 *acc, double2 *hou
     void **d_grids = reinterpret_cast<void **>(d_gi + nt);
     TCG_CUDA(cudaMemcpyAsync(d_grids, grids.data(), nt * sizeof(void *), cudaMemcpyHostToDevice, c->stream));
     TCG_CUDA(cudaMemcpyAsync(d_gi, gi.data(), nt * sizeof(GatherItem), cudaMemcpyHostToDevice, c->stream));
-    const int ntiles = (g.n0 * g.n1 + ZTC - 1) / ZTC;
     for (size_t b0 = 0; b0 < nt; b0 += 65535) {
         const unsigned nb = (unsigned)std::min<size_t>(65535, nt - b0);
         GridRefs gr;
         gr.dev = d_grids + b0;
-        TRY(launch(c, k_xy_inplace<double, -1>, dim3(g.n2, nb), dim3(256), smem_xy<double2>(g), g, gr));
-        TRY(launch(c, k_gather_z, dim3(ntiles, nb), dim3(256), smem_z<double2>(g, 0), g, (const GatherItem *)(d_gi + b0)));
+        TRY((grids_xy<double, -1>(c, g, gr, nb)));
+        TRY(gather_z(c, g, d_gi + b0, nb));
     }
     TCG_CUDA(cudaStreamSynchronize(c->stream));
     return TCG_OK;

@@ -72,14 +72,63 @@ __device__ __forceinline__ void acc_red(double2 *a, double2 v, double f)
     atomicAdd(&a->y, f * v.y);
 }
 
+// ------------------------------------------------- transforms of whole grids --
+// The four passes of a list of transforms: on the compiled cubic sizes in split
+// lines (fft_split.cuh, instantiated with the pair passes), else generic.
+template <typename T, int N> struct FastIO {
+    static int xy(tcg_ctx *c, const GridDesc &g, const GridRefs &gr, unsigned n, int dir);
+    static int z(tcg_ctx *c, const GridDesc &g, const GridRefs &gr, unsigned n, int dir, double scale);
+    static int sphere(tcg_ctx *c, const GridDesc &g, const SphereItem *items, unsigned n);
+    static int gather(tcg_ctx *c, const GridDesc &g, const GatherItem *items, unsigned n);
+};
+static bool io_fast(const tcg_ctx *c, const GridDesc &g)
+{
+    return !c->force_generic && g.n0 == g.n1 && g.n1 == g.n2 && fast_grid(g.n0);
+}
+#define TCG_IO(T, call)                                                    \
+    if (io_fast(c, g)) {                                                   \
+        switch (g.n0) {                                                    \
+        TCG_FAST_SIZES(TCG_IO_CASE)                                        \
+        default: break;                                                    \
+        }                                                                  \
+    }
+template <typename T, int DIR> static int grids_xy(tcg_ctx *c, const GridDesc &g, const GridRefs &gr, unsigned n)
+{
+#define TCG_IO_CASE(m) case m: return FastIO<T, m>::xy(c, g, gr, n, DIR);
+    TCG_IO(T, xy)
+#undef TCG_IO_CASE
+    return launch(c, k_xy_inplace<T, DIR>, dim3(g.n2, n), dim3(256), smem_xy<typename C2<T>::t>(g), g, gr);
+}
+template <typename T, int DIR> static int grids_z(tcg_ctx *c, const GridDesc &g, const GridRefs &gr, unsigned n, double scale)
+{
+#define TCG_IO_CASE(m) case m: return FastIO<T, m>::z(c, g, gr, n, DIR, scale);
+    TCG_IO(T, z)
+#undef TCG_IO_CASE
+    return launch(c, k_z_inplace<T, DIR>, dim3((g.n0 * g.n1 + ZTC - 1) / ZTC, n), dim3(256), smem_z<typename C2<T>::t>(g, 0), g, gr,
+                  scale);
+}
+template <typename T> static int sphere_z(tcg_ctx *c, const GridDesc &g, const SphereItem *items, unsigned n)
+{
+#define TCG_IO_CASE(m) case m: return FastIO<T, m>::sphere(c, g, items, n);
+    TCG_IO(T, sphere)
+#undef TCG_IO_CASE
+    return launch(c, k_sphere_z<T>, dim3((g.n0 * g.n1 + ZTC - 1) / ZTC, n), dim3(256), smem_z<typename C2<T>::t>(g, 0), g, items,
+                  c->recip.as<const double>());
+}
+static int gather_z(tcg_ctx *c, const GridDesc &g, const GatherItem *items, unsigned n)
+{
+#define TCG_IO_CASE(m) case m: return FastIO<double, m>::gather(c, g, items, n);
+    TCG_IO(double, gather)
+#undef TCG_IO_CASE
+    return launch(c, k_gather_z, dim3((g.n0 * g.n1 + ZTC - 1) / ZTC, n), dim3(256), smem_z<double2>(g, 0), g, items);
+}
+
 // ---------------------------------------------------------------- sphere --
 template <typename T>
 static int sphere_to_r(tcg_ctx *c, const std::vector<SphereItem> &items)
 {
-    using V = typename C2<T>::t;
     const GridDesc &g = c->gd;
     if (items.empty()) return TCG_OK;
-    const int nz_tiles = (g.n0 * g.n1 + ZTC - 1) / ZTC;
     const size_t n = items.size();
     std::vector<void *> outs(n);
     for (size_t i = 0; i < n; i++) outs[i] = items[i].out;
@@ -90,11 +139,10 @@ static int sphere_to_r(tcg_ctx *c, const std::vector<SphereItem> &items)
     TCG_CUDA(cudaMemcpyAsync(d_outs, outs.data(), n * sizeof(void *), cudaMemcpyHostToDevice, c->stream));
     for (size_t b0 = 0; b0 < n; b0 += 65535) {
         const unsigned nb = (unsigned)std::min<size_t>(65535, n - b0);
-        TRY(launch(c, k_sphere_z<T>, dim3(nz_tiles, nb), dim3(256), smem_z<V>(g, 0), g,
-                   (const SphereItem *)(d_items + b0), c->recip.as<const double>()));
+        TRY(sphere_z<T>(c, g, d_items + b0, nb));
         GridRefs gr;
         gr.dev = d_outs + b0;
-        TRY(launch(c, k_xy_inplace<T, +1>, dim3(g.n2, nb), dim3(256), smem_xy<V>(g), g, gr));
+        TRY((grids_xy<T, +1>(c, g, gr, nb)));
     }
     TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->items is reused by the next caller
     return TCG_OK;
@@ -104,17 +152,15 @@ static int sphere_to_r(tcg_ctx *c, const std::vector<SphereItem> &items)
 template <typename T, int DIR>
 static int fft3_list(tcg_ctx *c, const std::vector<void *> &grids, const GridDesc *on = nullptr)
 {
-    using V = typename C2<T>::t;
     const GridDesc &g = on ? *on : c->gd;
     if (grids.empty()) return TCG_OK;
     const size_t n = grids.size();
-    const int ntiles = (g.n0 * g.n1 + ZTC - 1) / ZTC;
     const double scale = DIR < 0 ? 1.0 / (double)g.N : 1.0;
     if (n <= 8) {   // pointers by value: nothing to upload, nothing to wait for
         GridRefs gr;
         for (size_t i = 0; i < n; i++) gr.inl[i] = grids[i];
-        TRY(launch(c, k_xy_inplace<T, DIR>, dim3(g.n2, (unsigned)n), dim3(256), smem_xy<V>(g), g, gr));
-        return launch(c, k_z_inplace<T, DIR>, dim3(ntiles, (unsigned)n), dim3(256), smem_z<V>(g, 0), g, gr, scale);
+        TRY((grids_xy<T, DIR>(c, g, gr, (unsigned)n)));
+        return grids_z<T, DIR>(c, g, gr, (unsigned)n, scale);
     }
     TRY(c->items.ensure(n * sizeof(void *)));
     void **d = c->items.as<void *>();
@@ -123,8 +169,8 @@ static int fft3_list(tcg_ctx *c, const std::vector<void *> &grids, const GridDes
         const unsigned nb = (unsigned)std::min<size_t>(65535, n - b0);
         GridRefs gr;
         gr.dev = d + b0;
-        TRY(launch(c, k_xy_inplace<T, DIR>, dim3(g.n2, nb), dim3(256), smem_xy<V>(g), g, gr));
-        TRY(launch(c, k_z_inplace<T, DIR>, dim3(ntiles, nb), dim3(256), smem_z<V>(g, 0), g, gr, scale));
+        TRY((grids_xy<T, DIR>(c, g, gr, nb)));
+        TRY((grids_z<T, DIR>(c, g, gr, nb, scale)));
     }
     TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->items is reused by the next caller
     return TCG_OK;
@@ -136,15 +182,14 @@ static int fft3_strided(tcg_ctx *c, typename C2<T>::t *first, size_t n)
 {
     using V = typename C2<T>::t;
     const GridDesc &g = c->gd;
-    const int ntiles = (g.n0 * g.n1 + ZTC - 1) / ZTC;
     const double scale = DIR < 0 ? 1.0 / (double)g.N : 1.0;
     for (size_t b0 = 0; b0 < n; b0 += 65535) {
         const unsigned nb = (unsigned)std::min<size_t>(65535, n - b0);
         GridRefs gr;
         gr.base = reinterpret_cast<char *>(first + b0 * g.N);
         gr.stride = (size_t)g.N * sizeof(V);
-        TRY(launch(c, k_xy_inplace<T, DIR>, dim3(g.n2, nb), dim3(256), smem_xy<V>(g), g, gr));
-        TRY(launch(c, k_z_inplace<T, DIR>, dim3(ntiles, nb), dim3(256), smem_z<V>(g, 0), g, gr, scale));
+        TRY((grids_xy<T, DIR>(c, g, gr, nb)));
+        TRY((grids_z<T, DIR>(c, g, gr, nb, scale)));
     }
     return TCG_OK;
 }
