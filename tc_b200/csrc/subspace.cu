@@ -2,16 +2,17 @@
 // device, in FP64 (Diagonalization::block_davidson, diagonalization_davidson.cpp:
 // 462-600; diagonalization_utils.cpp:7-119):
 //   tcg_subspace_ritz   H_n,sub = Vref^H (H_n V) (ZGEMM), H_sub = sum_n H_n,sub,
-//                       H_sub X = X D (general complex eigensolve, cuSOLVER
-//                       Xgeev), eigenpairs sorted by the real part, X^-1 (LU),
-//                       Ritz vectors V X and left vectors Vref (X^-1)^H (ZGEMM),
+//                       H_sub X = X D (general complex eigensolve, in one CTA
+//                       up to order EIG_MAX, cuSOLVER Xgeev beyond), eigenpairs
+//                       sorted by the real part, X^-1 (LU), Ritz vectors V X and
+//                       left vectors Vref (X^-1)^H (ZGEMM),
 //                       energies diag(Xl^H H_n,sub X)
 //   tcg_gram_schmidt    Gram_Schmidt / Gram_Schmidt_biortho of a block of vectors
 //   tcg_davidson_expand the new trial vectors of one block: preconditioned
 //                       residuals (make_a_new_trial_vector), each orthonormalised
 //                       against the basis and appended unless it vanishes
 // The band-by-band contractions are plain library GEMMs (cuBLAS ZGEMM runs
-// them on the FP64 tensor pipe); the eigensolve and LU are cuSOLVER.
+// them on the FP64 tensor pipe); the LU is cuSOLVER's.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -69,6 +70,31 @@ struct Handles {
 };
 std::mutex g_mu;
 Handles g_h[64];
+cudaMemPool_t g_pool[64];
+
+// Scratch of the calls comes from a stream-ordered pool per device (safe for
+// several threads and streams) that keeps at most 64 MB between calls; cudaMalloc
+// and cudaFree took 2 of the 2.5 ms of an expansion.
+int scratch_pool(cudaMemPool_t *out)
+{
+    int dev = 0;
+    SUB_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(TCG_ERR_UNSUPPORTED, "device index >= 64");
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool;
+        SUB_CUDA(cudaMemPoolCreate(&pool, &props));
+        unsigned long long keep = 64ull << 20;
+        SUB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        g_pool[dev] = pool;
+    }
+    *out = g_pool[dev];
+    return TCG_OK;
+}
 
 int handles(Handles **out)
 {
@@ -86,23 +112,28 @@ int handles(Handles **out)
     return TCG_OK;
 }
 
-// scratch of one call: one device allocation, parts handed out in order, freed on return
+// scratch of one call: one allocation on the call's stream, parts handed out in order, freed on return
 struct Scratch {
     char *base = nullptr;
     size_t used = 0, cap = 0;
+    cudaStream_t st;
+    explicit Scratch(cudaStream_t s) : st(s) {}
     ~Scratch()
     {
-        if (base) cudaFree(base);
+        if (base) cudaFreeAsync(base, st);
     }
     static size_t part(size_t bytes) { return (std::max<size_t>(bytes, 16) + 255) / 256 * 256; }
     int reserve(size_t bytes)
     {
-        if (cudaMalloc((void **)&base, std::max<size_t>(bytes, 256)) != cudaSuccess) {
+        cudaMemPool_t pool;
+        const int rc = scratch_pool(&pool);
+        if (rc) return rc;
+        cap = std::max<size_t>(bytes, 256);
+        if (cudaMallocFromPoolAsync((void **)&base, cap, pool, st) != cudaSuccess) {
             cudaGetLastError();
             base = nullptr;
             return fail(TCG_ERR_NOMEM, "device allocation failed");
         }
-        cap = std::max<size_t>(bytes, 256);
         return TCG_OK;
     }
     template <typename X> X *get(size_t n)
@@ -425,6 +456,319 @@ int mgs(int nv, int npw, double2 *V, double2 *T, int nbasis, int *ints, int *row
     return TCG_OK;
 }
 
+// ------------------------------------------- eigenproblem of small matrices --
+// General complex eigenproblem A X = X D of order n <= EIG_MAX in one CTA: the
+// matrix in shared memory, Householder reduction to Hessenberg form, explicit
+// single-shift QR (the iteration of the EISPACK routine COMQR2, Peters and
+// Wilkinson 1970, with the deflation test of Ahues and Tisseur 1997), triangular
+// back substitution.  The rows of a sweep are a wavefront: the thread of column k
+// carries its running element in a register, forms rotation k as soon as rotation
+// k - 1 has arrived, and one barrier later every column applies it.  The columns
+// (and Z, by the other half of the CTA) then need no barrier at all: a thread
+// walks its own row.  What bounds it is the chain of some n^2 rotations (one
+// reciprocal root and a barrier each).  An implicit sweep with two barriers and
+// three roots per rotation took 13 ms at n = 96, this one 6.1; the library
+// eigensolve, which splits the work between host and device, takes 15 to 37 ms.
+constexpr int EIG_MAX = 112, ET = 256;   // threads 0-127: rows / columns of H; 128-255: rows of Z
+
+__device__ __forceinline__ double2 zadd(double2 a, double2 b) { return {a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ double2 zsub(double2 a, double2 b) { return {a.x - b.x, a.y - b.y}; }
+__device__ __forceinline__ double2 zmul(double2 a, double2 b) { return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x}; }
+__device__ __forceinline__ double2 zmulc(double2 a, double2 b) { return {a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x}; }  // conj(a) b
+__device__ __forceinline__ double zabs1(double2 a) { return fabs(a.x) + fabs(a.y); }
+__device__ __forceinline__ double zabs(double2 a) { return sqrt(a.x * a.x + a.y * a.y); }
+// a / b without overflow of |b|^2 (Smith 1962)
+__device__ __forceinline__ double2 zdiv(double2 a, double2 b)
+{
+    if (fabs(b.x) >= fabs(b.y)) {
+        const double r = b.y / b.x, d = b.x + b.y * r;
+        return {(a.x + a.y * r) / d, (a.y - a.x * r) / d};
+    }
+    const double r = b.x / b.y, d = b.x * r + b.y;
+    return {(a.x * r + a.y) / d, (a.y * r - a.x) / d};
+}
+__device__ __forceinline__ double2 zsqrt(double2 a)
+{
+    if (a.x == 0.0 && a.y == 0.0) return {0.0, 0.0};
+    const double t = sqrt(0.5 * (fabs(a.x) + zabs(a)));
+    if (a.x >= 0.0) return {t, a.y / (2.0 * t)};
+    return {fabs(a.y) / (2.0 * t), copysign(t, a.y)};
+}
+
+// A: n x n (column-major, overwritten work copy not needed afterwards); w [n]:
+// eigenvalues; VR [n x n]: eigenvectors, unit norm, largest component real and
+// positive; Z [n x n]: scratch; info: 0, or > 0 when the iteration did not
+// converge or a result is not finite
+__global__ void __launch_bounds__(ET) k_eig(int n, const double2 *A, double2 *w, double2 *VR, double2 *Z, int *info)
+{
+    extern __shared__ __align__(16) unsigned char eig_smem[];
+    const int ld = n | 1, t = threadIdx.x, lane = t & 31, warp = t >> 5, r0 = t & 127;
+    const bool zside = t >= 128;
+    double2 *H = reinterpret_cast<double2 *>(eig_smem);     // H[r + ld c]
+    double2 *vec = H + (size_t)ld * n;                       // [ET / 32][EIG_MAX] vectors
+    __shared__ double red[ET / 32];
+    __shared__ int ired[ET / 32];
+    const double ulp = 2.220446049250313e-16, tiny = 2.2250738585072014e-308 / ulp * n;
+    auto h = [&](int r, int c) -> double2 & { return H[r + ld * c]; };
+    for (int i = t; i < n * n; i += ET) {
+        h(i % n, i / n) = A[i];
+        Z[i] = make_double2(i % n == i / n ? 1.0 : 0.0, 0.0);
+    }
+    __syncthreads();
+    auto sum = [&](double x) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        __syncthreads();
+        if (lane == 0) red[warp] = x;
+        __syncthreads();
+        double s = 0;
+#pragma unroll
+        for (int i = 0; i < ET / 32; i++) s += red[i];
+        return s;
+    };
+    // ---- Hessenberg: reflectors I - tau v v^H, v[k + 1] = 1, on rows and columns k + 1 ...
+    for (int k = 0; k + 2 < n; k++) {
+        const bool in = t > k + 1 && t < n;
+        const double2 x = in ? h(t, k) : double2{0, 0}, al = h(k + 1, k);
+        const double xn = sum(x.x * x.x + x.y * x.y);
+        if (xn == 0.0 && al.y == 0.0) continue;              // uniform
+        const double beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn), al.x);
+        const double2 tau = {(beta - al.x) / beta, -al.y / beta};
+        const double2 sc = zdiv(double2{1.0, 0.0}, double2{al.x - beta, al.y});
+        __syncthreads();
+        if (t == k + 1) vec[t] = {1.0, 0.0};
+        if (in) vec[t] = zmul(sc, x);
+        __syncthreads();
+        // right: H <- H (I - tau v v^H) and Z <- Z (I - tau v v^H), thread = row
+        if (r0 < n) {
+            double2 *M = zside ? Z + r0 : H + r0;
+            const int lm = zside ? n : ld;
+            double2 a = {0, 0};
+            for (int c = k + 1; c < n; c++) a = zadd(a, zmul(M[(size_t)lm * c], vec[c]));
+            a = zmul(tau, a);
+            for (int c = k + 1; c < n; c++)
+                M[(size_t)lm * c] = zsub(M[(size_t)lm * c], zmul(a, double2{vec[c].x, -vec[c].y}));
+        }
+        __syncthreads();
+        // left: H <- (I - conj(tau) v v^H) H, thread = column
+        if (t >= k && t < n) {
+            double2 a = {0, 0};
+            for (int r = k + 1; r < n; r++) a = zadd(a, zmulc(vec[r], h(r, t)));
+            a = zmulc(tau, a);
+            for (int r = k + 1; r < n; r++) h(r, t) = zsub(h(r, t), zmul(vec[r], a));
+        }
+        __syncthreads();
+        if (t > k + 1 && t < n) h(t, k) = {0, 0};
+        __syncthreads();
+    }
+    // ---- QR iteration
+    int fail = 0, i = n - 1, its = 0;
+    const int maxit = 40 * (n > 10 ? n : 10);
+    for (int total = 0; i >= 0; total++) {
+        if (total > maxit) {
+            fail = 1;
+            break;
+        }
+        // largest k <= i whose subdiagonal element is negligible (0: none)
+        int k = 0;
+        if (t >= 1 && t <= i) {
+            const double2 s = h(t, t - 1);
+            bool small = zabs1(s) <= tiny;
+            if (!small) {
+                double tst = zabs1(h(t - 1, t - 1)) + zabs1(h(t, t));
+                if (tst == 0.0) {
+                    if (t >= 2) tst += zabs1(h(t - 1, t - 2));
+                    if (t + 1 <= i) tst += zabs1(h(t + 1, t));
+                }
+                if (zabs1(s) <= ulp * tst) {
+                    const double p = zabs1(s), q = zabs1(h(t - 1, t)), d = zabs1(h(t, t)), e = zabs1(zsub(h(t - 1, t - 1), h(t, t)));
+                    const double ab = fmax(p, q), ba = fmin(p, q), aa = fmax(d, e), bb = fmin(d, e), q2 = aa + ab;
+                    small = ba * (ab / q2) <= fmax(tiny, ulp * (bb * (aa / q2)));
+                }
+            }
+            if (small) k = t;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
+        __syncthreads();
+        if (lane == 0) ired[warp] = k;
+        __syncthreads();
+        int l = 0;
+#pragma unroll
+        for (int q = 0; q < ET / 32; q++) l = max(l, ired[q]);
+        if (l > 0 && t == 0) h(l, l - 1) = {0, 0};
+        if (l >= i) {
+            i--;
+            its = 0;
+            __syncthreads();
+            continue;
+        }
+        its++;
+        // shift
+        double2 sh;
+        if (its % 30 == 10) {
+            sh = h(l, l);
+            sh.x += 0.75 * fabs(h(l + 1, l).x) + 0.75 * fabs(h(l + 1, l).y);
+        } else if (its % 30 == 20) {
+            sh = h(i, i);
+            sh.x += 0.75 * fabs(h(i, i - 1).x) + 0.75 * fabs(h(i, i - 1).y);
+        } else {
+            sh = h(i, i);
+            const double2 u = zmul(zsqrt(h(i - 1, i)), zsqrt(h(i, i - 1)));
+            double s = zabs1(u);
+            if (s != 0.0) {
+                const double2 d = zsub(h(i - 1, i - 1), sh), x = {0.5 * d.x, 0.5 * d.y};
+                const double sx = zabs1(x);
+                s = fmax(s, sx);
+                const double2 xs = {x.x / s, x.y / s}, us = {u.x / s, u.y / s};
+                double2 y = zsqrt(zadd(zmul(xs, xs), zmul(us, us)));
+                y = {s * y.x, s * y.y};
+                if (sx > 0.0 && (x.x / sx) * y.x + (x.y / sx) * y.y < 0.0) y = {-y.x, -y.y};
+                sh = zsub(sh, zmul(u, zdiv(u, zadd(x, y))));
+            }
+        }
+        __syncthreads();                                      // the shift's elements have been read
+        // rows: G_k (k = l ... i - 1) on rows k, k + 1 of H - sh, thread = column; p = the running
+        // element of row k.  Thread k forms G_k = 1/r [conj(a) conj(b); -b a] from its column.
+        double2 p = {0, 0};
+        if (t >= l && t < n) p = h(l, t);
+        if (t == l) p = zsub(p, sh);
+        for (int k2 = l; k2 < i; k2++) {
+            double2 q = {0, 0};
+            if (t >= k2 && t < n) q = h(k2 + 1, t);
+            if (t == k2 + 1) q = zsub(q, sh);
+            if (t == k2) {
+                double2 a = p, b = q;
+                double n2 = a.x * a.x + a.y * a.y + (b.x * b.x + b.y * b.y), s = 1.0;
+                if (!(n2 > 1e-280 && n2 < 1e280)) {
+                    s = fmax(fmax(fabs(a.x), fabs(a.y)), fmax(fabs(b.x), fabs(b.y)));
+                    if (s > 0.0 && isfinite(s)) {
+                        a = {a.x / s, a.y / s};
+                        b = {b.x / s, b.y / s};
+                    } else {
+                        a = {1.0, 0.0};
+                        b = {0.0, 0.0};
+                    }
+                    n2 = a.x * a.x + a.y * a.y + (b.x * b.x + b.y * b.y);
+                }
+                const double ir = rsqrt(n2);
+                vec[k2] = {a.x * ir, a.y * ir};
+                vec[EIG_MAX + k2] = {b.x * ir, b.y * ir};
+                h(k2, k2) = {s * (n2 * ir), 0.0};
+                h(k2 + 1, k2) = {0, 0};
+            }
+            __syncthreads();
+            if (t > k2 && t < n) {
+                const double2 ca = vec[k2], cb = vec[EIG_MAX + k2];
+                h(k2, t) = zadd(zmulc(ca, p), zmulc(cb, q));
+                p = zsub(zmul(ca, q), zmul(cb, p));
+            }
+        }
+        if (t >= i && t < n) h(i, t) = p;
+        __syncthreads();
+        // columns: G_k^H on columns k, k + 1 of H (rows 0 ... i) and Z, thread = row; x = the
+        // running element of column k, the columns after it on their way
+        {
+            const int rows = zside ? n : i + 1;
+            if (r0 < rows) {
+                double2 *M = zside ? Z + r0 : H + r0;
+                const size_t lm = zside ? n : ld;
+                const int kb = zside ? l : max(l, r0 - 1);
+                double2 x = M[lm * kb], y[4];
+                int k2 = kb;
+                const bool dg = !zside && r0 >= l;
+                auto step = [&](double2 yk) {
+                    const double2 ca = vec[k2], cb = vec[EIG_MAX + k2];
+                    double2 f = zadd(zmul(x, ca), zmul(yk, cb));
+                    if (dg && k2 == r0) f = zadd(f, sh);
+                    M[lm * k2] = f;
+                    x = zsub(zmulc(ca, yk), zmulc(cb, x));
+                    k2++;
+                };
+#pragma unroll
+                for (int m = 0; m < 4; m++)
+                    if (kb + 1 + m <= i) y[m] = M[lm * (kb + 1 + m)];
+                while (k2 + 4 <= i) {
+#pragma unroll
+                    for (int m = 0; m < 4; m++) {
+                        const double2 yk = y[m];
+                        if (k2 + 5 <= i) y[m] = M[lm * (k2 + 5)];
+                        step(yk);
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < 4; m++)
+                    if (k2 < i) step(y[m]);
+                if (dg && r0 == i) x = zadd(x, sh);
+                M[lm * i] = x;
+            }
+        }
+        __syncthreads();
+    }
+    // ---- eigenvalues and vectors
+    if (!fail) {
+        if (t < n) w[t] = h(t, t);
+        double2 *x = vec + warp * EIG_MAX;
+        bool bad = false;
+        for (int k = warp; k < n; k += ET / 32) {
+            const double2 lam = h(k, k);
+            const double smin = fmax(ulp * zabs1(lam), tiny);
+            for (int r = lane; r <= k; r += 32) x[r] = r == k ? double2{1.0, 0.0} : double2{-h(r, k).x, -h(r, k).y};
+            __syncwarp();
+            for (int j = k - 1; j >= 0; j--) {
+                double2 d = zsub(h(j, j), lam);
+                if (zabs1(d) < smin) d = {smin, 0.0};
+                const double2 xj = zdiv(x[j], d);
+                __syncwarp();
+                if (lane == 0) x[j] = xj;
+                for (int r = lane; r < j; r += 32) x[r] = zsub(x[r], zmul(xj, h(r, j)));
+                __syncwarp();
+            }
+            double2 v[(EIG_MAX + 31) / 32];
+            double nrm = 0, big = -1.0;
+            int at = 0;
+#pragma unroll
+            for (int e = 0; e < (EIG_MAX + 31) / 32; e++) {
+                const int r = lane + 32 * e;
+                v[e] = {0, 0};
+                if (r < n) {
+                    for (int j = 0; j <= k; j++) v[e] = zadd(v[e], zmul(Z[r + (size_t)n * j], x[j]));
+                    const double m = v[e].x * v[e].x + v[e].y * v[e].y;
+                    nrm += m;
+                    if (m > big) { big = m; at = r; }
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+                const double ob = __shfl_xor_sync(0xffffffffu, big, o);
+                const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+                if (ob > big || (ob == big && oa < at)) { big = ob; at = oa; }
+            }
+            double2 top = {0, 0};
+#pragma unroll
+            for (int e = 0; e < (EIG_MAX + 31) / 32; e++)
+                if (lane + 32 * e == at) top = v[e];
+            top.x = __shfl_sync(0xffffffffu, top.x, at & 31);
+            top.y = __shfl_sync(0xffffffffu, top.y, at & 31);
+            const double nn = sqrt(nrm), bt = sqrt(big);
+            const double2 f = {top.x / bt / nn, -top.y / bt / nn};
+            bad = bad || !isfinite(f.x) || !isfinite(f.y) || !isfinite(nn);
+#pragma unroll
+            for (int e = 0; e < (EIG_MAX + 31) / 32; e++) {
+                const int r = lane + 32 * e;
+                double2 o = zmul(v[e], f);
+                if (r == at) o.y = 0.0;
+                if (r < n) VR[r + (size_t)n * k] = o;
+            }
+            __syncwarp();
+        }
+        if (bad) fail = 2;
+    }
+    fail = __syncthreads_or(fail);
+    if (t == 0) *info = fail;
+}
+
 // make_a_new_trial_vector (diagonalization_utils.cpp:165-211) for vector b
 // of a block, one CTA each: with the kinetic expectation
 // t = <phi| |k+G|^2 |phi> / <phi|phi> and x = |k+G|^2 / t, the Payne
@@ -494,7 +838,7 @@ extern "C" int tcg_davidson_expand(int32_t nbasis, int32_t nblock, int32_t npw, 
     *nbasis_out = nbasis;
     if (nblock == 0) return TCG_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    Scratch S;
+    Scratch S(st);
     int rc;
     const size_t nt = (size_t)nblock * npw;
     if ((rc = S.reserve(Scratch::part(nt * sizeof(double2)) + Scratch::part(nblock * sizeof(double2)) +
@@ -529,20 +873,15 @@ extern "C" int tcg_subspace_ritz(int32_t ndim, int32_t npw, int32_t nout, int32_
     cudaStream_t st = (cudaStream_t)stream;
     SUB_BLAS(cublasSetStream(hd->blas, st));
     SUB_SOLV(cusolverDnSetStream(hd->solver, st));
-    Scratch S;
+    Scratch S(st);
     const size_t nn = (size_t)ndim * ndim;
     const void *HV[3] = {H1V, H2V, H3V};
-    // workspace sizes of the eigensolve and the LU (the matrix arguments are not read)
-    size_t dws = 0, hws = 0;
+    // workspace size of the LU (the matrix argument is not read)
     int lwork = 0;
-    SUB_SOLV(cusolverDnXgeev_bufferSize(hd->solver, hd->params, CUSOLVER_EIG_MODE_NOVECTOR, CUSOLVER_EIG_MODE_VECTOR,
-                                        ndim, CUDA_C_64F, nullptr, ndim, CUDA_C_64F, nullptr, CUDA_C_64F, nullptr, ndim,
-                                        CUDA_C_64F, nullptr, ndim, CUDA_C_64F, &dws, &hws));
     SUB_SOLV(cusolverDnZgetrf_bufferSize(hd->solver, ndim, ndim, nullptr, ndim, &lwork));
     if ((rc = S.reserve(9 * Scratch::part(nn * sizeof(double2)) + Scratch::part(ndim * sizeof(double2)) +
-                        Scratch::part(3 * (size_t)ndim * sizeof(double2)) + Scratch::part(dws) +
-                        Scratch::part((size_t)lwork * sizeof(double2)) + 2 * Scratch::part(ndim * sizeof(int)) +
-                        Scratch::part(64 * sizeof(int)))))
+                        Scratch::part(3 * (size_t)ndim * sizeof(double2)) + Scratch::part((size_t)lwork * sizeof(double2)) +
+                        2 * Scratch::part(ndim * sizeof(int)) + Scratch::part(64 * sizeof(int)))))
         return rc;
     double2 *Hn[3] = {nullptr, nullptr, nullptr};
     for (int n = 0; n < 3; n++)
@@ -550,7 +889,7 @@ extern "C" int tcg_subspace_ritz(int32_t ndim, int32_t npw, int32_t nout, int32_
     double2 *H = S.get<double2>(nn), *A = S.get<double2>(nn), *VR = S.get<double2>(nn), *X = S.get<double2>(nn);
     double2 *Xinv = S.get<double2>(nn), *XL = S.get<double2>(nn), *W = S.get<double2>(ndim);
     double2 *E = S.get<double2>(3 * (size_t)ndim);
-    void *dwork = S.get<char>(dws), *lw = S.get<double2>(lwork);
+    void *lw = S.get<double2>(lwork);
     int *dinfo = S.get<int>(64), *dperm = S.get<int>(ndim), *ipiv = S.get<int>(ndim);
     // H_n,sub(i, j) = <Vref_i | H_n V_j>   (diagonalization_davidson.cpp:462-475)
     const cuDoubleComplex one = make_cuDoubleComplex(1, 0), zero = make_cuDoubleComplex(0, 0);
@@ -560,18 +899,36 @@ extern "C" int tcg_subspace_ritz(int32_t ndim, int32_t npw, int32_t nout, int32_
                                  npw, (const cuDoubleComplex *)HV[n], npw, &zero, (cuDoubleComplex *)Hn[n], ndim));
     k_add3<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>((int)nn, Hn[0], Hn[1], Hn[2], H);
     SUB_CUDA(cudaGetLastError());
-    SUB_CUDA(cudaMemcpyAsync(A, H, nn * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-    // H_sub X = X D (ComplexEigenSolver, :479-486)
-    std::vector<unsigned char> hwork(std::max<size_t>(hws, 16));
-    SUB_SOLV(cusolverDnXgeev(hd->solver, hd->params, CUSOLVER_EIG_MODE_NOVECTOR, CUSOLVER_EIG_MODE_VECTOR, ndim,
-                             CUDA_C_64F, A, ndim, CUDA_C_64F, W, CUDA_C_64F, nullptr, ndim, CUDA_C_64F, VR, ndim,
-                             CUDA_C_64F, dwork, dws, hwork.data(), hws, dinfo));
-    int info = 0;
+    // H_sub X = X D (ComplexEigenSolver, :479-486): in one CTA up to order EIG_MAX (what its
+    // shared memory holds), by cuSOLVER beyond and where that iteration does not converge
+    int info = -1;
     std::vector<double2> w(ndim);
-    SUB_CUDA(cudaMemcpyAsync(&info, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
-    SUB_CUDA(cudaMemcpyAsync(w.data(), W, ndim * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    SUB_CUDA(cudaStreamSynchronize(st));
-    if (info != 0) return fail(TCG_ERR_NUMERIC, "diagonalization of H_subspace failed");
+    if (ndim <= EIG_MAX) {
+        const size_t sm = ((size_t)(ndim | 1) * ndim + ET / 32 * EIG_MAX) * sizeof(double2);
+        SUB_CUDA(cudaFuncSetAttribute(k_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 256));
+        k_eig<<<1, ET, sm, st>>>(ndim, H, W, VR, Xinv, dinfo);
+        SUB_CUDA(cudaGetLastError());
+        SUB_CUDA(cudaMemcpyAsync(&info, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
+        SUB_CUDA(cudaMemcpyAsync(w.data(), W, ndim * sizeof(double2), cudaMemcpyDeviceToHost, st));
+        SUB_CUDA(cudaStreamSynchronize(st));
+    }
+    if (info != 0) {
+        size_t dws = 0, hws = 0;
+        SUB_SOLV(cusolverDnXgeev_bufferSize(hd->solver, hd->params, CUSOLVER_EIG_MODE_NOVECTOR, CUSOLVER_EIG_MODE_VECTOR,
+                                            ndim, CUDA_C_64F, A, ndim, CUDA_C_64F, W, CUDA_C_64F, nullptr, ndim, CUDA_C_64F,
+                                            VR, ndim, CUDA_C_64F, &dws, &hws));
+        Scratch S2(st);
+        if ((rc = S2.reserve(Scratch::part(dws)))) return rc;
+        std::vector<unsigned char> hwork(std::max<size_t>(hws, 16));
+        SUB_CUDA(cudaMemcpyAsync(A, H, nn * sizeof(double2), cudaMemcpyDeviceToDevice, st));
+        SUB_SOLV(cusolverDnXgeev(hd->solver, hd->params, CUSOLVER_EIG_MODE_NOVECTOR, CUSOLVER_EIG_MODE_VECTOR, ndim,
+                                 CUDA_C_64F, A, ndim, CUDA_C_64F, W, CUDA_C_64F, nullptr, ndim, CUDA_C_64F, VR, ndim,
+                                 CUDA_C_64F, S2.get<char>(dws), dws, hwork.data(), hws, dinfo));
+        SUB_CUDA(cudaMemcpyAsync(&info, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
+        SUB_CUDA(cudaMemcpyAsync(w.data(), W, ndim * sizeof(double2), cudaMemcpyDeviceToHost, st));
+        SUB_CUDA(cudaStreamSynchronize(st));
+        if (info != 0) return fail(TCG_ERR_NUMERIC, "diagonalization of H_subspace failed");
+    }
     // sort by the real part, ascending (sort_eigen, diagonalization_utils.cpp:82-119)
     std::vector<int> perm(ndim);
     std::iota(perm.begin(), perm.end(), 0);
@@ -625,7 +982,7 @@ extern "C" int tcg_gram_schmidt(int32_t nvec, int32_t npw, void *V, void *Vl, vo
     if (nvec < 0 || npw < 1 || !V) return fail(TCG_ERR_ARG, "bad Gram-Schmidt arguments");
     cudaStream_t st = (cudaStream_t)stream;
     if (nvec == 0) return TCG_OK;
-    Scratch S;
+    Scratch S(st);
     int rc;
     double2 *v = (double2 *)V, *l = (double2 *)Vl;
     if (!l) {

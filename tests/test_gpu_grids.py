@@ -141,3 +141,31 @@ def test_expansion_edges(npw, nbasis, nblock):
     n = davidson_expand(V, nbasis, dev(phi), [dev(H)], dev(kg2), eig)
     assert n == len(rows)
     assert np.abs(V[:n].cpu().numpy() - np.array(rows)).max() < 1e-10
+
+
+@pytest.mark.parametrize("kind", ["general", "hermitian", "degenerate", "triangular"])
+@pytest.mark.parametrize("n", [1, 2, 3, 17, 32, 33, 64, 96, 112, 113])
+def test_subspace_eigen(n, kind):
+    """the one-CTA eigensolve (up to order 112) and the library's beyond: with unit
+    vectors as the basis the Ritz vectors are the eigenvectors themselves.
+    |H X - X D| is the backward error of a QR iteration, some n eps |H|."""
+    import torch
+    from tc_b200.context import subspace_ritz
+    rng = np.random.default_rng(n)
+    H = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    if kind == "hermitian":
+        H = H + H.conj().T
+    elif kind == "degenerate":
+        Q = np.linalg.qr(H)[0]
+        H = (Q * np.repeat(np.arange(n), 3)[:n]) @ Q.conj().T
+    elif kind == "triangular":
+        H = np.triu(H) + 3.0 * np.diag(np.arange(n))
+    V = np.eye(n, n + 5, dtype=complex)
+    HV = H.T @ V                                          # row j: H V_j
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    w, e, Vo, _ = subspace_ritz(dev(V), [dev(HV), None, None], n)
+    X = Vo.cpu().numpy()[:, :n].T
+    nrm = np.linalg.norm(H)
+    assert np.all(np.diff(w.real) >= 0)
+    assert np.abs(np.linalg.norm(X, axis=0) - 1.0).max() <= 1e-12
+    assert np.abs(H @ X - X * w).max() <= 50 * n * 2.2e-16 * nrm
