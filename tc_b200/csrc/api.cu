@@ -260,7 +260,7 @@ extern "C" int tcg_ctx_create(const tcg_system_desc *sys, int32_t precision, tcg
     if (const char *e = getenv("TCG_MIN_TARGETS")) c->min_targets = atoi(e);
     if (const char *e = getenv("TCG_Z_KERNELS"))    // "line" / "split": override the per-term choice
         c->z_kernels = !strcmp(e, "line") ? 1 : (!strcmp(e, "split") ? 2 : (!strcmp(e, "t6") ? 3 : (!strcmp(e, "t6r") ? 4 : 0)));
-    h.red_n = choose_reduced(h);
+    h.red_n = choose_reduced(h, c->prec == TCG_PREC_FP64);
     if ((rc = make_grid(c, h.un, c->ugd, c->utw64, c->utw32)) ||
         (rc = up(c->recip, h.recip, sizeof h.recip, c->stream)) ||
         (rc = up(c->phase, sys->phase, ngi * sizeof(double2), c->stream)) ||

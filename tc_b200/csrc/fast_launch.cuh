@@ -42,7 +42,7 @@ int run_chunk_fast(tcg_ctx *c, const Op &op, int items, int nt, bool do_xyf, boo
         const int np = bl ? op.m.pmax : N * N;
         return launch_tagged(c, tagname(Op::NAME, "z"), (double)items * (nf_eff + (Op::ZINV ? nb_eff : 0)) * gb,
                              sl::k_z<T, Op, SH>, dim3((np + 31) / 32, items), dim3(SH::ZTHREADS),
-                             sl::smem_z<V, SH>(Op::NF), op);
+                             sl::smem_z<T, Op, SH>(), op);
     };
     if (slx && slz) {
         TRY(z_split());

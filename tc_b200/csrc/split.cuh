@@ -562,13 +562,17 @@ template <typename V, class S, class Op> __host__ inline size_t smem_xyi(bool pr
 // zsrc(o) < ZK, so only ZK transformed inputs and one sum stay in registers
 // (with all inputs of 2x3A kept, 80 registers and 4 CTAs left the pass waiting
 // for its loads: issue slots 43% busy, long_scoreboard the main stall).
+template <typename T, class Op> __host__ __device__ constexpr bool zk_shared()
+{
+    return sizeof(T) == 8 && Op::ZINV && Op::NB > (Op::ZMO >= 0 ? 1 : 0);
+}
 template <typename T, class Op, class S>
 __global__ void __launch_bounds__(S::ZTHREADS, ctas_for(S::ZTHREADS, sizeof(T) == 4 ? (Op::NF > 4 ? 96 : 64) : 112)) k_z(Op op)
 {
     using V = typename C2<T>::t;
     constexpr int N = S::N, A = S::A, B = S::B, TC = 32, NF = Op::NF, ZK = Op::ZK;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    V *E = reinterpret_cast<V *>(smem_raw);   // [max(NF, 2)][N][TC] exchange buffers
+    V *E = reinterpret_cast<V *>(smem_raw);   // [N][TC] exchange buffers, one per input
     const int item = blockIdx.y;
     const int t = threadIdx.x / TC, cl = threadIdx.x % TC;
     // pruning: the CTA takes its 32 pencils from the pair's list (active
@@ -607,7 +611,11 @@ __global__ void __launch_bounds__(S::ZTHREADS, ctas_for(S::ZTHREADS, sizeof(T) =
         }
     }
     __syncthreads();
-    V K[ZK][A], mix[Op::ZMO >= 0 ? A : 1];
+    // FP64: the kept inputs go back to the entries of the exchange buffers that only this
+    // thread reads (in registers they spilled: 300 to 570 bytes per thread)
+    constexpr bool KS = zk_shared<T, Op>();
+    V K[KS ? 1 : ZK][KS ? 1 : A], v[A];
+    V *const own = E + t * A * TC + cl;
     if (t < B) {
 #pragma unroll
         for (int f = 0; f < NF; f++) {
@@ -615,14 +623,17 @@ __global__ void __launch_bounds__(S::ZTHREADS, ctas_for(S::ZTHREADS, sizeof(T) =
             step2<V, A, B, -1>(E + f * N * TC + cl, TC, t, X);   // z = t + B m
             if (f < ZK) {
 #pragma unroll
-                for (int m = 0; m < A; m++) K[f < ZK ? f : 0][m] = X[m];
+                for (int m = 0; m < A; m++) {
+                    if constexpr (KS) own[(f * N + m) * TC] = X[m];
+                    else K[f < ZK ? f : 0][m] = X[m];
+                }
             }
             if constexpr (Op::ZMO >= 0) {
                 if (f >= Op::ZM0) {
 #pragma unroll
                     for (int m = 0; m < A; m++) {
                         const V w = cscale(X[m], act ? op.zmixc(zc, f, t + B * m) : (T)0);
-                        mix[m] = f == Op::ZM0 ? w : cadd(mix[m], w);
+                        v[m] = f == Op::ZM0 ? w : cadd(v[m], w);
                     }
                 }
             }
@@ -631,25 +642,21 @@ __global__ void __launch_bounds__(S::ZTHREADS, ctas_for(S::ZTHREADS, sizeof(T) =
     Tw<V, A> twi;
     if (Op::ZINV) twi.load(op.g, t < B ? t : 0);
     __syncthreads();                          // the exchange buffers are free
+    if constexpr (KS) E += ZK * N * TC;
     int buf = 0;
 #pragma unroll 1
     for (int i = 0; i < Op::NB; i++) {
-        // the mixed output first: its registers are then free
+        // the mixed output first: v holds it
         const int o = Op::ZMO > 0 ? (i == 0 ? Op::ZMO : (i <= Op::ZMO ? i - 1 : i)) : i;
         const bool blo = prune && ((Op::BLO >> o) & 1);
         if (blo && allin) continue;       // uniform over the CTA
-        V v[A];
-        if (t < B) {
-            if (o == Op::ZMO) {
+        if (t < B && (Op::ZMO < 0 || i > 0)) {
+            const int k = op.zsrc(o);
 #pragma unroll
-                for (int m = 0; m < A; m++) v[m] = mix[Op::ZMO >= 0 ? m : 0];
-            } else {
-                const int k = op.zsrc(o);
-#pragma unroll
-                for (int m = 0; m < A; m++) {
-                    const T w = act ? op.zoutc(zc, o, t + B * m) : (T)0;
-                    v[m] = cscale(ZK > 1 && k ? K[ZK - 1][m] : K[0][m], w);
-                }
+            for (int m = 0; m < A; m++) {
+                const T w = act ? op.zoutc(zc, o, t + B * m) : (T)0;
+                if constexpr (KS) v[m] = cscale(own[((ZK > 1 && k ? (ZK - 1) * N : 0) + m) * TC], w);
+                else v[m] = cscale(ZK > 1 && k ? K[ZK - 1][m] : K[0][m], w);
             }
         }
         if (Op::ZINV) {
@@ -674,9 +681,10 @@ __global__ void __launch_bounds__(S::ZTHREADS, ctas_for(S::ZTHREADS, sizeof(T) =
         }
     }
 }
-template <typename V, class S> __host__ inline size_t smem_z(int nf)
+template <typename T, class Op, class S> __host__ inline size_t smem_z()
 {
-    return sizeof(V) * (size_t)(nf < 2 ? 2 : nf) * S::N * 32;
+    constexpr int out = zk_shared<T, Op>() ? Op::ZK + 2 : 2, nb = Op::NF > out ? Op::NF : out;
+    return sizeof(typename C2<T>::t) * (size_t)nb * S::N * 32;
 }
 
 } // namespace sl

@@ -124,9 +124,14 @@ static double miller_extent(const Host &h, int i)
     return sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]) / (2.0 * PI_D);
 }
 
-// Edge of the smallest compiled cubic grid that gives the caller's results (0:
-// none smaller than the caller's).  Sets h.rmax.
-static int choose_reduced(Host &h)
+// Edge of the cheapest compiled cubic grid that gives the caller's results (0:
+// none smaller than the caller's).  Sets h.rmax.  That is the smallest, except
+// where its lines split badly (15 = 5 x 3, 27 = 9 x 3, 45 = 9 x 5: most threads of
+// the shorter step wait) and the next size fits as well: a TC apply of 8 k-points
+// takes 1.02 ms on 15^3 and 0.93 on 16^3 (FP64 1.53 and 1.51), in FP64 12.7 ms on
+// 27^3 and 10.4 on 30^3, 1.58 on 45^3 and 1.52 on 48^3; in FP32 27 and 45 stay
+// ahead (5.08 and 5.37 ms, 0.93 and 0.98).
+static int choose_reduced(Host &h, bool fp64)
 {
     h.rmax = 0;
     int mmax[3] = {0, 0, 0};
@@ -164,10 +169,16 @@ static int choose_reduced(Host &h)
         for (int d = 0; d < 3; d++)
             if (!integral(h.un[d], d)) return 0;
     int best = 0;
+    bool done = false;                         // the size after the smallest has been looked at
     auto consider = [&](int n) {
         const int n3[3] = {n, n, n};
         const double pts = (double)n * n * n;
-        if (best || pts > (user_fast ? 0.9 : 1.0) * h.uN) return;
+        if (best) {
+            if (done) return;
+            done = true;
+            if (!(best == 15 || (fp64 && (best == 27 || best == 45)))) return;
+        }
+        if (pts > (user_fast ? 0.9 : 1.0) * h.uN) return;
         if (!(shortest_period(h, n3) > need)) return;
         for (int d = 0; d < 3; d++) {
             if (2 * mmax[d] >= n) return;      // the plane waves keep their signed indices

@@ -84,6 +84,16 @@ def test_work_grid_time_reversal(method, prec):
     check(s, abi.TERMS_HF if method == "HF" else abi.TERMS_TC, prec)
 
 
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,user", [(15, 20), (15, 15), (27, 32), (45, 48)])
+def test_work_grid_of_uneven_lines(n, user, prec):
+    """n^3 is the smallest work grid; the next size is taken where n's lines split
+    badly (15, in FP64 27 and 45) unless the caller's grid is smaller than that"""
+    ecut = 0.5 * (0.985 * n * np.sqrt(3.0) * 2.0 * np.pi / 10.26 / 6.0) ** 2
+    s = synth.small("TC", nr=(user, user, user), nk=1, ecut=ecut, nbands=2, nocc=1, seed=n)
+    check(s, abi.TERMS_TC, prec)
+
+
 def test_density_beyond_the_pair_sphere():
     """a density with a component outside the pair densities' sphere needs the
     caller's grid; the next state may go back to the smaller one"""
