@@ -150,7 +150,6 @@ static int grad_tables_tc2x(tcg_ctx *c, int s, double2 *dv2, double2 *du)
                                                  (unsigned)std::min<size_t>(65535, nb * 8 - q0)),
                        dim3(256), 0, (int)N, (int)std::min<size_t>(65535, nb * 8 - q0), (const V *const *)(dA + q0),
                        (const V *const *)(dB + q0), G8 + q0 * N));
-        TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->items is reused by the FFT helper
         std::vector<void *> grids(nb * 8);
         for (size_t q = 0; q < nb * 8; q++) grids[q] = G8 + q * N;
         TRY((fft3_list<double, -1>(c, grids)));
@@ -159,7 +158,6 @@ static int grad_tables_tc2x(tcg_ctx *c, int s, double2 *dv2, double2 *du)
         memcpy(rc.R, h.recip, sizeof rc.R);
         TRY(launch(c, k_grad_tc2x, dim3(pblocks), dim3(256), 0, c->gd, rc, (int)nb, (const GradPair *)c->items.p,
                    (const double2 *)G8, dv2, du));
-        TCG_CUDA(cudaStreamSynchronize(c->stream));
     }
     return TCG_OK;
 }

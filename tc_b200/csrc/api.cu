@@ -293,6 +293,20 @@ extern "C" int tcg_ctx_destroy(tcg_ctx *c)
     return TCG_OK;
 }
 
+// No infinity or NaN in x (x * 0 is 0 for every finite x).  Eight independent sums,
+// which the compiler turns into vector code: one value per 0.3 ns; a test and a
+// branch per value took 1 to 1.5 ns, 0.3 of the 7.1 ms of a TC state and apply on 32^3.
+static bool all_finite(const double *x, size_t n)
+{
+    double s[8] = {};
+    size_t i = 0;
+    for (; i + 8 <= n; i += 8)
+        for (int j = 0; j < 8; j++) s[j] += x[i + j] * 0.0;
+    for (; i < n; i++) s[0] += x[i] * 0.0;
+    for (int j = 1; j < 8; j++) s[0] += s[j];
+    return s[0] == 0.0;
+}
+
 // upload the orbital / filling part of a state (no R-space work)
 static int tcg_set_state_orbitals_only(tcg_ctx *c, const tcg_state_desc *st)
 {
@@ -323,8 +337,7 @@ static int tcg_set_state_orbitals_only(tcg_ctx *c, const tcg_state_desc *st)
             off += (size_t)h.nbands[s] * h.npw[k];
         }
     const size_t norb = off;
-    for (size_t i = 0; i < 2 * norb; i++)
-        if (!std::isfinite(st->phik[i])) return fail(TCG_ERR_NUMERIC, "non-finite orbital coefficient");
+    if (!all_finite(st->phik, 2 * norb)) return fail(TCG_ERR_NUMERIC, "non-finite orbital coefficient");
     h.occ_off.resize((size_t)h.nspin * h.nk_all);
     size_t g = 0;
     std::vector<double> occfill;
@@ -355,8 +368,7 @@ extern "C" int tcg_set_state(tcg_ctx *c, const tcg_state_desc *st)
     TRY(tcg_set_state_orbitals_only(c, st));
     Host &h = c->h;
     int rc;
-    for (size_t i = 0; i < 4 * (size_t)h.uN; i++)
-        if (!std::isfinite(st->density[i])) return fail(TCG_ERR_NUMERIC, "non-finite density");
+    if (!all_finite(st->density, 4 * (size_t)h.uN)) return fail(TCG_ERR_NUMERIC, "non-finite density");
     if ((rc = up(c->udens, st->density, 2 * (size_t)h.uN * sizeof(double2), c->stream))) return rc;
     TRY(place_state(c));
     rc = c->prec == TCG_PREC_FP64 ? build_occupied<double>(c) : build_occupied<float>(c);
@@ -432,8 +444,7 @@ extern "C" int tcg_apply(tcg_ctx *c, uint32_t mask, const int32_t *nb, const dou
     if (need2 && !h2) return fail(TCG_ERR_ARG, "h2 is NULL");
     if (need3 && !h3) return fail(TCG_ERR_ARG, "h3 is NULL");
     const size_t n = psi_count(c, nb);
-    for (size_t i = 0; i < 2 * n; i++)
-        if (!std::isfinite(psi[i])) return fail(TCG_ERR_NUMERIC, "non-finite value in psi");
+    if (!all_finite(psi, 2 * n)) return fail(TCG_ERR_NUMERIC, "non-finite value in psi");
     const size_t bytes = n * sizeof(double2);
     TRY(c->psi.ensure(bytes));
     TRY(c->h2.ensure(need2 ? bytes : 16));
@@ -490,8 +501,7 @@ extern "C" int tcg_apply_h1(tcg_ctx *c, uint32_t mask, const int32_t *nb, const 
     for (int i = 0; i < c->h.nspin * c->h.nk; i++)
         if (nb[i] < 0) return fail(TCG_ERR_ARG, "negative band count");
     const size_t n = psi_count(c, nb);
-    for (size_t i = 0; i < 2 * n; i++)
-        if (!std::isfinite(psi[i])) return fail(TCG_ERR_NUMERIC, "non-finite value in psi");
+    if (!all_finite(psi, 2 * n)) return fail(TCG_ERR_NUMERIC, "non-finite value in psi");
     const size_t bytes = n * sizeof(double2);
     TRY(c->psi.ensure(std::max<size_t>(16, bytes)));
     TRY(c->h1buf.ensure(std::max<size_t>(16, bytes)));

@@ -230,7 +230,6 @@ static int apply_h1_impl(tcg_ctx *c, uint32_t mask, const int32_t *nb, const dou
         for (size_t b0 = 0; b0 < nt; b0 += 65535)
             TRY(launch(c, k_kinetic, dim3(4, (unsigned)std::min<size_t>(65535, nt - b0)), dim3(256), 0,
                        (const KinItem *)(c->items.as<KinItem>() + b0), c->gd, rc));
-        TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->items is reused below
     }
     if ((mask & TCG_TERM_PSEUDO) && h.nl_ncomp > 0) {
         std::vector<NLItem> it(nt);
@@ -247,7 +246,6 @@ static int apply_h1_impl(tcg_ctx *c, uint32_t mask, const int32_t *nb, const dou
         const double *dval = reinterpret_cast<const double *>(c->nlD.as<char>() + h.nl_dval_off);
         TRY(launch(c, k_nonlocal, dim3((unsigned)nt), dim3(256), (2 * nc + 256) * sizeof(double2),
                    (const NLItem *)c->items.p, nc, dptr, dptr + nc + 1, dval));
-        TCG_CUDA(cudaStreamSynchronize(c->stream));
     }
     if ((mask & TCG_TERM_PSEUDO) && h.have_vloc) {
         TRY(c->Rpsi.ensure(nt * N * sizeof(V)));

@@ -610,7 +610,6 @@ static int plan_chunks(tcg_ctx *c, DBuf &meta, int ntg, const std::vector<int> &
         p.sb = reinterpret_cast<const int *>(base + (size_t)p.sb);
         p.pent = reinterpret_cast<const int *>(base + (size_t)p.pent);
     }
-    TCG_CUDA(cudaStreamSynchronize(c->stream));
     return TCG_OK;
 }
 
@@ -761,7 +760,6 @@ static int finalize_acc(tcg_ctx *c, const Targets &T, double2 *acc, double2 *hou
         TRY((grids_xy<double, -1>(c, g, gr, nb)));
         TRY(gather_z(c, g, d_gi + b0, nb));
     }
-    TCG_CUDA(cudaStreamSynchronize(c->stream));
     return TCG_OK;
 }
 
@@ -835,7 +833,6 @@ static int div_2x(tcg_ctx *c, const Targets &T, const ApplyArgs &A, double2 *hou
     TRY(c->items.ensure(nt * sizeof(DivItem)));
     TCG_CUDA(cudaMemcpyAsync(c->items.p, di.data(), nt * sizeof(DivItem), cudaMemcpyHostToDevice, c->stream));
     TRY(launch(c, k_div_2x, dim3((unsigned)nt), dim3(256), 0, (const DivItem *)c->items.p));
-    TCG_CUDA(cudaStreamSynchronize(c->stream));
     return TCG_OK;
 }
 
@@ -934,7 +931,6 @@ static int hf_cube_table(tcg_ctx *c, bool &ok)
     else
         TRY(launch(c, k_tables, dim3(148 * 8), dim3(256), 0, c->gd, rc, make_jastrow(h), (int)TAB_HF, 1, hg, 0, (int)npair,
                    (const double *)c->meta.p, invN, c->hftab.as<double>()));
-    TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->meta is reused
     c->hftab_ok = true;
     return TCG_OK;
 }
@@ -974,7 +970,6 @@ static int run_hf2x_cube(tcg_ctx *c, const Targets &Tg, double2 *acc)
         TRY(hf_cube<T>(c, a));
         TRY(launch(c, cube_sum<V>, dim3((unsigned)std::min<size_t>(148 * 8, (TR.n * N + 255) / 256)), dim3(256), 0,
                    (size_t)TR.n * N, a.splits, (const V *)a.part, acc + (size_t)TR.t0 * N));
-        TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->meta is reused
     }
     return TCG_OK;
 }
@@ -1240,7 +1235,6 @@ static int run_tc3a3b3b4b6(tcg_ctx *c, const Targets &Tg, const ApplyArgs &A, do
                 TRY(launch(c, k_div3b6_add<T>, dim3((unsigned)std::min<size_t>(32, (N + 255) / 256), nb), dim3(256), 0, it,
                            (int)N, maxocc, (const double2 *)fd));
             }
-            TCG_CUDA(cudaStreamSynchronize(c->stream));
         }
         // stage C: 3b4 (:651-770); after the fused first stage also 3b3 and,
         // with band_fused, tc3a2a4b2b5's 3b5 (OpTC3X)
@@ -1574,7 +1568,6 @@ static int qp_finish(tcg_ctx *c)
             TRY(launch(c, k_rot_store<T>, dim3(gx, (unsigned)n), dim3(256), 0, (int)N, dit, (const double2 *)R,
                        c->Qt.as<V>(), c->Bt.as<V>()));
         }
-        TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->items is reused below
         // 3b2 local potential (:922-958): V3b2[s](r) += IFFT[ sum_d G_d u' FFT(qsum3b2_d) ]
         {
             std::vector<void *> grids;

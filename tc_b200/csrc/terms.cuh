@@ -144,7 +144,6 @@ static int sphere_to_r(tcg_ctx *c, const std::vector<SphereItem> &items)
         gr.dev = d_outs + b0;
         TRY((grids_xy<T, +1>(c, g, gr, nb)));
     }
-    TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->items is reused by the next caller
     return TCG_OK;
 }
 
@@ -172,7 +171,6 @@ static int fft3_list(tcg_ctx *c, const std::vector<void *> &grids, const GridDes
         TRY((grids_xy<T, DIR>(c, g, gr, nb)));
         TRY((grids_z<T, DIR>(c, g, gr, nb, scale)));
     }
-    TCG_CUDA(cudaStreamSynchronize(c->stream));   // c->items is reused by the next caller
     return TCG_OK;
 }
 
