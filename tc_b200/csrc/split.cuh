@@ -24,6 +24,7 @@
 // form, which staged planes in shared memory, made 8 to 10 with 3 times the
 // barriers).
 #pragma once
+#include <type_traits>
 #include "fft.cuh"
 #include "fast.cuh"
 
@@ -151,12 +152,22 @@ template <typename V, int Q> struct Tw {
 #pragma unroll
         for (int k = 1; k < Q; k++) w[k] = __ldg(&src[t * k]);
     }
+    __device__ __forceinline__ V operator()(int k) const { return w[k]; }
 };
-template <typename V, int Q, int DIR> __device__ __forceinline__ void step1(V (&u)[Q], const Tw<V, Q> &tw)
+// the same read from a table in shared memory when needed
+template <typename V> struct TwS {
+    const V *tab;
+    int t;
+    __device__ __forceinline__ V operator()(int k) const { return tab[t * k]; }
+};
+template <typename V, int Q, int DIR, class TW> __device__ __forceinline__ void step1(V (&u)[Q], const TW &tw)
 {
     dft<V, Q, DIR>(u);
 #pragma unroll
-    for (int k = 1; k < Q; k++) u[k] = DIR < 0 ? cmul(u[k], tw.w[k]) : cmulc(tw.w[k], u[k]);
+    for (int k = 1; k < Q; k++) {
+        const V w = tw(k);
+        u[k] = DIR < 0 ? cmul(u[k], w) : cmulc(w, u[k]);
+    }
 }
 // exchange: u[k1] of thread t goes to buf[(k1 P + t) stride], thread t < Q reads its P values
 template <typename V, int P, int Q> __device__ __forceinline__ void put(V *buf, int stride, int t, const V (&u)[Q])
@@ -174,8 +185,8 @@ template <typename V, int P, int Q, int DIR> __device__ __forceinline__ void ste
 // Forward XY transform of one plane.  In: u[m] = f(x = l, y = t + A m), t < A.
 // Out: v[m] = F(kx = t + B m, ky = l), t < B.  b0, b1: the two buffers; b0 holds
 // the last exchange, so the caller swaps them for its next transform.
-template <typename V, class S>
-__device__ __forceinline__ void plane_fwd(V *b0, V *b1, int t, int l, V (&u)[S::B], const Tw<V, S::B> &tw, V (&v)[S::A])
+template <typename V, class S, class TW>
+__device__ __forceinline__ void plane_fwd(V *b0, V *b1, int t, int l, V (&u)[S::B], const TW &tw, V (&v)[S::A])
 {
     constexpr int A = S::A, B = S::B, PAD = S::PAD;
     const bool on = S::LP == S::N || l < S::N;
@@ -201,8 +212,8 @@ __device__ __forceinline__ void plane_fwd(V *b0, V *b1, int t, int l, V (&u)[S::
 }
 // Inverse XY transform.  In: u[m] = F(kx = t + B m, ky = l), t < B.
 // Out: v[m] = f(x = l, y = t + A m), t < A.
-template <typename V, class S>
-__device__ __forceinline__ void plane_inv(V *b0, V *b1, int t, int l, V (&u)[S::A], const Tw<V, S::A> &tw, V (&v)[S::B])
+template <typename V, class S, class TW>
+__device__ __forceinline__ void plane_inv(V *b0, V *b1, int t, int l, V (&u)[S::A], const TW &tw, V (&v)[S::B])
 {
     constexpr int A = S::A, B = S::B, PAD = S::PAD;
     const bool on = S::LP == S::N || l < S::N;
@@ -355,9 +366,9 @@ template <typename V, class S, class Op> __host__ inline size_t smem_xyf()
 // 27-k case).  They and the next step's G plane are therefore copied
 // asynchronously into slots of shared memory that belong to the reading thread
 // alone, so a thread waits for its own copies and the passes' barriers stay the
-// only ones (20.9 ms, with registers for three sums and no spills; 24.2 with one
-// CTA more and spills).  FP64 planes beyond 32^2 leave no room for the slots:
-// there operands are loaded in place and the sums live in shared memory.
+// only ones (20.3 ms with registers for three sums; 23.0 with one CTA more and
+// spills).  FP64 planes beyond 32^2 leave no room for the slots: there operands
+// are loaded in place and the sums live in shared memory.
 // GS > 1: the first GS - 1 outputs of a group wait in registers.
 constexpr int MAXSRC = 64;           // sources per chunk (plan_chunks): rows of pencil masks in shared memory
 
@@ -368,9 +379,22 @@ template <class Op, class S, typename V> struct Lay {
     static constexpr size_t ACC = STG ? 0 : sizeof(V) * (size_t)Op::NACC * B * S::THREADS;
     static constexpr size_t OPS = STG ? sizeof(V) * (size_t)Op::NOPS * B * S::THREADS : 0;
     static constexpr size_t GPL = STG ? sizeof(V) * (size_t)S::N * S::N : 0;
-    static constexpr size_t TOTAL = PLANES + ACC + OPS + GPL;
     // registers: in FP32 96 (3 CTAs of 6 warps) with three sums per point, 72 with one
     static constexpr int REGS = sizeof(V) == 8 ? 66 + 2 * Op::NACC * B : (STG ? 108 + 4 * Op::NACC * B : 112);
+    // The twiddles come from a table in shared memory where their registers would be spilled
+    // (by more than the compiler saves elsewhere): 2x3A on 30^3 4.34 -> 3.33 ms in FP64 (312
+    // bytes of spills), 21.9 -> 20.3 ms in FP32 (60 bytes); where they fit the reads cost 1 to
+    // 3% (16^3 FP64 1.86 -> 1.90, one sum on 30^3 0.383 -> 0.396).
+    // CAP: what launch_bounds leaves a thread (16384 registers per quarter of an SM)
+    static constexpr int WARPS = (S::THREADS + 31) / 32 * ctas_for(S::THREADS, REGS);
+    static constexpr int CAP = 512 / ((WARPS + 3) / 4) / 8 * 8;
+    static constexpr bool TWS = STG && REGS + (int)sizeof(V) / 4 * (S::A + B - 2) > CAP + 16;
+    static constexpr size_t TWT = TWS ? sizeof(V) * (size_t)S::N : 0;
+    // FP32: the density of re-forwarded planes at the thread's points, read once per CTA (from
+    // global memory it cost a wait per source: 48^3 13.4 -> 13.1 ms)
+    static constexpr bool RW = STG && sizeof(V) == 8 && Op::REFWD && Op::NRW == 1;
+    static constexpr size_t DEN = RW ? sizeof(V) * (size_t)B * S::THREADS : 0;
+    static constexpr size_t TOTAL = PLANES + ACC + OPS + GPL + DEN + TWT;
 };
 template <class Op, class S, typename V> struct Acc {
     static constexpr bool SM = !Lay<Op, S, V>::STG;
@@ -416,10 +440,24 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
 #pragma unroll
         for (int m = 0; m < B; m++) acc.at(a, m) = czero<V>();
     V keep[Op::GS][B];
-    Tw<V, A> twi;
-    twi.load(op.g, t < B ? t : 0);
-    Tw<V, B> twf;
-    if (Op::REFWD) twf.load(op.g, t);
+    V *den = reinterpret_cast<V *>(smem_raw + L::PLANES + L::ACC + L::OPS + L::GPL) + threadIdx.x;
+    if constexpr (L::RW) {
+        if (on)
+#pragma unroll
+            for (int m = 0; m < B; m++) den[m * S::THREADS] = __ldg(op.refwd_dens(0) + p0 + (size_t)A * m * N);
+    }
+    std::conditional_t<L::TWS, TwS<V>, Tw<V, A>> twi;
+    std::conditional_t<L::TWS, TwS<V>, Tw<V, B>> twf;
+    if constexpr (L::TWS) {
+        V *tab = reinterpret_cast<V *>(smem_raw + L::TOTAL - L::TWT);
+        for (int i = threadIdx.x; i < N; i += S::THREADS) tab[i] = twsrc<V>(op.g)[i];
+        twi = {tab, t < B ? t : 0};
+        twf = {tab, t};
+        __syncthreads();
+    } else {
+        twi.load(op.g, t < B ? t : 0);
+        if (Op::REFWD) twf.load(op.g, t);
+    }
     auto mask = [&](int si, int b) { return prune && ((Op::BLO >> b) & 1) ? sbits[si * N + l] : ~0ull; };
     V nx[L::STG ? 1 : A];
     auto fetch = [&](int si, int b) {
@@ -518,7 +556,10 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
             V w[A];
             if (on) {
 #pragma unroll
-                for (int m = 0; m < B; m++) v[m] = op.refwd_load(tj, item, bg, p0 + (size_t)A * m * N, v[m]);
+                for (int m = 0; m < B; m++) {
+                    if constexpr (L::RW) v[m] = op.refwd_mul(item, v[m], den[m * S::THREADS]);
+                    else v[m] = op.refwd_load(tj, item, bg, p0 + (size_t)A * m * N, v[m]);
+                }
             }
             plane_fwd<V, S>(b0, b1, t, l, v, twf, w);
             {

@@ -275,6 +275,10 @@ struct OpBase {
     __device__ int nsrc(int) const { return ns; }
     __device__ int item_of(int tj, int si) const { return tj * ns + si; }
     __device__ bool refwd_want(int) const { return false; }
+    // v times the density of output b's branch (densities refwd_dens, NRW of them)
+    static constexpr int NRW = 0;
+    __device__ const V *refwd_dens(int) const { return nullptr; }
+    __device__ V refwd_mul(int, V v, V) const { return v; }
     __device__ V refwd_load(int, int, int, size_t, V v) const { return v; }
     __device__ V *refwd_grid(int, int) const { return nullptr; }
     __device__ V xyf_load(int, int, int, int, int, size_t) const { return czero<V>(); }
@@ -722,10 +726,12 @@ struct OpTC3A : OpBase<T> {
         }
     }
     __device__ bool refwd_want(int b) const { return b > 0; }
-    __device__ V refwd_load(int, int, int b, size_t p, V v) const
+    static constexpr int NRW = NX;
+    __device__ const V *refwd_dens(int xs) const { return densT + (size_t)xs * this->g.N; }
+    __device__ V refwd_mul(int, V v, V n) const { return cmul(v, n); }   // orbital * n_s2 (:332)
+    __device__ V refwd_load(int, int item, int b, size_t p, V v) const
     {
-        const int xs = EQ ? 0 : (b - 1) / 3;
-        return cmul(v, __ldg(&densT[(size_t)xs * this->g.N + p]));   // orbital * n_s2 (:332)
+        return refwd_mul(item, v, __ldg(refwd_dens(EQ ? 0 : (b - 1) / 3) + p));
     }
     // one sum per output: b3 f v phi_q (b = 0), v phi_q of the branch x = s
     __device__ const V *xyi_operand(int, int b, int si) const
@@ -1154,11 +1160,13 @@ struct OpTC2X3 : OpTC2X<T> {
     double fa4;
     int band;
     __device__ bool refwd_want(int b) const { return b > 0; }
-    __device__ V refwd_load(int, int item, int, size_t p, V v) const
+    static constexpr int NRW = 1;
+    __device__ const V *refwd_dens(int) const { return densT; }
+    __device__ V refwd_mul(int item, V v, V n) const
     {
-        const int si = item % this->ns;
-        return cscale(cmul(v, __ldg(&densT[p])), (decltype(v.x))this->fill[si]);   // f orbital * n (:332)
+        return cscale(cmul(v, n), (decltype(v.x))this->fill[item % this->ns]);   // f orbital * n (:332)
     }
+    __device__ V refwd_load(int, int item, int, size_t p, V v) const { return refwd_mul(item, v, __ldg(densT + p)); }
     __device__ V *refwd_grid(int item, int b) const { return tmp2 + ((size_t)item * 3 + (b - 1)) * this->g.N; }
     // qsum_d += f w_d phi_q (:305-328); tc2x's own sum goes through the registers
     __device__ void xyi_extra(int tj, int item, int b, size_t p, const V *v) const
