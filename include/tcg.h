@@ -346,17 +346,19 @@ int tcg_set_tuning(tcg_ctx *ctx, int64_t tmp_budget_bytes);
 /* Kernel forms of the pass pipelines (the choices an autotuner explores; no
  * reference counterpart).  xy: 0 = each term's default (split lines on the
  * grids that have them), 1 = one thread per line, 2 = a lane pair per line,
- * 3 = split lines (six threads per line at 36^3, four at 48^3); z: 0 =
- * default, 1 = one thread per z-line, 2 = a lane pair, 3 = split lines with
- * the inputs in shared memory, 4 = split lines with the inputs in registers
- * (3 and 4 need a 36^3 or 48^3 grid).  xy 1 or 2 and z 1 or 2 turn the
- * pruning of band-limited grids off (only the split-line kernels honour it).  Flags, each
- * 0 or 1: prefetch (the inverse XY pass copies the next plane set while it
- * transforms the current one), prune (band-limited grids on the pencils
- * their support meets), fuse (tc2x, tc3a3b3b4b6 and tc3a2a4b2b5's band part
- * share their transforms), qp_sacc / sacc (shared-memory accumulation in the
- * occupied-pair / first-stage inverse XY passes).  min_targets: targets per
- * chunk (0 = default).  tcg_get_forms reads the current choice. */
+ * 3 = split lines; z: 0 = default, 1 = one thread per z-line, 2 = a lane
+ * pair, 3 and 4 = split lines (one kernel since their inputs need no copy in
+ * shared memory).  xy = 3 and z = 3, 4 are refused except on 36^3 and 48^3
+ * (elsewhere split lines are the default anyway); 1 and 2 act on cubic grids of
+ * side 12, 16, 24, 32, 36, 40, 48, turn the pruning of band-limited grids off
+ * (only the split lines honour it) and keep the library on the caller's grid.
+ * Flags, each 0 or 1: prefetch (the one-thread and lane-pair inverse XY passes copy
+ * the next plane set while they transform the current one; split lines always
+ * do), prune (band-limited grids on the pencils their support meets), fuse
+ * (tc2x, tc3a3b3b4b6 and tc3a2a4b2b5's band part share their transforms),
+ * qp_sacc / sacc (kept for callers that set them: the inverse XY passes always
+ * sum a chunk's sources on chip).  min_targets: targets per chunk (0 =
+ * default).  tcg_get_forms reads the current choice. */
 typedef struct tcg_forms {
     int32_t xy, z, prefetch, prune, fuse, qp_sacc, sacc, min_targets;
 } tcg_forms;

@@ -1,9 +1,10 @@
 """Build step of the CUDA library libtcg_b200.so (in-tree, sm_100a).
 
-api.cu (C-ABI, orchestration, generic kernels), cube.cu (on-chip hf2x), subspace.cu (the dense
-Davidson subspace step on cuBLAS / cuSOLVER) and one instance of fast_inst.cu
-per compiled cubic grid size and precision are compiled in parallel into tc_b200/_build/
-and linked into tc_b200/libtcg_b200.so.
+api.cu (C-ABI, orchestration, generic kernels), cube.cu (on-chip hf2x), subspace.cu
+(the dense Davidson subspace step), any_inst.cu per precision (run-time shapes) and
+one instance of fast_inst.cu per compiled cubic grid size and precision are compiled in
+parallel into tc_b200/_build/ and linked into tc_b200/libtcg_b200.so, the device code
+compressed for size (173 MB otherwise).
 """
 import concurrent.futures as cf
 import os

@@ -6,6 +6,8 @@
 // is uniform over the grid, its operands stay in registers (9 of them, unused
 // ones predicated off).  The generic passes (passes.cuh) run one shared-memory
 // sweep and one barrier per radix and remain for lengths that do not factor so.
+// A TC state and apply on 20 x 18 x 21 with two spins in FP64: 19.3 ms with them,
+// 14.3 with these.
 // MT: most threads of an XY CTA (256: up to 255 registers, FP64 without spills;
 // sl::MAXTHR for longer lines).
 #pragma once

@@ -2,6 +2,9 @@
 // on both sides) on the compiled cubic sizes, in split lines (split.cuh): orbitals
 // onto the grid, accumulators back onto the sphere, the per-state fields.  The
 // generic forms (passes.cuh) make one shared-memory sweep and one barrier per radix.
+// The passes move each grid four times; where there are enough grids to fill the
+// device memory traffic bounds them (gradient tables on 40^3: 2.74 -> 1.52 ms), for a
+// few grids the launch and one line's latency do (5 us a pass).
 #pragma once
 #include "terms.cuh"
 #include "split.cuh"
