@@ -64,7 +64,8 @@ extern "C" {
 #define TCG_METHOD_BITC  2
 
 #define TCG_PREC_FP64    0   /* complex128 everywhere                          */
-#define TCG_PREC_MIXED   1   /* complex64 FFTs / pair products, FP64 accumulation */
+#define TCG_PREC_MIXED   1   /* complex64 FFTs / pair products, FP64 accumulation
+                                (FP32 sums over at most 8 sources)               */
 
 /* ---- term mask ----------------------------------------------------------
  * Bit i selects one of the reference routines.  hf2x and tc2x add to H2,

@@ -249,6 +249,15 @@ __global__ void __launch_bounds__(MT) k_xyi(Op op, sl::AnyShape S, int nt)
                         });
                     }
             }
+            if (mine && (si + 1 == ns || sl::flush_due<V>(si)))
+                for (int a = 0; a < NA; a++)
+#pragma unroll
+                    for (int m = 0; m < MX; m++)
+                        if (m < g.b1) {
+                            V *s = acc + (a * g.b1 + m) * nthr;
+                            op.xyi_put(tj, bg, a, p0 + m * ystep, *s);
+                            *s = czero<V>();
+                        }
             if (Op::REFWD && op.refwd_want(bg)) {
                 if (mine) {
 #pragma unroll
@@ -268,15 +277,6 @@ __global__ void __launch_bounds__(MT) k_xyi(Op op, sl::AnyShape S, int nt)
                 }
             }
         }
-        if (mine)
-            for (int a = 0; a < NA; a++)
-#pragma unroll
-                for (int m = 0; m < MX; m++)
-                    if (m < g.b1) {
-                        V *s = acc + (a * g.b1 + m) * nthr;
-                        op.xyi_put(tj, bg, a, p0 + m * ystep, *s);
-                        *s = czero<V>();
-                    }
     }
 }
 

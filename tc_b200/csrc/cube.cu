@@ -6,7 +6,6 @@ namespace {
 template <typename T, int N> int call_n(tcg_ctx *c, const CubeCall<T> &a)
 {
     using V = typename C2<T>::t;
-    constexpr int PX = N + (N % 2 == 0 ? 1 : 0);
     cube::TwN<V, N> tw;
     for (int i = 0; i < N; i++) {
         if constexpr (sizeof(T) == 4) tw.w[i] = c->htw32[i];
@@ -14,7 +13,7 @@ template <typename T, int N> int call_n(tcg_ctx *c, const CubeCall<T> &a)
     }
     const double gb = (double)N * N * N * sizeof(V);
     return launch_tagged(c, tagname("hf2x", "cube"), 2.0 * a.nt * a.ns * gb, cube::k_hf<T, N>, dim3(a.nt, a.splits),
-                         dim3((N * N + 31) / 32 * 32), sizeof(V) * (size_t)N * N * PX, a, tw);
+                         dim3((N * N + 31) / 32 * 32), cube::smem_hf<T, N>(), a, tw);
 }
 } // namespace
 

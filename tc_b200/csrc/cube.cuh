@@ -55,6 +55,15 @@ template <typename V, int N, int A, int B, int DIR> __device__ __forceinline__ v
 // Sizes: the cube and, per thread, one z line and its sums in registers.
 // 20^3 complex64 keeps 400 threads of about 110 registers (one CTA per SM),
 // 18^3 complex128 324 of about 180; larger grids go through the passes.
+// shared memory: the grid, in FP32 also its FP64 sums
+template <typename T, int N> __host__ __device__ constexpr size_t cube_bytes()
+{
+    return (sizeof(typename C2<T>::t) * (size_t)N * N * (N + (N % 2 == 0 ? 1 : 0)) + 15) / 16 * 16;
+}
+template <typename T, int N> constexpr size_t smem_hf()
+{
+    return cube_bytes<T, N>() + (sizeof(T) == 4 ? sizeof(double2) * (size_t)N * N * N : 0);
+}
 template <typename T, int N> constexpr bool fits() { return sizeof(T) == 4 ? N <= 20 : N <= 18; }
 
 template <typename T, int N>
@@ -76,6 +85,13 @@ __global__ void __launch_bounds__((N * N + 31) / 32 * 32, sl::ctas_for(N *N, siz
     V sum[N];
 #pragma unroll
     for (int i = 0; i < N; i++) sum[i] = czero<V>();
+    // FP32: the sums of every FLUSH sources are added here, each thread's to its own entries
+    // (shared memory that one CTA per SM leaves free; in device memory it cost 12% of the pass)
+    double2 *S = reinterpret_cast<double2 *>(smem_raw + cube_bytes<T, N>()) + (on ? l : 0);
+    if (sizeof(T) == 4 && on) {
+#pragma unroll
+        for (int z = 0; z < N; z++) S[z * N2] = {0.0, 0.0};
+    }
     V *cz = C + q * PX + p, *cy = C + q * N * PX + p, *cx = C + (q * N + p) * PX;
     for (int si = s0; si < s1; si++) {
         const V *phi = a.Rocc + (size_t)si * N3 + (on ? l : 0);
@@ -119,18 +135,25 @@ __global__ void __launch_bounds__((N * N + 31) / 32 * 32, sl::ctas_for(N *N, siz
         __syncthreads();
         if (on) {
             // the next source's product overwrites only the column this thread reads here
-            const T f = (T)a.fill[si];
+            const double f = a.fill[si];
 #pragma unroll
             for (int z = 0; z < N; z++) v[z] = cz[z * N * PX];
             line<V, N, A, B, +1>(v, tw);
 #pragma unroll
-            for (int z = 0; z < N; z++) sum[z] = cadd(sum[z], cscale(cmul(v[z], __ldg(&phi[z * N2])), f));
+            for (int z = 0; z < N; z++) sum[z] = cadd(sum[z], cscale64(cmul(v[z], __ldg(&phi[z * N2])), f));
+            if (sl::flush_due<V>(si - s0)) {
+#pragma unroll
+                for (int z = 0; z < N; z++) {
+                    S[z * N2] = cadd(S[z * N2], to64(sum[z]));
+                    sum[z] = czero<V>();
+                }
+            }
         }
     }
     if (on) {
-        V *o = a.part + ((size_t)blockIdx.y * gridDim.x + tj) * N3 + l;
+        double2 *o = a.part + ((size_t)blockIdx.y * gridDim.x + tj) * N3 + l;
 #pragma unroll
-        for (int z = 0; z < N; z++) o[z * N2] = sum[z];
+        for (int z = 0; z < N; z++) o[z * N2] = sizeof(T) == 4 ? cadd(S[z * N2], to64(sum[z])) : to64(sum[z]);
     }
 }
 

@@ -48,6 +48,14 @@ template <typename V> __device__ __forceinline__ V cmul(V a, V b) { return {a.x 
 // conj(a) * b
 template <typename V> __device__ __forceinline__ V cmulc(V a, V b) { return {a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x}; }
 template <typename V, typename S> __device__ __forceinline__ V cscale(V a, S s) { return {a.x * s, a.y * s}; }
+// a f with f in FP64: the FP32 product takes both halves of f (a filling such as 0.3,
+// rounded once, would scale a whole term by up to 1 +- 6e-8)
+__device__ __forceinline__ double2 cscale64(double2 a, double f) { return {a.x * f, a.y * f}; }
+__device__ __forceinline__ float2 cscale64(float2 a, double f)
+{
+    const float h = (float)f, l = (float)(f - (double)h);
+    return {fmaf(a.x, h, a.x * l), fmaf(a.y, h, a.y * l)};
+}
 template <typename V> __device__ __forceinline__ V cconj(V a) { return {a.x, -a.y}; }
 // i * s * a  (s = +-1)
 template <typename V> __device__ __forceinline__ V cmuli(V a, int s) { return s > 0 ? V{-a.y, a.x} : V{a.y, -a.x}; }

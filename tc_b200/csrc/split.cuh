@@ -357,8 +357,8 @@ template <typename V, class S, class Op> __host__ inline size_t smem_xyf()
 // One (target, z) plane per CTA.  The outputs b (in groups of GS) run outside,
 // the chunk's sources inside, and a group's sums over the sources (at most
 // Op::NACC of them: xyi_add) stay with the thread that owns the points, in
-// registers; each reaches the FP64 accumulators once per group and chunk
-// (xyi_put).
+// registers; each reaches the FP64 accumulators once per group and chunk, in FP32
+// after every FLUSH sources (xyi_put).
 // What bounds the pass is the latency of its operands (phi_q, grad phi_q, Q_q at
 // the plane: read by every target, so from L2): loaded where they are used, they
 // stalled each step for longer than its transforms took (issue slots 27% busy,
@@ -371,6 +371,13 @@ template <typename V, class S, class Op> __host__ inline size_t smem_xyf()
 // are loaded in place and the sums live in shared memory.
 // GS > 1: the first GS - 1 outputs of a group wait in registers.
 constexpr int MAXSRC = 64;           // sources per chunk (plan_chunks): rows of pencil masks in shared memory
+// FP32 sums cover at most FLUSH sources before they go to the FP64 accumulators, so that
+// their rounding stays below that of the products they add (a transform of 6 lines and two
+// complex products each) however many sources there are.  Against one sum per chunk 8
+// cost 2.6 to 3.8% of a mixed pass (27 k-points on 30^3 73.6 -> 76.0 ms, eight atoms on
+// 48^3 40.2 -> 41.8), 4 cost 5.5 to 9% (78.9, 43.7).
+constexpr int FLUSH = 8;
+template <typename V> __device__ __forceinline__ bool flush_due(int si) { return sizeof(V) == 8 && (si + 1) % FLUSH == 0; }
 
 template <class Op, class S, typename V> struct Lay {
     static constexpr int B = S::B;
@@ -575,7 +582,7 @@ __global__ void __launch_bounds__(S::THREADS, ctas_for(S::THREADS, Lay<Op, S, ty
                     if ((bits >> (B * m)) & 1) dst[(size_t)B * m * N] = w[m];
             }
         }
-        if (bn != bg) {                          // the group's last source
+        if (bn != bg || flush_due<V>(si)) {      // the group's last source
             if (on) {
 #pragma unroll
                 for (int a = 0; a < NA; a++)

@@ -63,11 +63,11 @@ __global__ void k_dot3(int N, const double2 *a, const typename C2<T>::t *b, doub
 }
 
 // acc += the splits' sums of the on-chip hf2x, in order
-template <typename V> __global__ void cube_sum(size_t n, int nsplit, const V *part, double2 *acc)
+static __global__ void cube_sum(size_t n, int nsplit, const double2 *part, double2 *acc)
 {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         double2 s = acc[i];
-        for (int k = 0; k < nsplit; k++) s = cadd(s, to64(part[(size_t)k * n + i]));
+        for (int k = 0; k < nsplit; k++) s = cadd(s, part[(size_t)k * n + i]);
         acc[i] = s;
     }
 }
@@ -894,7 +894,7 @@ template <typename T> struct CubeCall {
     const T *tab;
     const int *tb, *sb;
     int nSB, ns, per, nt, splits;
-    V *part;
+    double2 *part;
 };
 template <typename T> int hf_cube(tcg_ctx *c, const CubeCall<T> &call);
 template <typename T> bool hf_cube_has(int n);
@@ -952,13 +952,13 @@ static int run_hf2x_cube(tcg_ctx *c, const Targets &Tg, double2 *acc)
         // about 8 CTAs per SM in all (a partly filled last round then costs
         // little), at least 4 sources each, at most 1 GiB of partial sums
         int splits = std::max(1, std::min((148 * 8 + TR.n - 1) / TR.n, (ns + 3) / 4));
-        splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ((size_t)1 << 30) / (TR.n * N * sizeof(V))));
+        splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ((size_t)1 << 30) / (TR.n * N * sizeof(double2))));
         a.per = (ns + splits - 1) / splits;
         a.splits = (ns + a.per - 1) / a.per;
         std::vector<int> idx(TR.key);
         idx.insert(idx.end(), S.key.begin(), S.key.end());
         TRY(up(c->meta, idx.data(), idx.size() * sizeof(int), c->stream));
-        TRY(c->tmp.ensure((size_t)a.splits * TR.n * N * sizeof(V)));
+        TRY(c->tmp.ensure((size_t)a.splits * TR.n * N * sizeof(double2)));
         a.Rpsi = c->Rpsi.as<V>() + (size_t)TR.t0 * N;
         a.Rocc = c->Rocc.as<V>() + S.base * N;
         a.fill = c->occfill.as<double>() + S.base;
@@ -966,10 +966,10 @@ static int run_hf2x_cube(tcg_ctx *c, const Targets &Tg, double2 *acc)
         a.tb = c->meta.as<int>();
         a.sb = a.tb + TR.n;
         a.nSB = h.nk_all;
-        a.part = c->tmp.as<V>();
+        a.part = c->tmp.as<double2>();
         TRY(hf_cube<T>(c, a));
-        TRY(launch(c, cube_sum<V>, dim3((unsigned)std::min<size_t>(148 * 8, (TR.n * N + 255) / 256)), dim3(256), 0,
-                   (size_t)TR.n * N, a.splits, (const V *)a.part, acc + (size_t)TR.t0 * N));
+        TRY(launch(c, cube_sum, dim3((unsigned)std::min<size_t>(148 * 8, (TR.n * N + 255) / 256)), dim3(256), 0,
+                   (size_t)TR.n * N, a.splits, (const double2 *)a.part, acc + (size_t)TR.t0 * N));
     }
     return TCG_OK;
 }

@@ -296,7 +296,8 @@ struct OpBase {
     // NACC of them, made with at most NOPS operand grids of the source
     // (xyi_operand(k, b0, si), null where unused): xyi_add(si, b0, vals[GS], o,
     // add) calls add(slot, value) for the group b0's contributions at a point,
-    // xyi_put(tj, b0, slot, p, sum) adds a finished sum to its accumulator.
+    // xyi_put(tj, b0, slot, p, sum) adds a finished sum to its FP64 accumulator (FP32: after
+    // every sl::FLUSH sources).
     static constexpr int NACC = 1, NOPS = 1;
     __device__ const V *xyi_operand(int, int, int) const { return nullptr; }
     template <class F> __device__ void xyi_add(int, int, const V *, const V *, F &&) const {}
@@ -394,7 +395,7 @@ struct OpHF2X : OpBase<T> {
     __device__ const V *xyi_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
     template <class F> __device__ void xyi_add(int si, int, const V *v, const V *o, F &&add) const
     {
-        add(0, cscale(cmul(v[0], o[0]), (T)(fill[si])));
+        add(0, cscale64(cmul(v[0], o[0]), fill[si]));
     }
     __device__ const V *xyf_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
     __device__ V xyf_pair(int tj, int, size_t p, const V *o) const { return cmulc(o[0], __ldg(&Rpsi[(size_t)tj * this->g.N + p])); }
@@ -453,7 +454,7 @@ struct OpTC2X : OpBase<T> {
     }
     template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
     {
-        add(0, cscale(cmul(v[0], o[0]), (T)(b == 0 ? fill[si] : -fill[si])));
+        add(0, cscale64(cmul(v[0], o[0]), b == 0 ? fill[si] : -fill[si]));
     }
     __device__ const V *xyf_operand(int, int, int si) const { return Rchi + (size_t)si * this->g.N; }
     __device__ V xyf_pair(int tj, int f, size_t p, const V *o) const
@@ -651,10 +652,9 @@ struct OpTC3A : OpBase<T> {
     static constexpr unsigned BLI = 0xF, BLO = (1u << NB) - 1;
     static constexpr bool REFWD = true;
     static constexpr bool ZSPLIT = false;    // one thread per z-line measured faster here
-    // accumulation through xyi_accum (FP64 red.add per source), so that the
-    // prefetching XYI kernel can transform the re-forwarded planes in place;
-    // with REGACC the per-output FP32 column sums over the chunk's sources
-    // (b = 0 -> acc, b = 1 + 3 xs + d -> qsum[d] when xs == s) are used instead
+    // one-thread and lane-pair forms: accumulation through xyi_accum (FP64 red.add per
+    // source), so that the prefetching XYI kernel can transform the re-forwarded planes
+    // in place
     static constexpr bool REGACC = false, BOUTER = true;
     __device__ bool regacc_grid(int b) const { return b == 0 || EQ || (b - 1) / 3 == s; }
     __device__ V xyi_term(int, int item, int b, size_t p, const V *v) const
@@ -740,7 +740,8 @@ struct OpTC3A : OpBase<T> {
     }
     template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
     {
-        if (regacc_grid(b)) add(0, cscale(cmul(v[0], o[0]), b == 0 ? (T)(fill[si] * b3) : (T)1));
+        const V t = cmul(v[0], o[0]);
+        if (regacc_grid(b)) add(0, b == 0 ? cscale64(t, fill[si] * b3) : t);
     }
     __device__ void xyi_put(int tj, int b, int, size_t p, V sum) const
     {
@@ -790,7 +791,7 @@ struct OpTC3B : OpBase<T> {
     __device__ const V *xyi_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
     template <class F> __device__ void xyi_add(int si, int, const V *v, const V *o, F &&add) const
     {
-        add(0, cscale(cmul(v[0], o[0]), (T)(b6)));
+        add(0, cmul(v[0], o[0]));
     }
     // in the coefficient planes / columns of tc3a3b3b4b6's tables, or after tc2x's
     // V_2body plane (c0 = 1) and in its u column (col = 1) in the shared pass
@@ -804,7 +805,7 @@ struct OpTC3B : OpBase<T> {
         else return this->zdu(c, 2, col >= 0 ? col : (EQ ? s : f / 3), f % 3, z);
     }
     __device__ T zoutc(const ZC &, int, int) const { return (T)0; }
-    __device__ void xyi_put(int tj, int, int, size_t p, V s) const { xyi_flush(tj, p, s); }
+    __device__ void xyi_put(int tj, int, int, size_t p, V s) const { acc_red(acc + (size_t)tj * this->g.N + p, to64(s), b6); }
     const V *Rocc;
     double2 *acc;
     V *tmp2;
@@ -861,7 +862,7 @@ struct OpTC3C : OpBase<T> {
     __device__ const V *xyi_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
     template <class F> __device__ void xyi_add(int si, int, const V *v, const V *o, F &&add) const
     {
-        add(0, cscale(cmul(v[0], o[0]), (T)(b4 * fill[si])));
+        add(0, cscale64(cmul(v[0], o[0]), b4 * fill[si]));
     }
     __device__ const V *xyf_operand(int, int, int si) const { return Rchi + (size_t)si * this->g.N; }
     __device__ V xyf_pair(int tj, int f, size_t p, const V *o) const
@@ -970,7 +971,7 @@ struct OpTC3X : OpBase<T> {
     __device__ const V *xyi_operand(int, int, int si) const { return Rocc + (size_t)si * this->g.N; }
     template <class F> __device__ void xyi_add(int si, int, const V *v, const V *o, F &&add) const
     {
-        add(0, cscale(cmul(v[0], o[0]), (T)(fill[si])));
+        add(0, cscale64(cmul(v[0], o[0]), fill[si]));
     }
     static constexpr int NSO = 2;
     __device__ const V *xyf_operand(int k, int f, int si) const
@@ -1060,15 +1061,15 @@ struct OpQP : OpBase<T> {
     }
     template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
     {
-        const T f1 = (T)fill[si];
+        const double f1 = fill[si];
         int xs, d;
         branch(b, xs, d);
         const V o1 = v[0];
-        if constexpr (BITC) add(0, cscale(cmulc(v[1], o1), -f1));                            // (:392-394)
-        else add(0, V{-f1 * (o1.x * o1.x + o1.y * o1.y), (T)0});                             // (:404-406)
+        if constexpr (BITC) add(0, cscale64(cmulc(v[1], o1), -f1));                          // (:392-394)
+        else add(0, cscale64(V{o1.x * o1.x + o1.y * o1.y, (T)0}, -f1));                      // (:404-406)
         if (xs == sq) {
-            add(1, cscale(cmul(o1, o[0]), f1));
-            if constexpr (BITC) add(2, cscale(cconj(cmul(v[1], o[1])), -f1));                // (:428-430)
+            add(1, cscale64(cmul(o1, o[0]), f1));
+            if constexpr (BITC) add(2, cscale64(cconj(cmul(v[1], o[1])), -f1));              // (:428-430)
         }
     }
     static constexpr int ZK = NF, ZMO = -1;
@@ -1198,8 +1199,7 @@ struct OpTC2X3 : OpTC2X<T> {
     }
     template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
     {
-        const T f = (T)this->fill[si];
-        const V w = cscale(v[0], f);
+        const V w = cscale64(v[0], this->fill[si]);
         if (b == 0) {
             add(0, cmul(w, o[0]));
             return;
@@ -1271,7 +1271,7 @@ struct OpBand : OpBase<T> {
     template <class F> __device__ void xyi_add(int si, int b, const V *v, const V *o, F &&add) const
     {
         const V w = cmul(v[0], o[0]);
-        add(0, b < 3 ? w : cscale(w, (T)(fb5 * fill[si])));
+        add(0, b < 3 ? w : cscale64(w, fb5 * fill[si]));
     }
     __device__ const V *xyf_operand(int, int f, int si) const
     {
