@@ -488,7 +488,6 @@ extern "C" int tcg_qp_finish(tcg_ctx *c)
 extern "C" int tcg_set_pseudo(tcg_ctx *c, const tcg_pseudo_desc *pp)
 {
     if (!c) return fail(TCG_ERR_ARG, "null context");
-    c->h.have_pseudo = false;
     return set_pseudo(c, pp);
 }
 

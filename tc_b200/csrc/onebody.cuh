@@ -90,6 +90,9 @@ __global__ void k_local_real(int N, const typename C2<T>::t *Rpsi, const double 
 static int set_pseudo(tcg_ctx *c, const tcg_pseudo_desc *pp)
 {
     Host &h = c->h;
+    // until this call has succeeded there is no pseudopotential, and a change of the work
+    // grid has no local potential to carry over
+    h.have_pseudo = h.have_vloc = false;
     if (!pp) return fail(TCG_ERR_ARG, "null pseudopotential descriptor");
     if (pp->nspecies < 0 || pp->natoms < 0) return fail(TCG_ERR_ARG, "negative species / atom count");
     if (pp->natoms > 0 && (!pp->species_of_atom || !pp->atom_pos || !pp->nproj || !pp->lbeta || !pp->dij ||
@@ -142,6 +145,8 @@ static int set_pseudo(tcg_ctx *c, const tcg_pseudo_desc *pp)
             }
         }
     }
+    for (int i = 0; pp->vloc && i < h.uN; i++)
+        if (!std::isfinite(pp->vloc[i])) return fail(TCG_ERR_NUMERIC, "non-finite local pseudopotential");
     // B per irreducible k (isym 0, spin 0's plane waves; the reference uses
     // Gindex_at_k[ispin][ik][0], identical for both spins)
     std::vector<double2> B;
@@ -186,14 +191,12 @@ static int set_pseudo(tcg_ctx *c, const tcg_pseudo_desc *pp)
     h.nl_dval_off = voff;
     TRY(up(c->nlB, B.data(), std::max<size_t>(1, B.size()) * sizeof(double2), c->stream));
     TRY(up(c->nlD, dbytes.data(), dbytes.size(), c->stream));
-    h.have_vloc = pp->vloc != nullptr;
-    if (h.have_vloc) {
-        for (int i = 0; i < h.uN; i++)
-            if (!std::isfinite(pp->vloc[i])) return fail(TCG_ERR_NUMERIC, "non-finite local pseudopotential");
+    if (pp->vloc) {
         TRY(up(c->uvloc, pp->vloc, (size_t)h.uN * sizeof(double), c->stream));
         TRY(place_vloc(c));
     }
     TCG_CUDA(cudaStreamSynchronize(c->stream));
+    h.have_vloc = pp->vloc != nullptr;
     h.have_pseudo = true;
     return TCG_OK;
 }

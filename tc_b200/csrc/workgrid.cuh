@@ -252,7 +252,7 @@ static int make_grid(tcg_ctx *c, const int *n, GridDesc &g, DBuf &tw64, DBuf &tw
 
 static int build_prune_table(tcg_ctx *c);
 
-// the local pseudopotential on the work grid (u, w: scratch on the two grids)
+// the local pseudopotential uvloc on the work grid (u, w: scratch on the two grids)
 static int place_vloc_on(tcg_ctx *c, double2 *u, double2 *w)
 {
     const Host &h = c->h;
@@ -265,8 +265,7 @@ static int place_vloc_on(tcg_ctx *c, double2 *u, double2 *w)
 }
 static int place_vloc(tcg_ctx *c)
 {
-    Host &h = c->h;
-    if (!h.have_vloc) return TCG_OK;
+    const Host &h = c->h;
     TRY(c->vloc.ensure((size_t)h.N * sizeof(double)));
     if (!h.reduced) {
         TCG_CUDA(cudaMemcpyAsync(c->vloc.p, c->uvloc.p, (size_t)h.N * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
@@ -341,7 +340,7 @@ static int configure_grid(tcg_ctx *c, bool reduced)
     c->prune_ok = false;
     c->any_ok = !c->fast_n && sl::any_shape(h.n, c->prec == TCG_PREC_FP64 ? sizeof(double2) : sizeof(float2), c->any);
     if (c->fast_n || c->any_ok) TRY(build_prune_table(c));
-    return place_vloc(c);
+    return h.have_vloc ? place_vloc(c) : TCG_OK;
 }
 
 // Choose the work grid for the state whose density is in c->udens and bring the

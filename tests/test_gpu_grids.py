@@ -15,6 +15,7 @@ import numpy as np
 import pytest
 
 from tc_b200 import abi, synth
+from tc_b200 import TCError
 from tc_b200.context import Context
 from oracle import oracle as O
 
@@ -109,6 +110,35 @@ def test_density_beyond_the_pair_sphere():
             g2, g3 = ctx.apply(abi.TERMS_TC)
             assert rel(g2, r2) < TOL["fp64"]
             assert rel(g3, r3) < TOL["fp64"]
+    s.density = plain
+
+
+def test_refused_pseudopotential_and_grid_change():
+    """a local potential that is refused (NaN) leaves none: the next state may change
+    the work grid, and the terms of an earlier pseudopotential are gone"""
+    s = synth.small("TC", nr=(32, 32, 32), nk=1, ecut=6.0, nbands=2, nocc=2, seed=4)
+    good, bad = synth.pseudo(s), synth.pseudo(s)
+    bad.vloc = np.where(np.arange(s.N) == 5, np.nan, bad.vloc)
+    z, y, x = np.meshgrid(*[np.arange(32) / 32.0] * 3, indexing="ij")
+    plain = s.density.copy()
+    wave = 0.05 * np.abs(plain).max() * np.cos(2 * np.pi * (13 * x + 2 * y - 11 * z)).ravel()
+    for first in (None, good):
+        with Context(s, "fp64") as ctx:
+            if first is not None:
+                ctx.set_pseudo(first)
+            with pytest.raises(TCError) as e:
+                ctx.set_pseudo(bad)
+            assert e.value.code == abi.TCG_ERR_NUMERIC
+            with pytest.raises(TCError) as e:
+                ctx.apply_h1(abi.TERM_PSEUDO)
+            assert e.value.code == abi.TCG_ERR_STATE
+            for dens in (plain + wave[None, :], plain):
+                s.density = dens
+                r2, _ = O.apply(s, abi.TERM_TC2X)
+                ctx.set_state()
+                assert rel(ctx.apply(abi.TERM_TC2X)[0], r2) < TOL["fp64"]
+            ctx.set_pseudo(good)
+            assert rel(ctx.apply_h1(abi.TERM_PSEUDO), O.apply_h1(s, abi.TERM_PSEUDO, good)) < TOL["fp64"]
     s.density = plain
 
 
