@@ -307,6 +307,12 @@ static bool all_finite(const double *x, size_t n)
     return s[0] == 0.0;
 }
 
+// No state, nor an occupied-pair stage begun for one, until the caller's is complete
+static void drop_state(tcg_ctx *c)
+{
+    c->h.have_state = c->h.qp_ready = c->h.qp_pending = false;
+}
+
 // upload the orbital / filling part of a state (no R-space work)
 static int tcg_set_state_orbitals_only(tcg_ctx *c, const tcg_state_desc *st)
 {
@@ -315,7 +321,7 @@ static int tcg_set_state_orbitals_only(tcg_ctx *c, const tcg_state_desc *st)
     if (!st->nbands || !st->nocc || !st->filling || !st->phik) return fail(TCG_ERR_ARG, "missing state arrays");
     const bool bitc = h.method == TCG_METHOD_BITC;
     if (bitc && !st->phik_left) return fail(TCG_ERR_ARG, "BITC needs phik_left");
-    h.have_state = false;
+    drop_state(c);
     h.nbands.assign(st->nbands, st->nbands + h.nspin);
     h.nocc.assign(st->nocc, st->nocc + h.nspin * h.nk);
     size_t nfill = 0;
@@ -387,12 +393,14 @@ extern "C" int tcg_refresh_state(tcg_ctx *c)
 {
     if (!c) return fail(TCG_ERR_ARG, "null context");
     if (!c->h.have_state) return fail(TCG_ERR_STATE, "no state to refresh");
+    drop_state(c);                                    // its grids may move to another work grid
     TRY(place_state(c));
     int rc = c->prec == TCG_PREC_FP64 ? build_occupied<double>(c) : build_occupied<float>(c);
     if (rc) return rc;
     rc = c->prec == TCG_PREC_FP64 ? state_terms<double>(c) : state_terms<float>(c);
     if (rc) return rc;
     TCG_CUDA(cudaStreamSynchronize(c->stream));
+    c->h.have_state = true;
     return TCG_OK;
 }
 
@@ -502,6 +510,7 @@ extern "C" int tcg_apply_h1(tcg_ctx *c, uint32_t mask, const int32_t *nb, const 
     const size_t n = psi_count(c, nb);
     if (!all_finite(psi, 2 * n)) return fail(TCG_ERR_NUMERIC, "non-finite value in psi");
     const size_t bytes = n * sizeof(double2);
+    TRY(ensure_grid(c));
     TRY(c->psi.ensure(std::max<size_t>(16, bytes)));
     TRY(c->h1buf.ensure(std::max<size_t>(16, bytes)));
     TCG_CUDA(cudaMemcpyAsync(c->psi.p, psi, bytes, cudaMemcpyHostToDevice, c->stream));
@@ -512,6 +521,9 @@ extern "C" int tcg_apply_h1(tcg_ctx *c, uint32_t mask, const int32_t *nb, const 
     TCG_CUDA(cudaStreamSynchronize(c->stream));
     return TCG_OK;
 }
+
+// Testing aid, not part of tcg.h.
+extern "C" void tcg_debug_fail_alloc(int32_t nth) { g_fail_alloc = nth > 0 ? nth : 0; }
 
 extern "C" int tcg_set_tuning(tcg_ctx *c, int64_t tmp_budget_bytes)
 {
@@ -708,6 +720,7 @@ extern "C" int tcg_density(tcg_ctx *c, const tcg_state_desc *st, double *out)
 {
     if (!c || !st || !out) return fail(TCG_ERR_ARG, "null argument");
     TRY(tcg_set_state_orbitals_only(c, st));
+    TRY(ensure_grid(c));
     Host &h = c->h;
     const size_t N = h.N;
     const bool bitc = h.method == TCG_METHOD_BITC;

@@ -27,6 +27,10 @@ struct Status {
         }                                                                                 \
     } while (0)
 
+// Failure injection of tests (tcg_debug_fail_alloc): the n-th allocation of a DBuf by
+// this thread fails; 0: none does.
+inline thread_local int g_fail_alloc = 0;
+
 // Device buffer (owned).
 struct DBuf {
     void *p = nullptr;
@@ -39,8 +43,9 @@ struct DBuf {
         p = nullptr;
         bytes = 0;
         if (b == 0) return TCG_OK;
-        if (cudaMalloc(&p, b) != cudaSuccess) {
+        if ((g_fail_alloc > 0 && --g_fail_alloc == 0) || cudaMalloc(&p, b) != cudaSuccess) {
             cudaGetLastError();
+            p = nullptr;
             set_error("cudaMalloc of %zu bytes failed", b);
             return TCG_ERR_NOMEM;
         }
@@ -226,6 +231,7 @@ struct tcg_ctx {
     bool prof = false;
     struct ProfRec { const void *fn; const char *tag; cudaEvent_t a, b; double bytes; };
     std::vector<ProfRec> prof_recs;
+    bool grid_ok = false;                   // the work grid's tables are complete (configure_grid)
 };
 
 namespace tcg {

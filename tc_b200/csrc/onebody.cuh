@@ -192,6 +192,7 @@ static int set_pseudo(tcg_ctx *c, const tcg_pseudo_desc *pp)
     TRY(up(c->nlB, B.data(), std::max<size_t>(1, B.size()) * sizeof(double2), c->stream));
     TRY(up(c->nlD, dbytes.data(), dbytes.size(), c->stream));
     if (pp->vloc) {
+        TRY(ensure_grid(c));
         TRY(up(c->uvloc, pp->vloc, (size_t)h.uN * sizeof(double), c->stream));
         TRY(place_vloc(c));
     }

@@ -280,10 +280,12 @@ static int place_vloc(tcg_ctx *c)
     return rc;
 }
 
-// Set up the work grid: the caller's, or red_n^3.
+// Set up the work grid: the caller's, or red_n^3.  When it fails half-way, c->grid_ok
+// stays clear and the next user of the grid sets it up again.
 static int configure_grid(tcg_ctx *c, bool reduced)
 {
     Host &h = c->h;
+    c->grid_ok = false;
     TCG_CUDA(cudaStreamSynchronize(c->stream));
     h.reduced = reduced;
     for (int d = 0; d < 3; d++) h.n[d] = reduced ? h.red_n : h.un[d];
@@ -340,8 +342,11 @@ static int configure_grid(tcg_ctx *c, bool reduced)
     c->prune_ok = false;
     c->any_ok = !c->fast_n && sl::any_shape(h.n, c->prec == TCG_PREC_FP64 ? sizeof(double2) : sizeof(float2), c->any);
     if (c->fast_n || c->any_ok) TRY(build_prune_table(c));
-    return h.have_vloc ? place_vloc(c) : TCG_OK;
+    if (h.have_vloc) TRY(place_vloc(c));
+    c->grid_ok = true;
+    return TCG_OK;
 }
+static int ensure_grid(tcg_ctx *c) { return c->grid_ok ? TCG_OK : configure_grid(c, c->h.reduced); }
 
 // Choose the work grid for the state whose density is in c->udens and bring the
 // density onto it.
@@ -372,7 +377,7 @@ static int place_state(tcg_ctx *c)
         for (int s = 0; s < 2; s++)
             if (!(m2[2 * s + 1] <= 1e-26 * m2[2 * s])) want = false;
     }
-    if (want != h.reduced) TRY(configure_grid(c, want));
+    if (want != h.reduced || !c->grid_ok) TRY(configure_grid(c, want));
     if (hf) return TCG_OK;
     TRY(c->dens.ensure(2 * (size_t)h.N * sizeof(double2)));
     if (!h.reduced) {

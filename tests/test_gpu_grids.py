@@ -11,6 +11,8 @@ grid, against the oracle.
 
 Tolerances as in test_gpu_parity.py: FP64 relative 1e-10, mixed 2e-5.
 """
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -140,6 +142,67 @@ def test_refused_pseudopotential_and_grid_change():
             ctx.set_pseudo(good)
             assert rel(ctx.apply_h1(abi.TERM_PSEUDO), O.apply_h1(s, abi.TERM_PSEUDO, good)) < TOL["fp64"]
     s.density = plain
+
+
+@pytest.mark.parametrize("how", ["set_state", "refresh_state"])
+def test_failed_allocation_during_a_grid_change(how):
+    """each allocation of a state that moves to another work grid fails in turn (on the
+    host): there is no state afterwards, and the next one is right"""
+    import ctypes
+    from tc_b200._lib import lib
+    arm = lib().tcg_debug_fail_alloc
+    arm.argtypes, arm.restype = [ctypes.c_int32], None
+    s = synth.small("TC", nr=(24, 24, 24), nk=1, ecut=3.5, nbands=2, nocc=2, seed=4)
+    plain = s.density.copy()
+    beyond = plain + 0.05 * np.abs(plain).max() * np.cos(2 * np.pi * 10 * (np.arange(s.N) % 24) / 24.0)[None, :]
+    d0 = O.density(s)
+    s.density = beyond
+    r2, r3 = O.apply(s, abi.TERMS_TC)
+    p2, p3 = O.apply(dataclasses.replace(s, density=plain), abi.TERMS_TC)
+    failures = 0
+    for nth in range(1, 200):
+        s.density = plain
+        with Context(s, "fp64") as ctx:
+            ctx.set_state()
+            if how == "set_state":
+                s.density, want = beyond, (r2, r3)
+            else:
+                ctx.set_forms(xy=1)                        # keeps to the caller's grid
+                want = (p2, p3)
+            arm(nth)
+            try:
+                getattr(ctx, how)()
+            except TCError as e:
+                assert e.code == abi.TCG_ERR_NOMEM
+            else:
+                break
+            finally:
+                arm(0)
+            failures += 1
+            for call in (lambda: ctx.apply(abi.TERMS_TC), ctx.refresh_state, ctx.qp_finish):
+                with pytest.raises(TCError) as e:
+                    call()
+                assert e.value.code == abi.TCG_ERR_STATE
+            assert rel(ctx.density(), d0) < 1e-12
+            assert rel(ctx.apply_h1(abi.TERM_KINETIC), O.apply_h1(s, abi.TERM_KINETIC)) < TOL["fp64"]
+            ctx.set_state()
+            g2, g3 = ctx.apply(abi.TERMS_TC)
+            assert rel(g2, want[0]) < TOL["fp64"]
+            assert rel(g3, want[1]) < TOL["fp64"]
+    s.density = plain
+    assert failures >= 8                                   # twiddles, maps, density, orbital grids, local potentials
+
+
+def test_no_stage_survives_its_state():
+    """the occupied-pair stage begun for a state is gone with it"""
+    s = synth.small("TC", nr=(12, 12, 12), nk=1, ecut=2.5, nbands=2, nocc=2, seed=4)
+    with Context(s, "fp64") as ctx:
+        ctx.set_state()
+        ctx.qp_partial(0, 1)
+        ctx.density()
+        with pytest.raises(TCError) as e:
+            ctx.qp_finish()
+        assert e.value.code == abi.TCG_ERR_STATE
 
 
 @pytest.mark.parametrize("method", ["HF", "TC", "BITC"])
