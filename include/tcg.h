@@ -344,6 +344,13 @@ int tcg_qp_finish(tcg_ctx *ctx);
  * counterpart (TC++ has no chunked pair pipeline). */
 int tcg_set_tuning(tcg_ctx *ctx, int64_t tmp_budget_bytes);
 
+/* The FFT grid the library works on: the caller's (nr), or a smaller cube that
+ * gives the same results (band-limited products; a TC / BITC density with a
+ * component of more than 1e-13 of its largest beyond twice the plane-wave sphere's
+ * radius keeps the caller's grid).  tcg_set_state and tcg_refresh_state choose it
+ * for the state's density; a change rebuilds the grid's tables on the host. */
+int tcg_work_grid(tcg_ctx *ctx, int32_t n[3]);
+
 /* Kernel forms of the pass pipelines (the choices an autotuner explores; no
  * reference counterpart).  xy: 0 = each term's default (split lines on the
  * grids that have them), 1 = one thread per line, 2 = a lane pair per line,

@@ -75,6 +75,12 @@ class Context:
     def set_tuning(self, tmp_budget):
         check(lib().tcg_set_tuning(self.handle, int(tmp_budget)))
 
+    def work_grid(self):
+        """(n0, n1, n2) of the FFT grid the library works on (tcg_work_grid)."""
+        n = (C.c_int32 * 3)()
+        check(lib().tcg_work_grid(self.handle, n))
+        return tuple(n)
+
     def forms(self):
         """The kernel forms in use (tcg_get_forms) as a dict."""
         f = abi.Forms()

@@ -522,6 +522,13 @@ extern "C" int tcg_apply_h1(tcg_ctx *c, uint32_t mask, const int32_t *nb, const 
     return TCG_OK;
 }
 
+extern "C" int tcg_work_grid(tcg_ctx *c, int32_t *n)
+{
+    if (!c || !n) return fail(TCG_ERR_ARG, "null argument");
+    for (int d = 0; d < 3; d++) n[d] = c->h.n[d];
+    return TCG_OK;
+}
+
 // Testing aid, not part of tcg.h.
 extern "C" void tcg_debug_fail_alloc(int32_t nth) { g_fail_alloc = nth > 0 ? nth : 0; }
 

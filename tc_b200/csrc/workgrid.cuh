@@ -125,12 +125,14 @@ static double miller_extent(const Host &h, int i)
 }
 
 // Edge of the cheapest compiled cubic grid that gives the caller's results (0:
-// none smaller than the caller's).  Sets h.rmax.  That is the smallest, except
-// where its lines split badly (15 = 5 x 3, 27 = 9 x 3, 45 = 9 x 5: most threads of
-// the shorter step wait) and the next size fits as well: a TC apply of 8 k-points
-// takes 1.02 ms on 15^3 and 0.93 on 16^3 (FP64 1.53 and 1.51), in FP64 12.7 ms on
-// 27^3 and 10.4 on 30^3, 1.58 on 45^3 and 1.52 on 48^3; in FP32 27 and 45 stay
-// ahead (5.08 and 5.37 ms, 0.93 and 0.98).
+// the caller's own).  Sets h.rmax.  That is the smallest, except where its lines
+// split badly (15 = 5 x 3, 27 = 9 x 3, 45 = 9 x 5: most threads of the shorter step
+// wait) and the next size fits as well or is the caller's own.  An apply at the
+// cutoff of the smaller size, ms on it and on the next:
+//            FP32 TC      HF            FP64 TC      HF
+//   15, 16   1.02  0.93   0.146 0.133   1.53  1.51   0.216 0.188   next in both
+//   27, 30   5.08  5.37   0.83  0.86    12.7  10.4   1.45  1.35    next in FP64
+//   45, 48   0.93  0.98   0.238 0.246   1.58  1.52   0.312 0.322   next in FP64 TC
 static int choose_reduced(Host &h, bool fp64)
 {
     h.rmax = 0;
@@ -176,7 +178,11 @@ static int choose_reduced(Host &h, bool fp64)
         if (best) {
             if (done) return;
             done = true;
-            if (!(best == 15 || (fp64 && (best == 27 || best == 45)))) return;
+            if (!(best == 15 || (fp64 && (best == 27 || (best == 45 && !hf))))) return;
+            if (h.un[0] == n && h.un[1] == n && h.un[2] == n) {
+                best = 0;
+                return;
+            }
         }
         if (pts > (user_fast ? 0.9 : 1.0) * h.uN) return;
         if (!(shortest_period(h, n3) > need)) return;

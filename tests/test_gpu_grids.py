@@ -30,11 +30,14 @@ def rel(a, b):
     return d / m if m > 0 else d
 
 
-def check(s, mask, prec):
+def check(s, mask, prec, edge=None):
+    """apply against the oracle; edge: the work grid's"""
     r2, r3 = O.apply(s, mask)
     with Context(s, prec) as ctx:
         ctx.set_state()
         g2, g3 = ctx.apply(mask)
+        if edge:
+            assert ctx.work_grid() == (edge,) * 3
     assert rel(g2, r2) < TOL[prec]
     if mask & ~abi.TERMS_H2:
         assert rel(g3, r3) < TOL[prec]
@@ -87,14 +90,32 @@ def test_work_grid_time_reversal(method, prec):
     check(s, abi.TERMS_HF if method == "HF" else abi.TERMS_TC, prec)
 
 
+def at_edge(n, fac):
+    """cutoff for which n^3 is the smallest grid with periods longer than fac R"""
+    return 0.5 * (0.985 * n * np.sqrt(3.0) * 2.0 * np.pi / 10.26 / fac) ** 2
+
+
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 @pytest.mark.parametrize("n,user", [(15, 20), (15, 15), (27, 32), (45, 48)])
 def test_work_grid_of_uneven_lines(n, user, prec):
     """n^3 is the smallest work grid; the next size is taken where n's lines split
-    badly (15, in FP64 27 and 45) unless the caller's grid is smaller than that"""
-    ecut = 0.5 * (0.985 * n * np.sqrt(3.0) * 2.0 * np.pi / 10.26 / 6.0) ** 2
-    s = synth.small("TC", nr=(user, user, user), nk=1, ecut=ecut, nbands=2, nocc=1, seed=n)
-    check(s, abi.TERMS_TC, prec)
+    badly (15, in FP64 27 and 45)"""
+    s = synth.small("TC", nr=(user, user, user), nk=1, ecut=at_edge(n, 6.0), nbands=2, nocc=1, seed=n)
+    edge = {(15, 20): 16, (15, 15): 15, (27, 32): 30, (45, 48): 48}[n, user] if prec == "fp64" or n == 15 else n
+    check(s, abi.TERMS_TC, prec, edge)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("method", ["HF", "TC"])
+@pytest.mark.parametrize("n,user", [(15, 16), (27, 30), (45, 48), (25, 27)])
+def test_work_grid_next_to_the_callers(n, user, method, prec):
+    """where the size that replaces a badly splitting one is the caller's own, the
+    caller's grid stays; other sizes one step below the caller's are taken (when they
+    save a tenth of the points)"""
+    s = synth.small(method, nr=(user, user, user), nk=1, ecut=at_edge(n, 6.0 if method == "TC" else 4.0), nbands=1, nocc=1)
+    stay = n == 15 or (prec == "fp64" and (n == 27 or (n == 45 and method == "TC")))
+    with Context(s, prec) as ctx:
+        assert ctx.work_grid() == ((user if stay else n),) * 3
 
 
 def test_density_beyond_the_pair_sphere():
