@@ -339,7 +339,9 @@ int tcg_qp_partial(tcg_ctx *ctx, int32_t rank, int32_t nranks, void **buf_dev, s
 int tcg_qp_finish(tcg_ctx *ctx);
 
 /* Tuning knob: bytes of pass temporaries one chunk of (target x source)
- * pairs may use (0 = default, 8 GiB).  Smaller chunks keep the temporaries
+ * pairs may use (0 = default, 8 GiB); the kernel table and the partial sums of
+ * the on-chip hf2x and the scratch of tc3a2a4b2b5's rotations stay within it too
+ * (and within 1 GiB each).  Smaller chunks keep the temporaries
  * resident in L2; larger ones launch fewer kernels.  No reference
  * counterpart (TC++ has no chunked pair pipeline). */
 int tcg_set_tuning(tcg_ctx *ctx, int64_t tmp_budget_bytes);

@@ -624,12 +624,14 @@ static int min_targets(const tcg_ctx *c)
 }
 
 // chunk budget: tmp slots bytes <= c->tmp_budget
+static size_t tmp_budget(const tcg_ctx *c) { return c->tmp_budget ? c->tmp_budget : ((size_t)8 << 30); }
 static size_t max_items_for(const tcg_ctx *c, int nslots, size_t vbytes)
 {
     const size_t per = (size_t)nslots * c->h.N * vbytes;
-    const size_t budget = c->tmp_budget ? c->tmp_budget : ((size_t)8 << 30);
-    return std::min<size_t>(65535, std::max<size_t>(1, budget / per));   // grid.y limit
+    return std::min<size_t>(65535, std::max<size_t>(1, tmp_budget(c) / per));   // grid.y limit
 }
+// scratch that gains nothing beyond 1 GiB
+static size_t small_budget(const tcg_ctx *c) { return std::min(tmp_budget(c), (size_t)1 << 30); }
 
 // Fast-path launcher, defined in fast_launch.cuh and instantiated per grid
 // size in fast_inst.cu (one translation unit per N).
@@ -900,16 +902,20 @@ template <typename T> int hf_cube(tcg_ctx *c, const CubeCall<T> &call);
 template <typename T> bool hf_cube_has(int n);
 
 // The kernel 1 / |k - q + G|^2 of every (irreducible k, all-k q) pair depends on
-// the geometry alone: laid out once per context (and work grid), if it stays
-// below 1 GiB.
+// the geometry alone: laid out once per context (and work grid), if the budget of
+// temporaries holds it, at most 1 GiB.  Otherwise hf2x takes the passes, whose
+// tables are as small as their chunks.
 template <typename T>
 static int hf_cube_table(tcg_ctx *c, bool &ok)
 {
     const Host &h = c->h;
     const size_t npair = (size_t)h.nk * h.nk_all;
-    ok = false;
-    if (!split_xy(c) || !split_z(c) || !hf_cube_has<T>(c->fast_n) || npair * h.N * sizeof(T) > ((size_t)1 << 30)) return TCG_OK;
-    ok = true;
+    ok = split_xy(c) && split_z(c) && hf_cube_has<T>(c->fast_n) && npair * h.N * sizeof(T) <= small_budget(c);
+    if (!ok) {
+        c->hftab.release();                           // of a larger budget
+        c->hftab_ok = false;
+        return TCG_OK;
+    }
     if (c->hftab_ok) return TCG_OK;
     std::vector<double> kq(3 * npair);
     for (int k = 0; k < h.nk; k++)
@@ -946,30 +952,34 @@ static int run_hf2x_cube(tcg_ctx *c, const Targets &Tg, double2 *acc)
         Sources S = sources_of(c, s);
         const int ns = (int)S.key.size();
         if (TR.n == 0 || ns == 0) continue;
-        CubeCall<T> a;
-        a.nt = TR.n;
-        a.ns = ns;
-        // about 8 CTAs per SM in all (a partly filled last round then costs
-        // little), at least 4 sources each, at most 1 GiB of partial sums
-        int splits = std::max(1, std::min((148 * 8 + TR.n - 1) / TR.n, (ns + 3) / 4));
-        splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ((size_t)1 << 30) / (TR.n * N * sizeof(double2))));
-        a.per = (ns + splits - 1) / splits;
-        a.splits = (ns + a.per - 1) / a.per;
         std::vector<int> idx(TR.key);
         idx.insert(idx.end(), S.key.begin(), S.key.end());
         TRY(up(c->meta, idx.data(), idx.size() * sizeof(int), c->stream));
-        TRY(c->tmp.ensure((size_t)a.splits * TR.n * N * sizeof(double2)));
-        a.Rpsi = c->Rpsi.as<V>() + (size_t)TR.t0 * N;
+        CubeCall<T> a;
+        a.ns = ns;
         a.Rocc = c->Rocc.as<V>() + S.base * N;
         a.fill = c->occfill.as<double>() + S.base;
         a.tab = c->hftab.as<T>();
-        a.tb = c->meta.as<int>();
-        a.sb = a.tb + TR.n;
+        a.sb = c->meta.as<int>() + TR.n;
         a.nSB = h.nk_all;
-        a.part = c->tmp.as<double2>();
-        TRY(hf_cube<T>(c, a));
-        TRY(launch(c, cube_sum, dim3((unsigned)std::min<size_t>(148 * 8, (TR.n * N + 255) / 256)), dim3(256), 0,
-                   (size_t)TR.n * N, a.splits, (const double2 *)a.part, acc + (size_t)TR.t0 * N));
+        // targets whose sums the budget holds at a time; of their sources about 8 CTAs
+        // per SM in all (a partly filled last round then costs little), at least 4 each,
+        // and as many partial sums as the budget holds
+        const size_t fit = std::max<size_t>(1, small_budget(c) / (N * sizeof(double2)));
+        for (int t0 = 0; t0 < TR.n; t0 += a.nt) {
+            a.nt = (int)std::min<size_t>(TR.n - t0, fit);
+            int splits = std::max(1, std::min((148 * 8 + a.nt - 1) / a.nt, (ns + 3) / 4));
+            splits = (int)std::max<size_t>(1, std::min<size_t>(splits, fit / a.nt));
+            a.per = (ns + splits - 1) / splits;
+            a.splits = (ns + a.per - 1) / a.per;
+            TRY(c->tmp.ensure((size_t)a.splits * a.nt * N * sizeof(double2)));
+            a.Rpsi = c->Rpsi.as<V>() + (size_t)(TR.t0 + t0) * N;
+            a.tb = c->meta.as<int>() + t0;
+            a.part = c->tmp.as<double2>();
+            TRY(hf_cube<T>(c, a));
+            TRY(launch(c, cube_sum, dim3((unsigned)std::min<size_t>(148 * 8, (a.nt * N + 255) / 256)), dim3(256), 0,
+                       (size_t)a.nt * N, a.splits, (const double2 *)a.part, acc + (size_t)(TR.t0 + t0) * N));
+        }
     }
     return TCG_OK;
 }
@@ -1430,9 +1440,9 @@ static int qp_finish(tcg_ctx *c)
     TRY(c->V3b2.ensure((size_t)ns * N * sizeof(double2)));
     TRY(launch(c, k_zero, dim3(pblocks), dim3(256), 0, c->V3a2.as<double2>(), (size_t)ns * N));
     TRY(launch(c, k_zero, dim3(pblocks), dim3(256), 0, c->V3b2.as<double2>(), (size_t)ns * N));
-    // fp64 work of the rotations: 6 + nspin grids per item, at most 1 GiB (as far as one item fits)
+    // fp64 work of the rotations: 6 + nspin grids per item, as many items as the budget holds (one at least)
     const size_t per = (size_t)(6 + ns) * N * sizeof(double2);
-    const size_t ng = std::max<size_t>(1, std::min<size_t>({h.nocc_grids, ((size_t)1 << 30) / per, (size_t)65535}));
+    const size_t ng = std::max<size_t>(1, std::min<size_t>({h.nocc_grids, small_budget(c) / per, (size_t)65535}));
     DBuf &rot = c->rotw;
     TRY(rot.ensure(ng * per));
     DBuf &q3b2 = c->q3b2w;

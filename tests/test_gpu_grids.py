@@ -81,6 +81,46 @@ def test_on_chip_exchange(n, ecut, prec):
     check(s, abi.TERM_HF2X, prec)
 
 
+@pytest.mark.parametrize("prec,n,ecut", [("mixed", 20, 12.0), ("fp64", 18, 10.0)])
+@pytest.mark.parametrize("budget", [1 << 20, 8 << 20])
+def test_exchange_within_the_budget(budget, prec, n, ecut):
+    """hf2x with a small budget of temporaries (1 MB: its kernel table does not fit and
+    the passes run; 8 MB: on chip, targets in parts): results, and the device memory
+    that an apply adds.  Besides twice the budget (temporaries and table) these are
+    the orbitals on the grid, the accumulators, psi and h2, and 8 MB of small
+    allocations; the partial sums alone were 47 MB in FP64 and 65 MB in mixed precision."""
+    import torch
+    s = synth.small("HF", nr=(36, 36, 36), nk=2, ecut=ecut, nbands=8, nocc=4, seed=n)
+    r2, _ = O.apply(s, abi.TERM_HF2X)
+    nt = 8 * 8
+    rest = nt * n ** 3 * (16 + (16 if prec == "fp64" else 8)) + 2 * s.psi.nbytes + (8 << 20)
+    for _ in range(2):                                     # the first loads the kernels
+        with Context(s, prec, tmp_budget=budget) as ctx:
+            ctx.set_state()
+            assert ctx.work_grid() == (n,) * 3
+            torch.cuda.synchronize()
+            free = torch.cuda.mem_get_info()[0]
+            g2, _ = ctx.apply(abi.TERM_HF2X)
+            grown = free - torch.cuda.mem_get_info()[0]
+            ctx.profile(True)
+            ctx.apply(abi.TERM_HF2X)
+            tags = set(ctx.profile_read())
+        assert rel(g2, r2) < TOL[prec]
+    assert ("hf2x:cube" in tags) == (budget > 1 << 20)
+    assert grown <= 2 * budget + rest
+
+
+def test_rotations_within_the_budget():
+    """tc3a2a4b2b5 with scratch for one rotated orbital at a time"""
+    s = synth.small("BITC", nr=(12, 12, 12), tr=True, ecut=2.5, nbands=2, nocc=2)
+    r2, r3 = O.apply(s, abi.TERMS_TC)
+    with Context(s, "fp64", tmp_budget=1 << 18) as ctx:
+        ctx.set_state()
+        g2, g3 = ctx.apply(abi.TERMS_TC)
+    assert rel(g2, r2) < TOL["fp64"]
+    assert rel(g3, r3) < TOL["fp64"]
+
+
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 @pytest.mark.parametrize("method", ["HF", "TC"])
 def test_work_grid_time_reversal(method, prec):
