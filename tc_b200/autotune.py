@@ -2,9 +2,9 @@
 
 The library's kernel choices (tcg_forms: the XY and Z kernel forms, the
 prefetching inverse XY pass, pruning of band-limited grids, the shared
-transforms of tc2x / tc3a3b3b4b6 / tc3a2a4b2b5, the shared-memory
-accumulations, the targets per chunk) have per-term defaults measured on the
-36^3 production grid.  autotune() times the caller's own step -- the
+transforms of tc2x / tc3a3b3b4b6 / tc3a2a4b2b5, the targets per chunk) have
+defaults; the forms of one thread or a lane pair per line also move the library
+from its smaller work grid to the caller's (Context.work_grid).  autotune() times the caller's own step -- the
 per-state refresh and one apply of the given terms on device buffers -- for
 each value of one knob at a time, keeps the fastest (coordinate descent, a
 second sweep while it still improves) and leaves the context set to it.  Every
@@ -13,15 +13,14 @@ not support are skipped.
 """
 from ._lib import TCError
 
-#: knobs in the order they are swept, with the values tried
+#: knobs in the order they are swept, with the values tried (xy = 3 and z = 3, 4 name the
+#: default's split lines, qp_sacc and sacc have no effect)
 KNOBS = (
     ("fuse", (1, 0)),
     ("prune", (1, 0)),
-    ("xy", (0, 1, 2, 3)),
-    ("z", (0, 1, 2, 3, 4)),
+    ("xy", (0, 1, 2)),
+    ("z", (0, 1, 2)),
     ("prefetch", (1, 0)),
-    ("qp_sacc", (1, 0)),
-    ("sacc", (0, 1)),
     ("min_targets", (0, 300, 1200)),
 )
 

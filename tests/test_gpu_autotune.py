@@ -47,7 +47,14 @@ def test_forms_round_trip_and_rejection():
         ctx.set_forms(xy=1, z=2, prefetch=0)
         assert ctx.forms() == dict(f, xy=1, z=2, prefetch=0)
         with pytest.raises(TCError) as e:
-            ctx.set_forms(xy=3)          # six threads per line exist for 36^3 only
+            ctx.set_forms(xy=3)          # by number on 36^3 and 48^3 only
         assert e.value.code == abi.TCG_ERR_UNSUPPORTED
         with pytest.raises(TCError):
             ctx.set_forms(z=9)
+
+
+def test_no_candidate_twice():
+    """every value of a knob is a kernel of its own"""
+    from tc_b200.autotune import KNOBS
+    assert dict(KNOBS)["xy"] == (0, 1, 2) and dict(KNOBS)["z"] == (0, 1, 2)
+    assert not {"qp_sacc", "sacc"} & set(dict(KNOBS))

@@ -342,23 +342,26 @@ def test_36_pruned_transforms(monkeypatch, method, prune, prec, tol):
 
 
 @pytest.mark.parametrize("method", ["TC", "BITC"])
-@pytest.mark.parametrize("sacc", ["qp-default", "qp-off", "3a3b6A-on"])
-def test_36_shared_memory_accumulation(monkeypatch, method, sacc):
-    """36^3 mixed precision: the inverse XY pass summing a chunk's sources in
-    FP32 shared-memory planes -- on by default for the occupied-pair stage of
-    tc3a2a4b2b5 (TCG_NO_QP_SACC turns it off), optional for the first stage
-    of tc3a3b3b4b6 (TCG_SACC) -- vs the oracle"""
-    if sacc == "qp-off":
-        monkeypatch.setenv("TCG_NO_QP_SACC", "1")
-    if sacc == "3a3b6A-on":
-        monkeypatch.setenv("TCG_SACC", "1")
+@pytest.mark.parametrize("sacc", ["qp-off", "3a3b6A-on"])
+def test_36_accumulation_flags(monkeypatch, method, sacc):
+    """36^3 mixed precision: the flags qp_sacc and sacc (TCG_NO_QP_SACC, TCG_SACC) are
+    read back as set and change nothing: the results are the default's bit for bit, and
+    the oracle's"""
     s = system(method, nr=(36, 36, 36), nk=2, ecut=4.0, nbands=3, nocc=2)
     for mask in (abi.TERM_TC3A2A4B2B5, abi.TERM_TC3A3B3B4B6):
         _, r3 = oracle_terms(s, mask)
-        with Context(s, "mixed") as ctx:
-            ctx.set_state()
-            _, g3 = ctx.apply(mask)
-        assert rel(g3, r3) < MIXED_TOL
+        out = []
+        for on in (False, True):
+            if on:
+                monkeypatch.setenv("TCG_NO_QP_SACC" if sacc == "qp-off" else "TCG_SACC", "1")
+            with Context(s, "mixed") as ctx:
+                f = ctx.forms()
+                assert (f["qp_sacc"], f["sacc"]) == ((1, 0) if not on else ((0, 0) if sacc == "qp-off" else (1, 1)))
+                ctx.set_state()
+                out.append(ctx.apply(mask)[1])
+            monkeypatch.undo()
+        assert rel(out[0], r3) < MIXED_TOL
+        assert np.array_equal(out[0], out[1])
 
 
 @pytest.mark.parametrize("prec,tol", [("fp64", FP64_TOL), ("mixed", MIXED_TOL)])
