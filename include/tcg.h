@@ -358,16 +358,20 @@ int tcg_work_grid(tcg_ctx *ctx, int32_t n[3]);
  * grids that have them), 1 = one thread per line, 2 = a lane pair per line,
  * 3 = split lines; z: 0 = default, 1 = one thread per z-line, 2 = a lane
  * pair, 3 and 4 = split lines (one kernel since their inputs need no copy in
- * shared memory).  xy = 3 and z = 3, 4 are refused except on 36^3 and 48^3
- * (elsewhere split lines are the default anyway); 1 and 2 act on cubic grids of
+ * shared memory).  Split lines are the default of every grid that has them, so
+ * 3 and 4 choose nothing new; they are refused unless the caller's grid is
+ * 36^3 or 48^3, as before.  1 and 2 act on cubic grids of
  * side 12, 16, 24, 32, 36, 40, 48, turn the pruning of band-limited grids off
- * (only the split lines honour it) and keep the library on the caller's grid.
+ * (only the split lines honour it) and keep the library on the caller's grid: when
+ * that moves the work grid, tcg_set_forms redoes the state's work as
+ * tcg_refresh_state does (an occupied-pair stage in progress is dropped; on an error
+ * the state is gone).
  * Flags, each 0 or 1: prefetch (the one-thread and lane-pair inverse XY passes copy
  * the next plane set while they transform the current one; split lines always
  * do), prune (band-limited grids on the pencils their support meets), fuse
  * (tc2x, tc3a3b3b4b6 and tc3a2a4b2b5's band part share their transforms),
- * qp_sacc / sacc (kept for callers that set them: the inverse XY passes always
- * sum a chunk's sources on chip).  min_targets: targets per chunk (0 =
+ * qp_sacc / sacc (without effect, kept for callers that set them: the inverse XY
+ * passes always sum on chip).  min_targets: targets per chunk (0 =
  * default).  tcg_get_forms reads the current choice. */
 typedef struct tcg_forms {
     int32_t xy, z, prefetch, prune, fuse, qp_sacc, sacc, min_targets;

@@ -264,7 +264,7 @@ extern "C" int tcg_ctx_create(const tcg_system_desc *sys, int32_t precision, tcg
     if ((rc = make_grid(c, h.un, c->ugd, c->utw64, c->utw32)) ||
         (rc = up(c->recip, h.recip, sizeof h.recip, c->stream)) ||
         (rc = up(c->phase, sys->phase, ngi * sizeof(double2), c->stream)) ||
-        (rc = configure_grid(c, h.red_n && c->xy_kernels == 0 && c->z_kernels == 0 && !c->force_generic))) {
+        (rc = configure_grid(c, forms_reduce(c)))) {
         tcg_ctx_destroy(c);
         return rc;
     }
@@ -547,6 +547,7 @@ extern "C" int tcg_set_forms(tcg_ctx *c, const tcg_forms *f)
     const int *un = c->h.un;
     if (!(un[0] == un[1] && un[1] == un[2] && split_line_grid(un[0])) && (f->xy == 3 || f->z >= 3))
         return fail(TCG_ERR_UNSUPPORTED, "split-line kernel forms need a 36^3 or 48^3 grid");
+    const bool before = forms_reduce(c);
     c->xy_kernels = f->xy;
     c->z_kernels = f->z;
     c->no_prefetch = !f->prefetch;
@@ -555,6 +556,10 @@ extern "C" int tcg_set_forms(tcg_ctx *c, const tcg_forms *f)
     c->qp_sacc = f->qp_sacc != 0;
     c->use_sacc = f->sacc != 0;
     c->min_targets = f->min_targets;
+    // forms that need the caller's grid, or give it up, take the state along (a density
+    // may keep the caller's grid in any case: then nothing moves)
+    const bool after = forms_reduce(c);
+    if (c->h.have_state && after != before && (after || c->h.reduced)) return tcg_refresh_state(c);
     return TCG_OK;
 }
 

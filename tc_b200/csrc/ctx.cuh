@@ -219,11 +219,11 @@ struct tcg_ctx {
     bool any_ok = false;                    // split-line passes with the run-time shape `any` (fast_n == 0)
     tcg::sl::AnyShape any;
     bool force_generic = false;             // use the generic pass kernels even if fast_n is set
-    int xy_kernels = 0;                     // fast XY passes: 0 default, 1 all line, 2 all lane-pair, 3 split lines (36^3, 48^3)
+    int xy_kernels = 0;                     // fast XY passes: 0 default (split lines), 1 all line, 2 all lane-pair, 3 split lines
     bool no_prefetch = false;               // fast XYI: no prefetch of the next plane set
     const char *stage = "misc";            // profiling tag of untagged launches (the current stage)
-    int z_kernels = 0;                      // fast Z pass: 0 per-term choice, 1 one thread per line, 2 lane pairs,
-                                            // 3 / 4 split lines in shared memory / registers (36^3, 48^3)
+    int z_kernels = 0;                      // fast Z pass: 0 default (split lines), 1 one thread per line, 2 lane
+                                            // pairs, 3 and 4 split lines
     size_t tmp_budget = 0;                  // bytes per chunk of pass temporaries (0: default 8 GiB)
     int min_targets = 0;                    // targets per chunk (0: default, about 12 waves of XYI CTAs)
     int64_t launches = 0;

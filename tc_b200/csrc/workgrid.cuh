@@ -352,6 +352,11 @@ static int configure_grid(tcg_ctx *c, bool reduced)
     c->grid_ok = true;
     return TCG_OK;
 }
+// The kernel forms in use run on the smaller grid: split lines, by default or by number
+static bool forms_reduce(const tcg_ctx *c)
+{
+    return c->h.red_n && (c->xy_kernels == 0 || c->xy_kernels == 3) && (c->z_kernels == 0 || c->z_kernels >= 3) && !c->force_generic;
+}
 static int ensure_grid(tcg_ctx *c) { return c->grid_ok ? TCG_OK : configure_grid(c, c->h.reduced); }
 
 // Choose the work grid for the state whose density is in c->udens and bring the
@@ -361,7 +366,7 @@ static int place_state(tcg_ctx *c)
     Host &h = c->h;
     const bool hf = h.method == TCG_METHOD_HF;
     const size_t uN = h.uN;
-    bool want = h.red_n && c->xy_kernels == 0 && c->z_kernels == 0 && !c->force_generic;
+    bool want = forms_reduce(c);
     if (want && !hf) {
         // density in G; its largest component beyond 2 R against its largest
         TRY(c->uwork.ensure(2 * uN * sizeof(double2) + 4 * sizeof(unsigned long long)));

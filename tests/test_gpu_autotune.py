@@ -53,6 +53,23 @@ def test_forms_round_trip_and_rejection():
             ctx.set_forms(z=9)
 
 
+def test_forms_take_effect_at_once():
+    """a form that needs the caller's grid moves the state there before the next apply,
+    the split lines by number stay on the smaller grid"""
+    s = synth.small("TC", nr=(36, 36, 36), nk=1, ecut=6.0, nbands=2, nocc=1, seed=9)
+    r2, r3 = O.apply(s, abi.TERMS_TC)
+    with Context(s, "fp64") as ctx:
+        ctx.set_state()
+        small = ctx.work_grid()
+        assert small[0] < 36
+        for forms, grid in ((dict(xy=3, z=4), small), (dict(xy=1, z=1), (36,) * 3), (dict(xy=0, z=0), small)):
+            ctx.set_forms(**forms)
+            assert ctx.work_grid() == grid, forms
+            g2, g3 = ctx.apply(abi.TERMS_TC)
+            assert rel(g2, r2) < 1e-10, forms
+            assert rel(g3, r3) < 1e-10, forms
+
+
 def test_no_candidate_twice():
     """every value of a knob is a kernel of its own"""
     from tc_b200.autotune import KNOBS

@@ -205,7 +205,7 @@ def test_refused_pseudopotential_and_grid_change():
     s.density = plain
 
 
-@pytest.mark.parametrize("how", ["set_state", "refresh_state"])
+@pytest.mark.parametrize("how", ["set_state", "set_forms"])
 def test_failed_allocation_during_a_grid_change(how):
     """each allocation of a state that moves to another work grid fails in turn (on the
     host): there is no state afterwards, and the next one is right"""
@@ -228,11 +228,13 @@ def test_failed_allocation_during_a_grid_change(how):
             if how == "set_state":
                 s.density, want = beyond, (r2, r3)
             else:
-                ctx.set_forms(xy=1)                        # keeps to the caller's grid
                 want = (p2, p3)
             arm(nth)
             try:
-                getattr(ctx, how)()
+                if how == "set_state":
+                    ctx.set_state()
+                else:
+                    ctx.set_forms(xy=1)                    # takes the state to the caller's grid
             except TCError as e:
                 assert e.code == abi.TCG_ERR_NOMEM
             else:
