@@ -531,7 +531,9 @@ __global__ void __launch_bounds__(ET) k_eig(int n, const double2 *A, double2 *w,
         const bool in = t > k + 1 && t < n;
         const double2 x = in ? h(t, k) : double2{0, 0}, al = h(k + 1, k);
         const double xn = sum(x.x * x.x + x.y * x.y);
-        if (xn == 0.0 && al.y == 0.0) continue;              // uniform
+        // nothing to annihilate (uniform).  Squares may underflow while x does not: then beta
+        // is 0 and the results are not finite, which the caller takes to the library
+        if (xn == 0.0 && al.y == 0.0 && !__syncthreads_or(zabs1(x) > 0.0)) continue;
         const double beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn), al.x);
         const double2 tau = {(beta - al.x) / beta, -al.y / beta};
         const double2 sc = zdiv(double2{1.0, 0.0}, double2{al.x - beta, al.y});

@@ -309,6 +309,25 @@ def test_expansion_edges(npw, nbasis, nblock):
     assert np.abs(V[:n].cpu().numpy() - np.array(rows)).max() < 1e-10
 
 
+@pytest.mark.parametrize("scale", [0.0, 1e-170, 1e-110, 1e110, 1e150])
+@pytest.mark.parametrize("n", [3, 17, 96])
+@pytest.mark.parametrize("real", [False, True])
+def test_subspace_eigen_of_extreme_norm(n, scale, real):
+    """matrices whose squared elements under- or overflow; eigenvalues and residual in
+    units of the scale, tolerance as in test_subspace_eigen"""
+    import torch
+    from tc_b200.context import subspace_ritz
+    rng = np.random.default_rng(n)
+    H = (rng.standard_normal((n, n)) + (0j if real else 1j) * rng.standard_normal((n, n))) * (scale > 0)
+    V = np.eye(n, n + 5, dtype=complex)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    w, _, Vo, _ = subspace_ritz(dev(V), [dev(scale * H.T @ V), None, None], n)
+    X = Vo.cpu().numpy()[:, :n].T
+    w = w / scale if scale else w
+    assert np.abs(np.linalg.norm(X, axis=0) - 1.0).max() <= 1e-12
+    assert np.abs(H @ X - X * w).max() <= 50 * n * 2.2e-16 * np.linalg.norm(H)
+
+
 @pytest.mark.parametrize("kind", ["general", "hermitian", "degenerate", "triangular"])
 @pytest.mark.parametrize("n", [1, 2, 3, 17, 32, 33, 64, 96, 112, 113])
 def test_subspace_eigen(n, kind):
