@@ -176,6 +176,23 @@ def test_density_beyond_the_pair_sphere():
     s.density = plain
 
 
+@pytest.mark.parametrize("nr,edge", [((18, 20, 16), None), ((16, 24, 18), None), ((30, 30, 30), 24)])
+def test_pencils_of_the_pair_balls(nr, edge):
+    """the table of needed pencils (several k-differences, unequal sides): the pruned
+    transforms give what the full ones give, up to the rounding of FP64"""
+    s = synth.small("TC", nr=nr, nk=2, ecut=4.0 if edge is None else 7.0, nbands=2, nocc=1, seed=2)
+    out = []
+    with Context(s, "fp64") as ctx:
+        if edge:
+            assert ctx.work_grid() == (edge,) * 3
+        for prune in (1, 0):
+            ctx.set_forms(prune=prune)
+            ctx.set_state()
+            out.append(ctx.apply(abi.TERMS_TC))
+    assert rel(out[0][0], out[1][0]) < 1e-12
+    assert rel(out[0][1], out[1][1]) < 1e-12
+
+
 def test_refused_pseudopotential_and_grid_change():
     """a local potential that is refused (NaN) leaves none: the next state may change
     the work grid, and the terms of an earlier pseudopotential are gone"""
