@@ -76,9 +76,15 @@ def test_run_time_shape_spin_channels(prec):
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 @pytest.mark.parametrize("n,ecut", [(12, 4.0), (15, 7.0), (16, 7.9), (18, 10.0), (20, 12.0)])
 def test_on_chip_exchange(n, ecut, prec):
-    """hf2x work grids of n^3 inside a finer grid; 16 sources"""
+    """hf2x work grids of n^3 inside a finer grid; 16 sources.  On chip up to 20^3, in
+    FP64 up to 18^3; 15^3 gives way to 16^3"""
     s = synth.small("HF", nr=(36, 36, 36), nk=2, ecut=ecut, nbands=3, nocc=2, seed=n)
-    check(s, abi.TERM_HF2X, prec)
+    check(s, abi.TERM_HF2X, prec, 16 if n == 15 else n)
+    with Context(s, prec) as ctx:
+        ctx.set_state()
+        ctx.profile(True)
+        ctx.apply(abi.TERM_HF2X)
+        assert ("hf2x:cube" in ctx.profile_read()) == (prec == "mixed" or n <= 18)
 
 
 @pytest.mark.parametrize("prec,n,ecut", [("mixed", 20, 12.0), ("fp64", 18, 10.0)])
@@ -127,7 +133,7 @@ def test_work_grid_time_reversal(method, prec):
     """k - q up to 4/3: the pair densities' sphere leaves the box of the caller's
     grid, whose own representation of those components defines the result"""
     s = synth.small(method, nr=(16, 16, 16), tr=True, ecut=5.0, nbands=2, nocc=1)
-    check(s, abi.TERMS_HF if method == "HF" else abi.TERMS_TC, prec)
+    check(s, abi.TERMS_HF if method == "HF" else abi.TERMS_TC, prec, 12 if method == "HF" else 16)
 
 
 def at_edge(n, fac):
@@ -158,6 +164,57 @@ def test_work_grid_next_to_the_callers(n, user, method, prec):
         assert ctx.work_grid() == ((user if stay else n),) * 3
 
 
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("method,F", [("TC", 1.2), ("BITC", 1.2), ("BITC", np.array([[1.3, 1.0], [1.0, 1.2]]))])
+def test_work_grid_spin_channels(method, F, prec):
+    """two spin channels, equal and unequal Jastrow channels, on a smaller grid"""
+    s = synth.small(method, nr=(24, 24, 24), nk=2, ecut=3.5, nbands=2, nocc=1, nspin=2, F=F, seed=8)
+    check(s, abi.TERMS_TC, prec, 16)
+
+
+def refine(s, n):
+    """the system on a finer n^3 grid, with the density of its orbitals there"""
+    n0 = np.array(s.nr)
+    w = np.stack([s.gindex % n0[0], (s.gindex // n0[0]) % n0[1], s.gindex // (n0[0] * n0[1])], 1)
+    m = np.mod(np.where(w > n0 // 2, w - n0, w), n)
+    s = dataclasses.replace(s, nr=(n, n, n), gindex=(m[:, 0] + n * (m[:, 1] + n * m[:, 2])).astype(np.int32))
+    s.density = O.density(s)
+    return s
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("term", ["hf2x", "tc2x", "tc3a1", "tc3b1", "tc3a2a4b2b5", "tc3a3b3b4b6"])
+def test_work_grid_of_a_symmetry_reduced_run(term, prec):
+    """silicon with rotations and the (1/4, 1/4, 1/4) translation, on a caller's grid
+    fine enough for a smaller work grid (a multiple of 4 for TC / BITC, on which the
+    translation is integral)"""
+    from test_qe_symmetry import qe_system
+    if term not in _qe:
+        s = refine(qe_system("HF" if term == "hf2x" else "BITC"), 24)
+        _qe[term] = s, O.apply(s, abi.TERM_NAMES[term])
+    s, (r2, r3) = _qe[term]
+    with Context(s, prec) as ctx:
+        ctx.set_state()
+        assert ctx.work_grid() == ((16,) * 3 if term == "hf2x" else (20,) * 3)
+        g2, g3 = ctx.apply(abi.TERM_NAMES[term])
+    ref, got = (r2, g2) if abi.TERM_NAMES[term] & abi.TERMS_H2 else (r3, g3)
+    assert rel(got, ref) < TOL[prec]
+
+
+_qe = {}
+
+
+@pytest.mark.parametrize("amplitude,edge", [(3e-14, 16), (3e-13, 24)])
+def test_density_at_the_threshold(amplitude, edge):
+    """a component beyond the pair densities' sphere just below 1e-13 of the largest is
+    dropped with the smaller grid, just above it the caller's grid is used; either
+    way the results are the oracle's for that density"""
+    s = synth.small("TC", nr=(24, 24, 24), nk=1, ecut=3.5, nbands=2, nocc=2, seed=4)
+    wave = 2.0 * amplitude * s.density[0].real.mean() * np.cos(2 * np.pi * 10 * (np.arange(s.N) % 24) / 24.0)
+    s.density = s.density + wave[None, :]
+    check(s, abi.TERMS_TC, "fp64", edge)
+
+
 def test_density_beyond_the_pair_sphere():
     """a density with a component outside the pair densities' sphere needs the
     caller's grid; the next state may go back to the smaller one"""
@@ -166,10 +223,13 @@ def test_density_beyond_the_pair_sphere():
     z, y, x = np.meshgrid(*[np.arange(32) / 32.0] * 3, indexing="ij")
     wave = 0.05 * np.abs(plain).max() * np.cos(2 * np.pi * (13 * x + 2 * y - 11 * z)).ravel()
     with Context(s, "fp64") as ctx:
-        for dens in (plain, plain + wave[None, :], plain):
+        small = ctx.work_grid()
+        assert small[0] < 32
+        for dens, grid in ((plain, small), (plain + wave[None, :], (32,) * 3), (plain, small)):
             s.density = dens
             r2, r3 = O.apply(s, abi.TERMS_TC)
             ctx.set_state()
+            assert ctx.work_grid() == grid
             g2, g3 = ctx.apply(abi.TERMS_TC)
             assert rel(g2, r2) < TOL["fp64"]
             assert rel(g3, r3) < TOL["fp64"]
