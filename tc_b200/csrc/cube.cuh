@@ -12,7 +12,8 @@
 // some 20 accesses and two grids of traffic each way.  Its floor is the
 // arithmetic: 6 line transforms per point, about 125 FP32 instructions at 20^3.
 // Measured 13.6 thousand cycles per pair there, one CTA per SM: an HF apply of 27
-// k-points (36^3, mixed) went from 4.37 to 2.12 ms, 1.77 of them here.
+// k-points (36^3, mixed) went from 4.37 to 2.03 ms, 1.81 of them here (1.77 with
+// FP32 sums over all sources).
 #pragma once
 #include "terms.cuh"
 #include "split.cuh"

@@ -366,7 +366,8 @@ template <typename V, class S, class Op> __host__ inline size_t smem_xyf()
 // 27-k case).  They and the next step's G plane are therefore copied
 // asynchronously into slots of shared memory that belong to the reading thread
 // alone, so a thread waits for its own copies and the passes' barriers stay the
-// only ones (20.3 ms with registers for three sums; 23.0 with one CTA more and
+// only ones (20.3 ms with registers for three sums, 22.4 with their FP64 additions
+// every FLUSH sources; 23.0 instead of 20.3 with one CTA more and
 // spills).  FP64 planes beyond 32^2 leave no room for the slots: there operands
 // are loaded in place and the sums live in shared memory.
 // GS > 1: the first GS - 1 outputs of a group wait in registers.

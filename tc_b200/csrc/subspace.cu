@@ -460,8 +460,10 @@ int mgs(int nv, int npw, double2 *V, double2 *T, int nbasis, int *ints, int *row
 // General complex eigenproblem A X = X D of order n <= EIG_MAX in one CTA: the
 // matrix in shared memory, Householder reduction to Hessenberg form, explicit
 // single-shift QR (the iteration of the EISPACK routine COMQR2, Peters and
-// Wilkinson 1970, with the deflation test of Ahues and Tisseur 1997), triangular
-// back substitution.  The rows of a sweep are a wavefront: the thread of column k
+// Wilkinson 1970, with the deflation test of Ahues and Tisseur 1997; this test with
+// its fallback for zero diagonals, the scaled Wilkinson shift and the exceptional
+// shifts at iterations 10 and 20 of 30 follow LAPACK's ZLAHQR), triangular back
+// substitution (its smallest pivot as in LAPACK's ZTREVC).  The rows of a sweep are a wavefront: the thread of column k
 // carries its running element in a register, forms rotation k as soon as rotation
 // k - 1 has arrived, and one barrier later every column applies it.  The columns
 // (and Z, by the other half of the CTA) then need no barrier at all: a thread

@@ -130,9 +130,9 @@ static double miller_extent(const Host &h, int i)
 // wait) and the next size fits as well or is the caller's own.  An apply at the
 // cutoff of the smaller size, ms on it and on the next:
 //            FP32 TC      HF            FP64 TC      HF
-//   15, 16   1.02  0.93   0.146 0.133   1.53  1.51   0.216 0.188   next in both
-//   27, 30   5.08  5.37   0.83  0.86    12.7  10.4   1.45  1.35    next in FP64
-//   45, 48   0.93  0.98   0.238 0.246   1.58  1.52   0.312 0.322   next in FP64 TC
+//   15, 16   0.96  0.88   0.129 0.120   1.47  1.45   0.173 0.164   next in both
+//   27, 30   5.15  5.20   0.81  0.85    12.5  9.12   1.41  1.32    next in FP64
+//   45, 48   0.88  0.91   0.217 0.214   1.51  1.46   0.290 0.293   next in FP64 TC
 static int choose_reduced(Host &h, bool fp64)
 {
     h.rmax = 0;

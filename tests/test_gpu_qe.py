@@ -3,7 +3,7 @@ test/example3; tests/golden/qe_si.npz): a symmetry-reduced k-set with 48
 space-group operations, 24 of them non-symmorphic (translation (1/4,1/4,1/4)),
 and time reversal.  This runs the rotated-k scatter (Gindex / phase of every
 equivalent k) and the rotation of the tc3a2a4b2b5 intermediates by U != 1 with
-a translation (k_rot_scalar / k_rot_vec) on the device."""
+a translation (k_rot) on the device."""
 import numpy as np
 import pytest
 
