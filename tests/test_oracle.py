@@ -139,7 +139,8 @@ def test_oracle_matches_golden_fixture(name):
     from golden.make_golden import mask_of, system
     s = system(name)
     ref = np.load(os.path.join(os.path.dirname(__file__), "golden", name + ".npz"))
-    assert np.array_equal(ref["psi"], s.psi)
+    # orthonormalised on the host, whose BLAS may sum in another order: one unit in the last place
+    assert np.abs(ref["psi"] - s.psi).max() <= 1e-15
     h2, h3 = O.apply(s, mask_of(s))
     for got, want in ((h2, ref["h2"]), (h3, ref["h3"])):
         m = np.abs(want).max()
