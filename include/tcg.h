@@ -171,7 +171,8 @@ int tcg_set_state(tcg_ctx *ctx, const tcg_state_desc *st);
 /* Redo the per-state work of the last tcg_set_state from the device-resident
  * copy (R-space orbitals, local three-body potentials, and -- on the next
  * apply -- the tc3a2a4b2b5 occupied-pair stage), without a host upload.
- * Equivalent to calling tcg_set_state again with the same arrays. */
+ * Equivalent to calling tcg_set_state again with the same arrays; after an error
+ * there is no state. */
 int tcg_refresh_state(tcg_ctx *ctx);
 
 /* Apply the selected terms to a block of trial orbitals and ACCUMULATE into

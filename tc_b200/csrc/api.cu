@@ -166,12 +166,14 @@ int tcg::build_prune_table(tcg_ctx *c)
                 if (fabs(ci) + bl.r * alen[i] >= (h.n[i] - 1) / 2.0) return TCG_OK;   // support could wrap
             }
         }
-    TRY(c->prune_tab.ensure(pt.bytes));
-    TRY(up(c->meta, ball.data(), pt.nent * sizeof(PruneBall), c->stream));
+    // the balls behind the table (an allocation of their own takes longer than the table)
+    const size_t at = (pt.bytes + 7) / 8 * 8;
+    TRY(c->prune_tab.ensure(at + pt.nent * sizeof(PruneBall)));
+    unsigned char *tab = c->prune_tab.as<unsigned char>();
+    TCG_CUDA(cudaMemcpyAsync(tab + at, ball.data(), pt.nent * sizeof(PruneBall), cudaMemcpyHostToDevice, c->stream));
     RecipC rc;
     memcpy(rc.R, h.recip, sizeof rc.R);
-    unsigned char *tab = c->prune_tab.as<unsigned char>();
-    TRY(launch(c, k_prune, dim3((unsigned)pt.nent), dim3(256), 0, c->gd, rc, (const PruneBall *)c->meta.p,
+    TRY(launch(c, k_prune, dim3((unsigned)pt.nent), dim3(256), 0, c->gd, rc, (const PruneBall *)(tab + at),
                reinterpret_cast<unsigned long long *>(tab), reinterpret_cast<int *>(tab + pt.nact),
                reinterpret_cast<unsigned short *>(tab + pt.perm)));
     c->prune_nact.resize(pt.nent);
